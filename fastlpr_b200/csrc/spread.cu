@@ -237,37 +237,79 @@ __global__ void tile_scan_kernel(int ntiles, int item_points, const int* __restr
   }
 }
 
-// Sorted structure-of-arrays records, one slot per point in tile order:
-//   rec_base[pos]          local base cell of the point inside its tile,
-//                          packed 10 bits per axis (T <= 1024);
-//   rec_frac[a * n + pos]  k_a - hx_a * m_a (offset of the knot from its cell);
-//   rec_val[c * n + pos]   value of channel c (ones channel excluded).
-template <typename Real>
-__global__ void bin_scatter_kernel(SpreadGeom g, int64_t n, const double* __restrict__ x,
-                                   const double* __restrict__ d_kmap,
-                                   const int* __restrict__ offsets, int* __restrict__ cursor,
-                                   int nv, ChanPtrs cp, int* __restrict__ rec_base,
-                                   int* __restrict__ rec_idx, Real* __restrict__ rec_frac,
-                                   Real* __restrict__ rec_val) {
+// Sorted records, one per point in tile order:
+//   rec_base[pos]  local base cell of the point inside its tile, packed 10
+//                  bits per axis (T <= 1024); rec_idx[pos] its index;
+//   rec[pos * stride + ..]  the knot offsets k_a - hx_a m_a of the d axes,
+//                  then the values of all channels (1 for the constant one),
+//                  padded to an even count of doubles.
+// A record is contiguous because its readers want all of it: they take the
+// points of one tile in an order of their own, and 16-byte pieces of one
+// record cost a quarter of the sectors that one scattered double per array
+// does, on the write side too (each warp turns its 32 records through shared
+// memory so that neighbouring lanes write neighbouring pieces).
+constexpr int kScatterSlots = 16;  // doubles of a record staged at a time
+
+__host__ __device__ inline int rec_stride(int d, int nchan) { return (d + nchan + 1) & ~1; }
+
+__global__ void __launch_bounds__(256)
+bin_scatter_kernel(SpreadGeom g, int64_t n, const double* __restrict__ x,
+                   const double* __restrict__ d_kmap, const int* __restrict__ offsets,
+                   int* __restrict__ cursor, int nchan, int ones_channel, ChanPtrs cp,
+                   int* __restrict__ rec_base, int* __restrict__ rec_idx,
+                   double* __restrict__ rec) {
+  constexpr int SS = kScatterSlots + 2;  // staging stride: 16-byte rows on distinct banks
   __shared__ KnotAxis s_ax[3];
+  __shared__ __align__(16) double s_rec[8][32 * SS];
   load_axes(g, d_kmap, s_ax);
   __syncthreads();
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int d = g.d, stride = rec_stride(d, nchan);
+  double* sr = s_rec[warp];
+  // whole warps go round together: the last one has idle lanes
+  for (int64_t i0 = ((int64_t)blockIdx.x * 8 + warp) * 32; i0 < n; i0 += (int64_t)gridDim.x * 256) {
+    const int64_t i = i0 + lane;
+    const int cnt = (int)min((int64_t)32, n - i0);
     int m[3];
     double k[3];
-    const int t = point_tile(g, s_ax, x, i, m, k);
-    const int pos = offsets[t] + atomicAdd(&cursor[t], 1);
-    int packed = 0;
-    for (int a = 0; a < g.d; ++a) {
-      int home = m[a] % g.L[a];
-      if (home < 0) home += g.L[a];
-      packed |= (home % g.T[a]) << (10 * a);
-      rec_frac[(int64_t)a * n + pos] = (Real)dsub(k[a], dmul(g.ax[a].hx, (double)m[a]));
+    int pos = 0;
+    if (lane < cnt) {
+      const int t = point_tile(g, s_ax, x, i, m, k);
+      pos = offsets[t] + atomicAdd(&cursor[t], 1);
+      int packed = 0;
+      for (int a = 0; a < d; ++a) {
+        int home = m[a] % g.L[a];
+        if (home < 0) home += g.L[a];
+        packed |= (home % g.T[a]) << (10 * a);
+      }
+      rec_base[pos] = packed;
+      rec_idx[pos] = (int)i;
     }
-    rec_base[pos] = packed;
-    rec_idx[pos] = (int)i;
-    for (int c = 0; c < nv; ++c) rec_val[(int64_t)c * n + pos] = (Real)cp.col[c][i];
+    for (int s0 = 0; s0 < stride; s0 += kScatterSlots) {
+      const int ns = min(kScatterSlots, stride - s0);
+      if (lane < cnt) {
+        for (int j = 0; j < ns; ++j) {
+          const int slot = s0 + j, c = slot - d;
+          double v = 0.0;
+          if (c < 0) {
+            v = dsub(k[slot], dmul(g.ax[slot].hx, (double)m[slot]));
+          } else if (c < nchan) {
+            v = ones_channel && c == 0 ? 1.0 : cp.col[c - ones_channel][i];
+          }
+          sr[lane * SS + j] = v;
+        }
+      }
+      __syncwarp();
+      const int nch = ns / 2;
+      for (int t0 = 0; t0 < cnt * nch; t0 += 32) {
+        const int t = t0 + lane, r = t / nch, ch = t - r * nch;
+        const int64_t p = __shfl_sync(0xffffffffu, pos, r & 31);
+        if (t < cnt * nch)
+          *reinterpret_cast<double2*>(rec + p * stride + s0 + 2 * ch) =
+              *reinterpret_cast<const double2*>(sr + r * SS + 2 * ch);
+      }
+      __syncwarp();
+    }
   }
 }
 
@@ -321,11 +363,11 @@ __device__ __forceinline__ double fexp(double v) { return exp(v); }
 // accumulator with one atomic per non-zero cell.
 template <typename Acc, typename Real, int NT1>
 __global__ void __launch_bounds__(kSpreadThreads)
-tile_accumulate_kernel(SpreadGeom g, int64_t n, int nchan, int ones_channel, int cgroup,
+tile_accumulate_kernel(SpreadGeom g, int nchan, int cgroup,
                        const int* __restrict__ offsets, const int* __restrict__ items,
-                       const int* __restrict__ rec_base, const Real* __restrict__ rec_frac,
-                       const Real* __restrict__ rec_val, const double* __restrict__ absum,
-                       int margin_bits, Acc* __restrict__ gacc) {
+                       const int* __restrict__ rec_base, const double* __restrict__ rec,
+                       int stride, const double* __restrict__ absum, int margin_bits,
+                       Acc* __restrict__ gacc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Acc* acc = reinterpret_cast<Acc*>(smem_raw);
   const int c_begin = blockIdx.y * cgroup;
@@ -381,13 +423,13 @@ tile_accumulate_kernel(SpreadGeom g, int64_t n, int nchan, int ones_channel, int
     Real wrow = Real(1);
     int cell = 0;
     for (int a = 0; a < d - 1; ++a) {
-      const Real fr = rec_frac[(int64_t)a * n + p];
+      const Real fr = (Real)rec[(int64_t)p * stride + a];
       const Real diff = fr - (Real)g.ax[a].hx * (Real)(j[a] - MSP);
       wrow *= fexp(-(diff * diff) / (Real)g.four_tau[a]);
       cell = cell * g.W[a] + ((packed >> (10 * a)) & 1023) + j[a];
     }
     cell = cell * Wl + ((packed >> (10 * (d - 1))) & 1023);
-    const Real frl = rec_frac[(int64_t)(d - 1) * n + p];
+    const Real frl = (Real)rec[(int64_t)p * stride + d - 1];
     Real w[NT1];
 #pragma unroll
     for (int jl = 0; jl < NT1; ++jl) {
@@ -395,8 +437,7 @@ tile_accumulate_kernel(SpreadGeom g, int64_t n, int nchan, int ones_channel, int
       w[jl] = wrow * fexp(-(diff * diff) / ftl);
     }
     for (int c = 0; c < nc; ++c) {
-      const int ch = c_begin + c;
-      const Real v = (ones_channel && ch == 0) ? Real(1) : rec_val[(int64_t)(ch - ones_channel) * n + p];
+      const Real v = (Real)rec[(int64_t)p * stride + d + c_begin + c];
       const Real sc = scale[c];
       Acc* dst = acc + c * tc + cell;
 #pragma unroll
@@ -427,25 +468,378 @@ tile_accumulate_kernel(SpreadGeom g, int64_t n, int nchan, int ones_channel, int
   }
 }
 
-// ---- 2-D path: per-cell register accumulation ------------------------------
-// Tiles of 8 x 8 cells.  A CTA takes the points of one work item in batches
-// of kBatch2; each batch is counting-sorted by cell in shared memory and its
-// 2 x NT1 tap weights and scaled channel values are cached there.  A warp
-// then takes one tile row l0 and a block of channel groups: lane
-// (jy, group) walks the points of that row cell by cell and sums, in
-// registers, the contributions of tap row jy to the NT1 + 7 cells of halo row
-// l0 + jy that the 8 cells of the row reach, for kUnitCh channels.  Only
-// those sums reach the shared tile (one atomic each), instead of one atomic
-// per (point, tap, channel).  In the fixed-point accumulator every product
-// is rounded to an integer before it is added, so sums stay exact and the
-// grid does not depend on the order of the points.
-constexpr int kT2 = 8;         // tile edge of the 2-D path
-constexpr int kBatch2 = 256;   // points per batch (one per thread while caching)
-constexpr int kUnitCh = 2;     // channels per lane
+// ---- 2-D path: one or two warps per work item -------------------------------
+// Tiles of 8 x 8 cells.  The warps of a CTA (one, or two that split the
+// channels) take the points of one work item: they sort them by cell
+// (counting sort of their indices), then walk them row of cells by row of
+// cells, 32 points at a time staged in shared memory (per-axis tap weights
+// and the records, copied in the background).  Lane (jm, group) holds, in
+// registers, the W = NT1 + 7 cells of one halo row for UC channels: halo row
+// r belongs to the lanes with jm = r mod NT1, so at tile row l0 they take tap
+// jy = (jm - l0) mod NT1, every lane of the NT1 footprint rows works, and a
+// row leaves the registers once, when the walk has passed it.  It goes
+// through a small shared buffer to one global atomic per non-zero cell: no
+// atomics on shared memory, no accumulator tile.  In the fixed-point
+// accumulator every product is rounded to an integer as it is added, so sums
+// are exact and the grid does not depend on the order of the points.
+//
+// Bound by the FP64 pipe (UC (NT1 + 1) multiply-adds per point and warp,
+// about 2.2 cycles each) and by latency: the multiply-add takes 23 cycles,
+// so the next point's values are read and scaled beside this point's sums,
+// and UC stays at 3 or less, which leaves registers for 12 to 16 warps.
+constexpr int kT2 = 8;            // tile edge of the 2-D path
+constexpr int kItem2 = 1024;      // most points of a work item
 
-// Register accumulators hold doubles in both precisions.  Fixed point: each
-// product is rounded to the nearest integer (ties to even, like
-// __double2ll_rn) by adding and subtracting 1.5 * 2^52 (exact for
+// Register accumulators of the tile kernels, one fused multiply-add per
+// product.  Fixed point with quantum q (a power of two): the register starts
+// at 1.5 * 2^52 q and stays in [2^52 q, 2^53 q), where every double is a
+// multiple of q (the sums stay below 2^50 q), so a = v w + a adds the product
+// rounded to the nearest multiple and the sum is exact.  A product halfway
+// between two multiples would round by the parity of the sum so far, that is
+// by the order of the points; factor() therefore sets the last mantissa bit
+// of v: with |v w| < 2^50 q and w <= 1 the product then has a non-zero bit
+// below q / 2 and no tie can occur.  (One FP64 instruction instead of a fused
+// multiply-add and a 64-bit integer add, or of a product and two roundings.)
+// Float64 accumulation adds the fused product.
+template <typename Acc>
+struct RegSum;
+template <>
+struct RegSum<long long> {
+  static constexpr double kBias = 6755399441055744.0;  // 1.5 * 2^52
+  __device__ static double zero(double q) { return kBias * q; }
+  __device__ static double factor(double v) {
+    return __longlong_as_double(__double_as_longlong(v) | 1ll);
+  }
+  // the sum in units of q, scale = 1 / q
+  __device__ static long long value(double a, double scale) {
+    return __double_as_longlong(a * scale) - __double_as_longlong(kBias);
+  }
+};
+template <>
+struct RegSum<double> {
+  __device__ static double zero(double) { return 0.0; }
+  __device__ static double factor(double v) { return v; }
+  __device__ static double value(double a, double) { return a; }
+};
+
+// Tap weights of one axis from the knot's offset f to its cell:
+// exp(-(f - hx j)^2 / ft) = exp(-f^2 / ft) r^j C_|j|, r = exp(2 f hx / ft),
+// C_j = exp(-(hx j)^2 / ft), for j = -MSP .. MSP into w (two exponentials
+// and one reciprocal per axis instead of an exponential and a division per tap).
+template <int NT1>
+__device__ __forceinline__ void tap_weights(double f, double hx, double inv_ft,
+                                            const double* __restrict__ cj, double* __restrict__ w) {
+  constexpr int MSP = (NT1 - 1) / 2;
+  const double e0 = exp(-(f * f) * inv_ft);
+  w[MSP] = e0;
+  if constexpr (MSP > 0) {
+    const double b = 2.0 * f * hx * inv_ft;
+    const double rp = exp(b), rm = 1.0 / rp;
+    double p = e0, m = e0;
+#pragma unroll
+    for (int j = 1; j <= MSP; ++j) {
+      p *= rp;
+      m *= rm;
+      const double c = cj[j];
+      w[MSP + j] = p * c;
+      w[MSP - j] = m * c;
+    }
+  }
+}
+
+// Tile that owns work item `item`: the largest t with items[t] <= item.  One
+// warp probes 32 places at a time (three dependent loads for 16,384 tiles
+// instead of fourteen).
+__device__ __forceinline__ int item_tile(const int* __restrict__ items, int ntiles, int item,
+                                         int lane) {
+  int lo = 0, hi = ntiles;  // items[lo] <= item < items[hi]
+  while (hi - lo > 1) {
+    const int step = (hi - lo + 31) / 32;
+    const int t = lo + lane * step;
+    const unsigned le = __ballot_sync(0xffffffffu, t < hi && items[t] <= item);
+    lo += (31 - __clz(le)) * step;  // lane 0 always holds
+    hi = min(hi, lo + step);
+  }
+  return lo;
+}
+
+__device__ __forceinline__ void copy16_async(double* dst, const double* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copies_wait() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// Channel groups of a warp: as many footprints of NT1 lanes as fit.
+__host__ __device__ constexpr int groups2(int nt1) { return nt1 < 4 ? 8 : 32 / nt1; }
+
+// Warps of one SM (one per CTA) that UC channels per lane leave registers for.
+__host__ __device__ constexpr int warps2(int nt1, int uc) {
+  const int regs = 2 * uc * (nt1 + 7) + 46;  // accumulators and working registers
+  return regs <= 128 ? 16 : (regs <= 176 ? 12 : (regs <= 200 ? 10 : 8));
+}
+
+// Shared memory of one CTA.  The rows that the lanes still hold at the end
+// go through the space of the staged points.
+template <int NT1, int UC, int NW>
+struct Stage2 {
+  static constexpr int W = kT2 + NT1 - 1;     // halo cells per axis
+  static constexpr int GPL = groups2(NT1);    // channel groups of a warp
+  static constexpr int NCW = UC * GPL;        // channels of a warp
+  static constexpr int NCB = NCW * NW;        // channels of the CTA
+  static constexpr int WXS = (NT1 + 1) & ~1;  // even row stride: two axis-1 weights per load
+  static constexpr int RS = (2 + NCB + 1) & ~1;  // staged record: 2 knot offsets, the values
+  static constexpr int WR = W | 1;            // row-buffer stride of one channel
+  struct Points {
+    double rec[2][33 * RS];  // records of this batch and of the next (and one read ahead)
+    double wx[32 * WXS];
+    double wy[33 * NT1];
+    double row[NCB * WR];
+    unsigned short order[kItem2];
+    unsigned char cell[kItem2];
+  };
+  union {
+    Points st;
+    double rows[NT1 * NCB * WR];
+  };
+  double scale[NCB], zero[NCB];
+  double cj[2][(NT1 - 1) / 2 + 1];
+  int off[kT2 * kT2 + 1];
+  int cur[kT2 * kT2];
+  int col[W];  // grid columns of the halo
+};
+
+// Adds `nrows` halo rows from grid row gr0 on, (rows, NCW, WR) registers of
+// one warp's lanes for its channels c_w .. c_w + nc of the CTA's, to the
+// global accumulator: one atomic per non-zero cell.
+template <typename Acc, typename S>
+__device__ __forceinline__ void add_rows(const SpreadGeom& g, const S& sh, const double* buf,
+                                         int nrows, int gr0, int c_begin, int c_w, int nc,
+                                         int lane, Acc* __restrict__ gacc) {
+  constexpr int W = S::W, N = S::NCW * W, U = (N + 31) / 32;
+  for (int r = 0; r < nrows; ++r) {
+    int gr = (gr0 + r) % g.L[0];
+    if (gr < 0) gr += g.L[0];
+    Acc* grow = gacc + (int64_t)(c_begin + c_w) * g.cells + (int64_t)gr * g.L[1];
+    const double* rb = buf + r * S::NCW * S::WR;
+    Acc v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int idx = u * 32 + lane, c = idx / W, j = idx - c * W;
+      v[u] = c < nc ? RegSum<Acc>::value(rb[c * S::WR + j], sh.scale[c_w + c]) : Acc(0);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int idx = u * 32 + lane, c = idx / W, j = idx - c * W;
+      if (v[u] != Acc(0)) AccOps<Acc>::add_global(grow + (int64_t)c * g.cells + sh.col[j], v[u]);
+    }
+  }
+}
+
+template <int NW>
+__device__ __forceinline__ void sync2() {
+  if constexpr (NW == 1)
+    __syncwarp();
+  else
+    __syncthreads();
+}
+
+template <typename Acc, int NT1, int UC, int NW>
+__global__ void __launch_bounds__(32 * NW, warps2(NT1, UC) / NW)
+tile_accumulate_2d_kernel(SpreadGeom g, int nchan, const int* __restrict__ offsets,
+                          const int* __restrict__ items, const int* __restrict__ rec_base,
+                          const double* __restrict__ rec, int stride,
+                          const double* __restrict__ absum, int margin_bits,
+                          Acc* __restrict__ gacc) {
+  using S = Stage2<NT1, UC, NW>;
+  constexpr int MSP = (NT1 - 1) / 2;
+  constexpr int NLC = kT2 * kT2;
+  constexpr int NT = 32 * NW;
+  constexpr int W = S::W, GPL = S::GPL, NCW = S::NCW, NCB = S::NCB, WXS = S::WXS, RS = S::RS,
+                WR = S::WR;
+  __shared__ __align__(16) unsigned char s_raw[sizeof(S)];
+  S& sh = *reinterpret_cast<S*>(s_raw);
+  int* const off = sh.off;
+  int* const cur = sh.cur;
+
+  const int item = blockIdx.x;
+  if (item >= items[g.ntiles]) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tile = item_tile(items, g.ntiles, item, lane);
+  const int p_begin = offsets[tile] + (item - items[tile]) * g.item_points;
+  const int np = min(offsets[tile + 1] - p_begin, g.item_points);
+  const int tc0 = tile / g.ntile[1], tc1 = tile - tc0 * g.ntile[1];
+  const int c_begin = blockIdx.y * NCB;
+  const int nc = min(nchan - c_begin, NCB);
+  const int c_w = warp * NCW, nc_w = min(max(nc - c_w, 0), NCW);
+  const int jm = lane % NT1, grp = lane / NT1;
+  const bool active = grp < GPL && grp * UC < nc_w;
+
+  const double hx0 = g.ax[0].hx, hx1 = g.ax[1].hx;
+  const double if0 = 1.0 / g.four_tau[0], if1 = 1.0 / g.four_tau[1];
+  for (int c = tid; c < NCB; c += NT) {
+    const double sc = (c < nc && absum != nullptr) ? fixed_scale(absum[c_begin + c], margin_bits) : 1.0;
+    sh.scale[c] = sc;
+    sh.zero[c] = RegSum<Acc>::zero(1.0 / sc);
+  }
+  if (tid < 2 * (MSP + 1)) {
+    const int ax = tid / (MSP + 1), j = tid - ax * (MSP + 1);
+    const double t = (ax == 0 ? hx0 : hx1) * (double)j;
+    sh.cj[ax][j] = exp(-(t * t) * (ax == 0 ? if0 : if1));
+  }
+  if (tid < W) {
+    const int gc = (tc1 * kT2 + tid - MSP) % g.L[1];
+    sh.col[tid] = gc < 0 ? gc + g.L[1] : gc;
+  }
+  // counting sort by cell
+  for (int i = tid; i < NLC; i += NT) cur[i] = 0;
+  sync2<NW>();
+#pragma unroll 4
+  for (int i = tid; i < np; i += NT) {
+    const int packed = rec_base[p_begin + i];
+    const int lc = (packed & 1023) * kT2 + ((packed >> 10) & 1023);
+    sh.st.cell[i] = (unsigned char)lc;
+    atomicAdd(&cur[lc], 1);
+  }
+  sync2<NW>();
+  if (warp == 0) {
+    const int a0 = cur[2 * lane], a1 = cur[2 * lane + 1];
+    int incl = a0 + a1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    const int excl = incl - a0 - a1;
+    off[2 * lane] = excl;
+    off[2 * lane + 1] = excl + a0;
+    if (lane == 31) off[NLC] = incl;
+    __syncwarp();
+    cur[2 * lane] = excl;
+    cur[2 * lane + 1] = excl + a0;
+  }
+  sync2<NW>();
+  for (int i = tid; i < np; i += NT)
+    sh.st.order[atomicAdd(&cur[sh.st.cell[i]], 1)] = (unsigned short)i;
+  sync2<NW>();
+
+  // records of the 32 points from b0 on, copied in the background in pieces
+  // of 16 bytes: the knot offsets, then this CTA's channels
+  const int npc = 1 + (nc + 1) / 2, dpt = NT / npc, dpc = NT - dpt * npc;
+  const int pt0 = tid / npc, pc0 = tid - pt0 * npc;
+  const double* rec_t = rec + (int64_t)p_begin * stride;
+  auto fetch = [&](int b0, int half) {
+    const int cnt = min(32, np - b0);
+    for (int pt = pt0, pc = pc0; pt < cnt;) {
+      copy16_async(&sh.st.rec[half][pt * RS + 2 * pc],
+                   rec_t + (int64_t)sh.st.order[b0 + pt] * stride + (pc ? c_begin : 0) + 2 * pc);
+      pc += dpc;
+      pt += dpt;
+      if (pc >= npc) {
+        pc -= npc;
+        ++pt;
+      }
+    }
+  };
+  fetch(0, 0);
+
+  const int vofs = c_w + (active ? grp * UC : 0);  // idle lanes repeat group 0 and drop it
+  double a[UC][W];
+#pragma unroll
+  for (int k = 0; k < UC; ++k)
+#pragma unroll
+    for (int j = 0; j < W; ++j) a[k][j] = sh.zero[vofs + k];
+  int row = 0, half = 0;
+  for (int b0 = 0; b0 < np; b0 += 32, half ^= 1) {
+    const int b1 = min(b0 + 32, np);
+    copies_wait();
+    sync2<NW>();  // this batch's records are there, the last one's readers done
+    if (b0 + lane < b1) {
+      const double2 f = *reinterpret_cast<const double2*>(&sh.st.rec[half][lane * RS]);
+      if (NW == 1 || warp == 0) tap_weights<NT1>(f.x, hx0, if0, sh.cj[0], sh.st.wy + lane * NT1);
+      if (NW == 1 || warp == 1) tap_weights<NT1>(f.y, hx1, if1, sh.cj[1], sh.st.wx + lane * WXS);
+    }
+    sync2<NW>();
+    fetch(b1, half ^ 1);
+    for (;;) {
+      int jy = jm - row % NT1;
+      if (jy < 0) jy += NT1;
+      const int* ro = off + row * kT2;
+      int pp = max(ro[0], b0) - b0;
+      const double* yp = sh.st.wy + pp * NT1 + jy;
+      const double* vp = sh.st.rec[half] + pp * RS + 2 + vofs;
+      const double2* xp = reinterpret_cast<const double2*>(sh.st.wx + pp * WXS);
+      double v[UC];  // the next point's values times its axis-0 weight
+#pragma unroll
+      for (int k = 0; k < UC; ++k) v[k] = RegSum<Acc>::factor(*yp * vp[k]);
+#pragma unroll
+      for (int cr = 0; cr < kT2; ++cr) {
+        const int pe = min(ro[cr + 1], b1) - b0;
+#pragma unroll 1
+        for (; pp < pe; ++pp) {
+          yp += NT1;
+          vp += RS;
+          const double wyn = *yp;
+          double u[UC], w[WXS];
+#pragma unroll
+          for (int k = 0; k < UC; ++k) u[k] = vp[k];
+#pragma unroll
+          for (int jx = 0; jx < NT1; jx += 2) {
+            const double2 q = xp[jx / 2];
+            w[jx] = q.x;
+            w[jx + 1] = q.y;
+          }
+          xp += WXS / 2;
+#pragma unroll
+          for (int jx = 0; jx < NT1; ++jx)
+#pragma unroll
+            for (int k = 0; k < UC; ++k) a[k][cr + jx] = __fma_rn(v[k], w[jx], a[k][cr + jx]);
+#pragma unroll
+          for (int k = 0; k < UC; ++k) v[k] = RegSum<Acc>::factor(wyn * u[k]);
+        }
+      }
+      if (ro[kT2] > b1) break;      // the row goes on in the next batch
+      if (row >= W - NT1) break;    // every lane on its last row
+      // halo row `row` is complete: its lanes hand it over and start row + NT1
+      double* rb = sh.st.row + c_w * WR;
+      if (active && jm == row % NT1) {
+        double* rp = rb + grp * UC * WR;
+#pragma unroll
+        for (int k = 0; k < UC; ++k) {
+          const double z = sh.zero[vofs + k];
+#pragma unroll
+          for (int j = 0; j < W; ++j) {
+            rp[k * WR + j] = a[k][j];
+            a[k][j] = z;
+          }
+        }
+      }
+      __syncwarp();
+      add_rows<Acc, S>(g, sh, rb, 1, tc0 * kT2 + row - MSP, c_begin, c_w, nc_w, lane, gacc);
+      __syncwarp();
+      ++row;
+    }
+  }
+  // the last NT1 rows, each in its own lanes
+  sync2<NW>();
+  double* rb = sh.rows + (size_t)warp * NT1 * NCW * WR;
+  if (active) {
+    int r = (jm - (W - NT1)) % NT1;  // position of this lane's row among W - NT1 .. W - 1
+    if (r < 0) r += NT1;
+    double* rp = rb + (r * NCW + grp * UC) * WR;
+#pragma unroll
+    for (int k = 0; k < UC; ++k)
+#pragma unroll
+      for (int j = 0; j < W; ++j) rp[k * WR + j] = a[k][j];
+  }
+  __syncwarp();
+  add_rows<Acc, S>(g, sh, rb, NT1, tc0 * kT2 + (W - NT1) - MSP, c_begin, c_w, nc_w, lane, gacc);
+}
+
+// Register accumulators of the 3-D path hold doubles in both precisions.
+// Fixed point: each product is rounded to the nearest integer (ties to even,
+// like __double2ll_rn) by adding and subtracting 1.5 * 2^52 (exact for
 // |v| < 2^51), and the integer sums stay below 2^50, so every addition is
 // exact; the flush converts the exact integer sum once.
 template <typename Acc>
@@ -469,211 +863,6 @@ __device__ __forceinline__ long long reg_value<long long>(double a) {
 template <>
 __device__ __forceinline__ double reg_value<double>(double a) {
   return a;
-}
-
-__device__ __forceinline__ void shared_add(long long* p, long long v) {
-  atomicAdd(reinterpret_cast<unsigned long long*>(p), (unsigned long long)v);
-}
-__device__ __forceinline__ void shared_add(double* p, double v) { atomicAdd(p, v); }
-
-// Register accumulators of the 2-D path.  Fixed point: the product v w is
-// rounded once to the nearest integer by the fused multiply-add
-// t = v w + 1.5 * 2^52 (every double in [2^52, 2^53) is an integer, and
-// |v w| < 2^50 keeps t there), and the bit pattern of t is
-// bits(1.5 * 2^52) + round(v w), so the register adds the bit patterns in
-// integer arithmetic (modulo 2^64) and the flush subtracts the bias once per
-// add it received.  One FP64 instruction per product; the sum is exact and
-// independent of the order of the points.  Float64 accumulation adds the
-// fused product.
-template <typename Acc>
-struct Reg2;
-template <>
-struct Reg2<long long> {
-  using T = unsigned long long;
-  static constexpr unsigned long long kBias = 0x4338000000000000ull;  // bits(1.5 * 2^52)
-  __device__ static void add(T& a, double v, double w) {
-    a += (unsigned long long)__double_as_longlong(__fma_rn(v, w, 6755399441055744.0));
-  }
-  __device__ static long long value(T a, int adds) {
-    return (long long)(a - (unsigned long long)adds * kBias);
-  }
-};
-template <>
-struct Reg2<double> {
-  using T = double;
-  __device__ static void add(T& a, double v, double w) { a = __fma_rn(v, w, a); }
-  __device__ static double value(T a, int) { return a; }
-};
-
-// Halo-row stride (odd) and channel stride (odd) of the shared tile.
-__host__ __device__ constexpr int row_stride2(int nt1) { return (kT2 + nt1 - 1) | 1; }
-__host__ __device__ constexpr int chan_stride2(int w0, int nt1) { return (w0 * row_stride2(nt1)) | 1; }
-
-template <typename Acc, int NT1>
-__global__ void __launch_bounds__(kBatch2, 2)
-tile_accumulate_2d_kernel(SpreadGeom g, int64_t n, int nchan, int ones_channel, int cgroup,
-                          const int* __restrict__ offsets, const int* __restrict__ items,
-                          const int* __restrict__ rec_base, const double* __restrict__ rec_frac,
-                          const double* __restrict__ rec_val, const double* __restrict__ absum,
-                          int margin_bits, Acc* __restrict__ gacc) {
-  constexpr int MSP = (NT1 - 1) / 2;
-  constexpr int NACC = kT2 + NT1 - 1;  // halo cells one tile row reaches
-  constexpr int RS = row_stride2(NT1);
-  constexpr int GPL = 32 / NT1;        // channel groups per warp
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ int cnt[kT2 * kT2];
-  __shared__ int off[kT2 * kT2 + 1];
-  __shared__ double scale[32];
-  const int c_begin = blockIdx.y * cgroup;
-  const int nc = min(nchan, c_begin + cgroup) - c_begin;
-  const int T0 = g.T[0], W0 = g.W[0];
-  const int CS = chan_stride2(W0, NT1);
-  Acc* acc = reinterpret_cast<Acc*>(smem_raw);                       // nc x CS
-  double* wy = reinterpret_cast<double*>(acc + (size_t)nc * CS);     // kBatch2 x NT1
-  double* wx = wy + kBatch2 * NT1;                                   // kBatch2 x NT1
-  double* vs = wx + kBatch2 * NT1;                                   // kBatch2 x nc
-
-  const int item = blockIdx.x;
-  if (item >= items[g.ntiles]) return;
-  int lo = 0, hi = g.ntiles;
-  while (hi - lo > 1) {
-    int mid = (lo + hi) >> 1;
-    if (items[mid] <= item) lo = mid; else hi = mid;
-  }
-  const int tile = lo;
-  const int p_begin = offsets[tile] + (item - items[tile]) * g.item_points;
-  const int p_end = min(offsets[tile + 1], p_begin + g.item_points);
-  const int tc0 = tile / g.ntile[1], tc1 = tile - tc0 * g.ntile[1];
-
-  for (int i = threadIdx.x; i < nc * CS; i += blockDim.x) acc[i] = Acc(0);
-  if (threadIdx.x < 32)
-    scale[threadIdx.x] =
-        (threadIdx.x < nc && absum != nullptr) ? fixed_scale(absum[c_begin + threadIdx.x], margin_bits)
-                                               : 1.0;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  const int jy = lane % NT1, gsub = lane / NT1;
-  const int ngrp = (nc + kUnitCh - 1) / kUnitCh;
-  const int ngblk = (ngrp + GPL - 1) / GPL;
-  const int nlc = T0 * kT2;
-  const double hx0 = g.ax[0].hx, hx1 = g.ax[1].hx;
-  const double ft0 = g.four_tau[0], ft1 = g.four_tau[1];
-
-  for (int b0 = p_begin; b0 < p_end; b0 += kBatch2) {
-    const int nb = min(kBatch2, p_end - b0);
-    __syncthreads();  // previous batch's readers are done
-    for (int i = threadIdx.x; i < nlc; i += blockDim.x) cnt[i] = 0;
-    __syncthreads();
-    const int q = threadIdx.x;
-    int lc = 0, rank = 0;
-    if (q < nb) {
-      const int packed = rec_base[b0 + q];
-      lc = (packed & 1023) * kT2 + ((packed >> 10) & 1023);
-      rank = atomicAdd(&cnt[lc], 1);
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {  // exclusive scan of the <= 64 cell counts
-      const int i0 = 2 * lane, i1 = 2 * lane + 1;
-      const int a0 = i0 < nlc ? cnt[i0] : 0, a1 = i1 < nlc ? cnt[i1] : 0;
-      int incl = a0 + a1;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-      }
-      const int excl = incl - a0 - a1;
-      if (i0 < nlc) off[i0] = excl;
-      if (i1 < nlc) off[i1] = excl + a0;
-      if (lane == 31) off[nlc] = incl;
-    }
-    __syncthreads();
-    if (q < nb) {
-      const int pos = off[lc] + rank;
-      const int p = b0 + q;
-      const double f0 = rec_frac[p], f1 = rec_frac[n + p];
-#pragma unroll 1
-      for (int j = 0; j < NT1; ++j) {
-        const double d0 = f0 - hx0 * (double)(j - MSP);
-        const double d1 = f1 - hx1 * (double)(j - MSP);
-        wy[pos * NT1 + j] = exp(-(d0 * d0) / ft0);
-        wx[pos * NT1 + j] = exp(-(d1 * d1) / ft1);
-      }
-      for (int c = 0; c < nc; ++c) {
-        const int ch = c_begin + c;
-        const double v = (ones_channel && ch == 0) ? 1.0 : rec_val[(int64_t)(ch - ones_channel) * n + p];
-        vs[pos * nc + c] = v * scale[c];
-      }
-    }
-    __syncthreads();
-    // warp items: (tile row l0, block of GPL channel groups)
-    for (int wi = warp; wi < T0 * ngblk; wi += nwarps) {
-      const int l0 = wi / ngblk, gb = wi - l0 * ngblk;
-      const int grp = gb * GPL + gsub;
-      const bool active = lane < NT1 * GPL && grp < ngrp;
-      const int c0 = grp * kUnitCh;
-      typename Reg2<Acc>::T a[kUnitCh][NACC];
-#pragma unroll
-      for (int k = 0; k < kUnitCh; ++k)
-#pragma unroll
-        for (int j = 0; j < NACC; ++j) a[k][j] = 0;
-      const int rowbase = l0 * kT2;
-#pragma unroll
-      for (int cr = 0; cr < kT2; ++cr) {
-        const int pe = off[rowbase + cr + 1];
-#pragma unroll 1
-        for (int pp = off[rowbase + cr]; pp < pe; ++pp) {
-          const double wyv = wy[pp * NT1 + jy];
-          double v[kUnitCh];
-#pragma unroll
-          for (int k = 0; k < kUnitCh; ++k)
-            v[k] = (active && c0 + k < nc) ? wyv * vs[pp * nc + c0 + k] : 0.0;
-#pragma unroll
-          for (int jx = 0; jx < NT1; ++jx) {
-            const double w = wx[pp * NT1 + jx];
-#pragma unroll
-            for (int k = 0; k < kUnitCh; ++k) Reg2<Acc>::add(a[k][cr + jx], v[k], w);
-          }
-        }
-      }
-      if (active) {
-        // adds register j received: one per point of the cell rows cr with
-        // 0 <= j - cr < NT1
-        int rows[kT2];
-#pragma unroll
-        for (int cr = 0; cr < kT2; ++cr) rows[cr] = off[rowbase + cr + 1] - off[rowbase + cr];
-        Acc* rowp = acc + (size_t)(l0 + jy) * RS;
-#pragma unroll
-        for (int j = 0; j < NACC; ++j) {
-          int adds = 0;
-#pragma unroll
-          for (int cr = 0; cr < kT2; ++cr)
-            if (j - cr >= 0 && j - cr < NT1) adds += rows[cr];
-#pragma unroll
-          for (int k = 0; k < kUnitCh; ++k) {
-            if (c0 + k < nc) {
-              const Acc val = Reg2<Acc>::value(a[k][j], adds);
-              if (val != Acc(0)) shared_add(rowp + (size_t)(c0 + k) * CS + j, val);
-            }
-          }
-        }
-      }
-    }
-  }
-  __syncthreads();
-
-  // flush: one global atomic per non-zero cell of the tile + halo
-  const int W1 = g.W[1];
-  for (int idx = threadIdx.x; idx < nc * W0 * W1; idx += blockDim.x) {
-    const int c = idx / (W0 * W1);
-    const int r = idx - c * (W0 * W1);
-    const int r0 = r / W1, r1 = r - r0 * W1;
-    const Acc v = acc[(size_t)c * CS + r0 * RS + r1];
-    if (v == Acc(0)) continue;
-    int gc0 = (tc0 * kT2 + r0 - g.msp) % g.L[0];
-    if (gc0 < 0) gc0 += g.L[0];
-    int gc1 = (tc1 * kT2 + r1 - g.msp) % g.L[1];
-    if (gc1 < 0) gc1 += g.L[1];
-    AccOps<Acc>::add_global(&gacc[(int64_t)(c_begin + c) * g.cells + (int64_t)gc0 * g.L[1] + gc1], v);
-  }
 }
 
 // ---- 3-D path: column ownership ------------------------------------------
@@ -716,9 +905,9 @@ __device__ __forceinline__ void column_dispatch(int bz, double (&acc)[7 + NT1], 
 
 template <typename Acc, int NT1>
 __global__ void __launch_bounds__(kThreads3)
-tile_columns_3d_kernel(SpreadGeom g, int64_t n, int ones_channel, const int* __restrict__ offsets,
+tile_columns_3d_kernel(SpreadGeom g, int ones_channel, const int* __restrict__ offsets,
                        const int* __restrict__ items, const int* __restrict__ rec_base,
-                       const double* __restrict__ rec_frac, const double* __restrict__ rec_val,
+                       const double* __restrict__ rec, int stride,
                        const double* __restrict__ absum, int margin_bits,
                        Acc* __restrict__ gacc) {
   constexpr int MSP = (NT1 - 1) / 2;
@@ -740,7 +929,6 @@ tile_columns_3d_kernel(SpreadGeom g, int64_t n, int ones_channel, const int* __r
   const int p_end = min(offsets[tile + 1], p_begin + g.item_points);
   const double sc = absum ? (double)fixed_scale(absum[ch], margin_bits) : 1.0;
   const bool ones = ones_channel && ch == 0;
-  const double* vals = ones ? nullptr : rec_val + (int64_t)(ch - ones_channel) * n;
 
   const int t = threadIdx.x;
   const bool owner = t < W * W;
@@ -755,12 +943,12 @@ tile_columns_3d_kernel(SpreadGeom g, int64_t n, int ones_channel, const int* __r
       const int pp = i / PP;
       const int r = i - pp * PP;
       const int a = r / NT1, j = r - a * NT1;
-      const double fr = rec_frac[(int64_t)a * n + b0 + pp];
+      const double fr = rec[(int64_t)(b0 + pp) * stride + a];
       const double diff = fr - g.ax[a].hx * (double)(j - MSP);
       double e = fexp(-(diff * diff) / g.four_tau[a]);
       if (a == 2) {
         // last axis: times the channel value and the fixed-point scale
-        if (!ones) e = __dmul_rn(e, vals[b0 + pp]);
+        if (!ones) e = __dmul_rn(e, rec[(int64_t)(b0 + pp) * stride + 3 + ch]);
         if (sc != 1.0) e = __dmul_rn(e, sc);
       }
       s_w[i] = e;
@@ -802,10 +990,6 @@ tile_columns_3d_kernel(SpreadGeom g, int64_t n, int ones_channel, const int* __r
     if (gc2 < 0) gc2 += g.L[2];
     AccOps<Acc>::add_global(base + gc2, reg_value<Acc>(acc[z]));
   }
-}
-
-static size_t smem_2d(int W0, int nt1, int cg) {
-  return sizeof(double) * ((size_t)cg * chan_stride2(W0, nt1) + (size_t)kBatch2 * (2 * nt1 + cg));
 }
 
 // Grid value = accumulator / fixed-point scale (a power of two, so the
@@ -877,6 +1061,27 @@ static void make_geom(SpreadGeom& g, int d, const int* L, int msp, const double*
   }
 }
 
+// Points per work item, the same for the spread and for the deposits that
+// read its records.  Grids with few tiles (small 1-D grids): about four items
+// per SM.  2-D path, one warp per item: at least 24 warps' worth of items per
+// SM (two rounds of the resident ones), 256 to 1024 points.
+static void size_items(SpreadGeom& g, int64_t n, bool path2) {
+  if (path2) {
+    const int64_t per = n / (24LL * sm_count());
+    int ip = 256;
+    while (ip < per && ip < kItem2) ip <<= 1;
+    if (ip < g.item_points) g.item_points = ip;
+    return;
+  }
+  const int64_t target = 4LL * sm_count();
+  if (g.ntiles < target) {
+    const int64_t per = (n + target - 1) / target;
+    int ip = 256;
+    while (ip < per && ip < g.item_points) ip <<= 1;
+    if (ip < g.item_points) g.item_points = ip;
+  }
+}
+
 static int margin_bits_for(const SpreadGeom& g) {
   int m = 1;
   for (int a = 0; a < g.d; ++a)
@@ -895,13 +1100,6 @@ static int channel_group(const SpreadGeom& g, int nchan, size_t acc_bytes) {
   return cg;
 }
 
-static int channel_group_2d(const SpreadGeom& g, int nchan) {
-  // two CTAs per SM
-  int cg = nchan < 32 ? nchan : 32;
-  while (cg > 1 && smem_2d(g.W[0], g.ntaps1, cg) > (size_t)110 * 1024) --cg;
-  return cg;
-}
-
 struct SpreadWs {
   int* point_tile;
   int* counts;
@@ -910,23 +1108,21 @@ struct SpreadWs {
   int* cursor;
   int* rec_base;
   int* rec_idx;
-  void* rec_frac;
-  void* rec_val;
+  double* rec;
   double* absum;
   void* gacc;
 };
 
 template <typename A>
 static void spread_layout(A& ar, int d, int64_t n, int ntiles, int nchan, int64_t cells,
-                          size_t real_bytes, SpreadWs* w) {
+                          SpreadWs* w) {
   auto p0 = ar.template take<int>(n);
   auto p1 = ar.template take<int>(ntiles);
   auto p2 = ar.template take<int>(ntiles + 1);
   auto p3 = ar.template take<int>(ntiles + 1);
   auto p4 = ar.template take<int>(ntiles);
   auto p5 = ar.template take<int>(n);
-  auto p6 = ar.template take<char>((size_t)d * n * real_bytes);
-  auto p7 = ar.template take<char>((size_t)(nchan > 1 ? nchan - 1 : 1) * n * real_bytes);
+  auto p6 = ar.template take<double>((size_t)rec_stride(d, nchan) * n);
   auto p8 = ar.template take<double>(FLPR_MAX_CHANNELS);
   auto p9 = ar.template take<double>((size_t)nchan * cells);
   auto p10 = ar.template take<int>(n);
@@ -937,8 +1133,7 @@ static void spread_layout(A& ar, int d, int64_t n, int ntiles, int nchan, int64_
     w->items = (int*)p3;
     w->cursor = (int*)p4;
     w->rec_base = (int*)p5;
-    w->rec_frac = (void*)p6;
-    w->rec_val = (void*)p7;
+    w->rec = (double*)p6;
     w->absum = (double*)p8;
     w->gacc = (void*)p9;
     w->rec_idx = (int*)p10;
@@ -955,7 +1150,7 @@ struct SizeArena {
 };
 
 template <int NT1>
-static int launch_accumulate(const SpreadGeom& g, int64_t n, int nchan, int ones_channel, int cg,
+static int launch_accumulate(const SpreadGeom& g, int nchan, int cg,
                              const SpreadWs& w, bool fixed, int margin, size_t smem, dim3 grid,
                              cudaStream_t s) {
   if (fixed) {
@@ -963,50 +1158,54 @@ static int launch_accumulate(const SpreadGeom& g, int64_t n, int nchan, int ones
     FLPR_CUDA(raise_dyn_smem(k, smem));
     FLPR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
                                    cudaSharedmemCarveoutMaxShared));
-    k<<<grid, kSpreadThreads, smem, s>>>(g, n, nchan, ones_channel, cg, w.offsets, w.items,
-                                         w.rec_base, (const double*)w.rec_frac,
-                                         (const double*)w.rec_val, w.absum, margin,
+    k<<<grid, kSpreadThreads, smem, s>>>(g, nchan, cg, w.offsets, w.items, w.rec_base, w.rec,
+                                         rec_stride(g.d, nchan), w.absum, margin,
                                          (long long*)w.gacc);
   } else {
     auto k = tile_accumulate_kernel<double, double, NT1>;
     FLPR_CUDA(raise_dyn_smem(k, smem));
     FLPR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
                                    cudaSharedmemCarveoutMaxShared));
-    k<<<grid, kSpreadThreads, smem, s>>>(g, n, nchan, ones_channel, cg, w.offsets, w.items,
-                                         w.rec_base, (const double*)w.rec_frac,
-                                         (const double*)w.rec_val, nullptr, margin,
+    k<<<grid, kSpreadThreads, smem, s>>>(g, nchan, cg, w.offsets, w.items, w.rec_base, w.rec,
+                                         rec_stride(g.d, nchan), nullptr, margin,
                                          (double*)w.gacc);
   }
   FLPR_LAUNCH_CHECK();
   return FLPR_OK;
 }
 
-template <int NT1>
-static int launch_accumulate_2d(const SpreadGeom& g, int64_t n, int nchan, int ones_channel,
-                                int cg, const SpreadWs& w, bool fixed, int margin, dim3 grid,
-                                cudaStream_t s) {
-  const size_t smem = smem_2d(g.W[0], NT1, cg);
-  if (fixed) {
-    auto k = tile_accumulate_2d_kernel<long long, NT1>;
-    FLPR_CUDA(raise_dyn_smem(k, smem));
-    FLPR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                   cudaSharedmemCarveoutMaxShared));
-    k<<<grid, kBatch2, smem, s>>>(g, n, nchan, ones_channel, cg, w.offsets, w.items, w.rec_base,
-                                  (const double*)w.rec_frac, (const double*)w.rec_val, w.absum,
-                                  margin, (long long*)w.gacc);
-  } else {
-    auto k = tile_accumulate_2d_kernel<double, NT1>;
-    FLPR_CUDA(raise_dyn_smem(k, smem));
-    FLPR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                   cudaSharedmemCarveoutMaxShared));
-    k<<<grid, kBatch2, smem, s>>>(g, n, nchan, ones_channel, cg, w.offsets, w.items, w.rec_base,
-                                  (const double*)w.rec_frac, (const double*)w.rec_val, nullptr,
-                                  margin, (double*)w.gacc);
-  }
+template <typename Acc, int NT1, int UC, int NW>
+static int launch_2d_k(const SpreadGeom& g, int nchan, const SpreadWs& w, const double* absum,
+                       int margin, int64_t max_items, cudaStream_t s) {
+  auto k = tile_accumulate_2d_kernel<Acc, NT1, UC, NW>;
+  FLPR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 cudaSharedmemCarveoutMaxShared));
+  constexpr int NCB = Stage2<NT1, UC, NW>::NCB;
+  k<<<dim3((unsigned)max_items, (unsigned)((nchan + NCB - 1) / NCB)), 32 * NW, 0, s>>>(
+      g, nchan, w.offsets, w.items, w.rec_base, w.rec, rec_stride(2, nchan), absum, margin,
+      (Acc*)w.gacc);
   FLPR_LAUNCH_CHECK();
   return FLPR_OK;
 }
 
+// Channels per lane and warps per item: the channels spread over the lane
+// groups of one warp while that needs at most three per lane, else of two
+// warps, which share the sort, the records and (one axis each) the weights.
+template <int NT1>
+static int launch_accumulate_2d(const SpreadGeom& g, int nchan, const SpreadWs& w, bool fixed,
+                                int margin, int64_t max_items, cudaStream_t s) {
+  constexpr int GPL = groups2(NT1);
+  const int uc = (nchan + GPL - 1) / GPL;
+#define FLPR_UC2(U, N)                                                                         \
+  return fixed ? launch_2d_k<long long, NT1, U, N>(g, nchan, w, w.absum, margin, max_items, s) \
+               : launch_2d_k<double, NT1, U, N>(g, nchan, w, nullptr, margin, max_items, s);
+  if (uc <= 1) FLPR_UC2(1, 1)
+  if (uc == 2) FLPR_UC2(2, 1)
+  if (uc == 3) FLPR_UC2(3, 1)
+  if (uc == 4) FLPR_UC2(2, 2)
+  FLPR_UC2(3, 2)
+#undef FLPR_UC2
+}
 
 // The column kernel covers 3-D tiles of 8^3 with at most 9 taps per axis
 // (halo columns fit one CTA of 256 threads).
@@ -1018,24 +1217,21 @@ static bool use_3d_columns(const SpreadGeom& g) {
 }
 
 template <int NT1>
-static int launch_columns_3d(const SpreadGeom& g, int64_t n, int nchan, int ones_channel,
+static int launch_columns_3d(const SpreadGeom& g, int nchan, int ones_channel,
                              const SpreadWs& w, bool fixed, int margin, dim3 grid,
                              cudaStream_t s) {
   const size_t smem = smem_3d(NT1);
   if (fixed) {
     auto k = tile_columns_3d_kernel<long long, NT1>;
     FLPR_CUDA(raise_dyn_smem(k, smem));
-    k<<<grid, kThreads3, smem, s>>>(g, n, ones_channel, w.offsets, w.items, w.rec_base,
-                                    (const double*)w.rec_frac, (const double*)w.rec_val, w.absum,
-                                    margin, (long long*)w.gacc);
+    k<<<grid, kThreads3, smem, s>>>(g, ones_channel, w.offsets, w.items, w.rec_base, w.rec,
+                                    rec_stride(3, nchan), w.absum, margin, (long long*)w.gacc);
   } else {
     auto k = tile_columns_3d_kernel<double, NT1>;
     FLPR_CUDA(raise_dyn_smem(k, smem));
-    k<<<grid, kThreads3, smem, s>>>(g, n, ones_channel, w.offsets, w.items, w.rec_base,
-                                    (const double*)w.rec_frac, (const double*)w.rec_val, nullptr,
-                                    margin, (double*)w.gacc);
+    k<<<grid, kThreads3, smem, s>>>(g, ones_channel, w.offsets, w.items, w.rec_base, w.rec,
+                                    rec_stride(3, nchan), nullptr, margin, (double*)w.gacc);
   }
-  (void)nchan;
   FLPR_LAUNCH_CHECK();
   return FLPR_OK;
 }
@@ -1055,7 +1251,7 @@ size_t flpr_spread_ws(int d, int64_t n, const int* h_L, int msp, int nchan, int 
   double tau[3] = {1, 1, 1}, kmap[27] = {0};
   make_geom(g, d, h_L, msp, tau, kmap);
   SizeArena ar;
-  spread_layout(ar, d, n, g.ntiles, nchan, g.cells, 8, nullptr);
+  spread_layout(ar, d, n, g.ntiles, nchan, g.cells, nullptr);
   return ar.used;
 }
 
@@ -1079,25 +1275,15 @@ static int spread_impl(int d, int64_t n, const double* d_x, const double* h_kmap
   cudaStream_t s = as_stream(stream);
   SpreadGeom g;
   make_geom(g, d, h_L, msp, h_tau, h_kmap);
-  {
-    // few tiles (small 1-D grids): smaller work items, about four per SM
-    const int64_t target = 4LL * sm_count();
-    if (g.ntiles < target) {
-      const int64_t per = (n + target - 1) / target;
-      int ip = 256;
-      while (ip < per && ip < g.item_points) ip <<= 1;
-      if (ip < g.item_points) g.item_points = ip;
-    }
-  }
+  size_items(g, n, use_2d_path(d, h_L, msp));
   ChanPtrs cp;
   memset(&cp, 0, sizeof(cp));
   for (int c = 0; c < nchan - ones_channel; ++c) cp.col[c] = h_cols[c];
   Arena ar(d_ws, ws_bytes);
   SpreadWs w;
   const bool fixed = (prec == FLPR_PREC_F32);
-  spread_layout(ar, d, n, g.ntiles, nchan, g.cells, 8, &w);
+  spread_layout(ar, d, n, g.ntiles, nchan, g.cells, &w);
   const int margin = margin_bits_for(g);
-  const int nv = nchan - ones_channel;
   FLPR_CUDA(cudaMemsetAsync(w.counts, 0, sizeof(int) * g.ntiles, s));
   FLPR_CUDA(cudaMemsetAsync(w.absum, 0, sizeof(double) * FLPR_MAX_CHANNELS, s));
   FLPR_CUDA(cudaMemsetAsync(w.gacc, 0, sizeof(double) * (size_t)nchan * g.cells, s));
@@ -1119,25 +1305,21 @@ static int spread_impl(int d, int64_t n, const double* d_x, const double* h_kmap
   // slot its cursor atomic returns, so more of them in flight hide it
   int nbs = (int)((n + 255) / 256);
   if (nbs > 32 * sm_count()) nbs = 32 * sm_count();
-  bin_scatter_kernel<double><<<nbs, 256, 0, s>>>(g, n, d_x, d_kmap, w.offsets, w.cursor, nv, cp,
-                                                w.rec_base, w.rec_idx, (double*)w.rec_frac,
-                                                (double*)w.rec_val);
+  bin_scatter_kernel<<<nbs, 256, 0, s>>>(g, n, d_x, d_kmap, w.offsets, w.cursor, nchan,
+                                         ones_channel, cp, w.rec_base, w.rec_idx, w.rec);
   FLPR_LAUNCH_CHECK();
 
   int64_t max_items = (int64_t)g.ntiles + (n + g.item_points - 1) / g.item_points;
   if (use_2d_path(d, h_L, msp)) {
-    const int cg2 = channel_group_2d(g, nchan);
-    FLPR_CHECK_ARG(cg2 >= 1, "spread: tile does not fit shared memory");
-    dim3 grid2((unsigned)max_items, (unsigned)((nchan + cg2 - 1) / cg2));
     int st = FLPR_OK;
     switch (g.ntaps1) {
-      case 1: st = launch_accumulate_2d<1>(g, n, nchan, ones_channel, cg2, w, fixed, margin, grid2, s); break;
-      case 3: st = launch_accumulate_2d<3>(g, n, nchan, ones_channel, cg2, w, fixed, margin, grid2, s); break;
-      case 5: st = launch_accumulate_2d<5>(g, n, nchan, ones_channel, cg2, w, fixed, margin, grid2, s); break;
-      case 7: st = launch_accumulate_2d<7>(g, n, nchan, ones_channel, cg2, w, fixed, margin, grid2, s); break;
-      case 9: st = launch_accumulate_2d<9>(g, n, nchan, ones_channel, cg2, w, fixed, margin, grid2, s); break;
-      case 11: st = launch_accumulate_2d<11>(g, n, nchan, ones_channel, cg2, w, fixed, margin, grid2, s); break;
-      case 13: st = launch_accumulate_2d<13>(g, n, nchan, ones_channel, cg2, w, fixed, margin, grid2, s); break;
+      case 1: st = launch_accumulate_2d<1>(g, nchan, w, fixed, margin, max_items, s); break;
+      case 3: st = launch_accumulate_2d<3>(g, nchan, w, fixed, margin, max_items, s); break;
+      case 5: st = launch_accumulate_2d<5>(g, nchan, w, fixed, margin, max_items, s); break;
+      case 7: st = launch_accumulate_2d<7>(g, nchan, w, fixed, margin, max_items, s); break;
+      case 9: st = launch_accumulate_2d<9>(g, nchan, w, fixed, margin, max_items, s); break;
+      case 11: st = launch_accumulate_2d<11>(g, nchan, w, fixed, margin, max_items, s); break;
+      case 13: st = launch_accumulate_2d<13>(g, nchan, w, fixed, margin, max_items, s); break;
       default: set_error("spread: msp=%d not supported (0..12)", g.msp); return FLPR_ERR_ARG;
     }
     if (st != FLPR_OK) return st;
@@ -1147,11 +1329,11 @@ static int spread_impl(int d, int64_t n, const double* d_x, const double* h_kmap
     dim3 grid3((unsigned)max_items, (unsigned)nchan);
     int st = FLPR_OK;
     switch (g.ntaps1) {
-      case 1: st = launch_columns_3d<1>(g, n, nchan, ones_channel, w, fixed, margin, grid3, s); break;
-      case 3: st = launch_columns_3d<3>(g, n, nchan, ones_channel, w, fixed, margin, grid3, s); break;
-      case 5: st = launch_columns_3d<5>(g, n, nchan, ones_channel, w, fixed, margin, grid3, s); break;
-      case 7: st = launch_columns_3d<7>(g, n, nchan, ones_channel, w, fixed, margin, grid3, s); break;
-      case 9: st = launch_columns_3d<9>(g, n, nchan, ones_channel, w, fixed, margin, grid3, s); break;
+      case 1: st = launch_columns_3d<1>(g, nchan, ones_channel, w, fixed, margin, grid3, s); break;
+      case 3: st = launch_columns_3d<3>(g, nchan, ones_channel, w, fixed, margin, grid3, s); break;
+      case 5: st = launch_columns_3d<5>(g, nchan, ones_channel, w, fixed, margin, grid3, s); break;
+      case 7: st = launch_columns_3d<7>(g, nchan, ones_channel, w, fixed, margin, grid3, s); break;
+      case 9: st = launch_columns_3d<9>(g, nchan, ones_channel, w, fixed, margin, grid3, s); break;
       default: set_error("spread: msp=%d not supported by the 3-D path", g.msp); return FLPR_ERR_ARG;
     }
     if (st != FLPR_OK) return st;
@@ -1165,19 +1347,19 @@ static int spread_impl(int d, int64_t n, const double* d_x, const double* h_kmap
   dim3 grid((unsigned)max_items, (unsigned)ngroups);
   int status = FLPR_OK;
   switch (g.ntaps1) {
-    case 1: status = launch_accumulate<1>(g, n, nchan, ones_channel, cg, w, fixed, margin, smem, grid, s); break;
-    case 3: status = launch_accumulate<3>(g, n, nchan, ones_channel, cg, w, fixed, margin, smem, grid, s); break;
-    case 5: status = launch_accumulate<5>(g, n, nchan, ones_channel, cg, w, fixed, margin, smem, grid, s); break;
-    case 7: status = launch_accumulate<7>(g, n, nchan, ones_channel, cg, w, fixed, margin, smem, grid, s); break;
-    case 9: status = launch_accumulate<9>(g, n, nchan, ones_channel, cg, w, fixed, margin, smem, grid, s); break;
-    case 11: status = launch_accumulate<11>(g, n, nchan, ones_channel, cg, w, fixed, margin, smem, grid, s); break;
-    case 13: status = launch_accumulate<13>(g, n, nchan, ones_channel, cg, w, fixed, margin, smem, grid, s); break;
-    case 15: status = launch_accumulate<15>(g, n, nchan, ones_channel, cg, w, fixed, margin, smem, grid, s); break;
-    case 17: status = launch_accumulate<17>(g, n, nchan, ones_channel, cg, w, fixed, margin, smem, grid, s); break;
-    case 19: status = launch_accumulate<19>(g, n, nchan, ones_channel, cg, w, fixed, margin, smem, grid, s); break;
-    case 21: status = launch_accumulate<21>(g, n, nchan, ones_channel, cg, w, fixed, margin, smem, grid, s); break;
-    case 23: status = launch_accumulate<23>(g, n, nchan, ones_channel, cg, w, fixed, margin, smem, grid, s); break;
-    case 25: status = launch_accumulate<25>(g, n, nchan, ones_channel, cg, w, fixed, margin, smem, grid, s); break;
+    case 1: status = launch_accumulate<1>(g, nchan, cg, w, fixed, margin, smem, grid, s); break;
+    case 3: status = launch_accumulate<3>(g, nchan, cg, w, fixed, margin, smem, grid, s); break;
+    case 5: status = launch_accumulate<5>(g, nchan, cg, w, fixed, margin, smem, grid, s); break;
+    case 7: status = launch_accumulate<7>(g, nchan, cg, w, fixed, margin, smem, grid, s); break;
+    case 9: status = launch_accumulate<9>(g, nchan, cg, w, fixed, margin, smem, grid, s); break;
+    case 11: status = launch_accumulate<11>(g, nchan, cg, w, fixed, margin, smem, grid, s); break;
+    case 13: status = launch_accumulate<13>(g, nchan, cg, w, fixed, margin, smem, grid, s); break;
+    case 15: status = launch_accumulate<15>(g, nchan, cg, w, fixed, margin, smem, grid, s); break;
+    case 17: status = launch_accumulate<17>(g, nchan, cg, w, fixed, margin, smem, grid, s); break;
+    case 19: status = launch_accumulate<19>(g, nchan, cg, w, fixed, margin, smem, grid, s); break;
+    case 21: status = launch_accumulate<21>(g, nchan, cg, w, fixed, margin, smem, grid, s); break;
+    case 23: status = launch_accumulate<23>(g, nchan, cg, w, fixed, margin, smem, grid, s); break;
+    case 25: status = launch_accumulate<25>(g, nchan, cg, w, fixed, margin, smem, grid, s); break;
     default: set_error("spread: msp=%d not supported (0..12)", g.msp); return FLPR_ERR_ARG;
   }
   if (status != FLPR_OK) return status;
@@ -1228,7 +1410,7 @@ int flpr_spread_grid64_channels(int d, int64_t n, const int* h_L, int msp, int n
   make_geom(g, d, h_L, msp, tau, kmap);
   Arena ar(const_cast<void*>(d_ws), ws_bytes);
   SpreadWs w;
-  spread_layout(ar, d, n, g.ntiles, nchan, g.cells, 8, &w);
+  spread_layout(ar, d, n, g.ntiles, nchan, g.cells, &w);
   int64_t fb64 = (g.cells + 255) / 256;
   if (fb64 > 16 * sm_count()) fb64 = 16 * sm_count();
   finalize_kernel<long long, double, true><<<(int)fb64, 256, 0, as_stream(stream)>>>(
@@ -1320,14 +1502,14 @@ template <int D>
 __global__ void __launch_bounds__(kDepThreads)
 tile_deposit_kernel(SpreadGeom g, DepositGeom dg, int64_t n, const double* __restrict__ x,
                     const int* __restrict__ offsets, const int* __restrict__ items,
-                    const int* __restrict__ rec_idx, const double* __restrict__ rec_val,
+                    const int* __restrict__ rec_idx, const double* __restrict__ rec, int stride,
                     const double* __restrict__ absum, unsigned long long* __restrict__ qacc,
                     unsigned long long* __restrict__ bacc) {
   constexpr int NC = 1 << D;
   constexpr int NP = dep_pairs(D);
   extern __shared__ __align__(16) unsigned long long sacc[];  // window cells x (C + NP)
   __shared__ double s_scale[kDepMaxChan + 1];
-  const int C = dg.C, stride = C + NP;
+  const int C = dg.C, wst = C + NP;
   const int W0 = dg.win[0], W1 = D == 2 ? dg.win[1] : 1;
   const int item = blockIdx.x;
   if (item >= items[g.ntiles]) return;
@@ -1356,7 +1538,7 @@ tile_deposit_kernel(SpreadGeom g, DepositGeom dg, int64_t n, const double* __res
       org[a] = j - kDepHalo;
     }
   }
-  for (int i = threadIdx.x; i < W0 * W1 * stride; i += kDepThreads) sacc[i] = 0ull;
+  for (int i = threadIdx.x; i < W0 * W1 * wst; i += kDepThreads) sacc[i] = 0ull;
   if (threadIdx.x < C) s_scale[threadIdx.x] = dep_scale(absum[dg.ones + threadIdx.x], 0);
   if (threadIdx.x == 0) s_scale[C] = dep_scale((double)n, 1);  // pair weights: sum <= n
   __syncthreads();
@@ -1415,13 +1597,13 @@ tile_deposit_kernel(SpreadGeom g, DepositGeom dg, int64_t n, const double* __res
       const double* w = s_w + t * NC;
       const int* cell = s_cell + t * NC;
       if (c < C) {
-        const double vs = rec_val[(int64_t)c * n + b0 + t] * s_scale[c];
+        const double vs = rec[(int64_t)(b0 + t) * stride + D + dg.ones + c] * s_scale[c];
 #pragma unroll
         for (int k = 0; k < NC; ++k) {
           const long long q = __double2ll_rn(w[k] * vs);
           if (q == 0) continue;
           if (cell[k] >= 0)
-            atomicAdd(&sacc[cell[k] * stride + c], (unsigned long long)q);
+            atomicAdd(&sacc[cell[k] * wst + c], (unsigned long long)q);
           else
             atomicAdd(&qacc[(int64_t)(-1 - cell[k]) * C + c], (unsigned long long)q);
         }
@@ -1435,7 +1617,7 @@ tile_deposit_kernel(SpreadGeom g, DepositGeom dg, int64_t n, const double* __res
                 __double2ll_rn((k == k2 ? 1.0 : 2.0) * w[k] * w[k2] * s_scale[C]);
             if (q == 0) continue;
             if (cell[0] >= 0)
-              atomicAdd(&sacc[cell[0] * stride + C + pr], (unsigned long long)q);
+              atomicAdd(&sacc[cell[0] * wst + C + pr], (unsigned long long)q);
             else
               atomicAdd(&bacc[(int64_t)(-1 - cell[0]) * NP + pr], (unsigned long long)q);
           }
@@ -1446,10 +1628,10 @@ tile_deposit_kernel(SpreadGeom g, DepositGeom dg, int64_t n, const double* __res
   }
   __syncthreads();
   // window -> global sums, one atomic per non-zero entry
-  for (int e = threadIdx.x; e < W0 * W1 * stride; e += kDepThreads) {
+  for (int e = threadIdx.x; e < W0 * W1 * wst; e += kDepThreads) {
     const unsigned long long v = sacc[e];
     if (v == 0ull) continue;
-    const int cell = e / stride, j = e - cell * stride;
+    const int cell = e / wst, j = e - cell * wst;
     const int l0 = D == 2 ? cell / W1 : cell, l1 = D == 2 ? cell - l0 * W1 : 0;
     const int g0 = org[0] + l0, g1 = org[1] + l1;
     if (g0 < 0 || g0 >= dg.G[0] || (D == 2 && (g1 < 0 || g1 >= dg.G[1]))) continue;  // stays 0
@@ -1563,19 +1745,10 @@ int flpr_deposit_sorted(int d, int64_t n, const double* d_x, const int* h_L, int
   SpreadGeom g;
   double tau[3] = {1, 1, 1}, kmap[27] = {0};
   make_geom(g, d, h_L, msp, tau, kmap);
-  {
-    // the work items the spread used (it shrinks them on grids with few tiles)
-    const int64_t target = 4LL * sm_count();
-    if (g.ntiles < target) {
-      const int64_t per = (n + target - 1) / target;
-      int ip = 256;
-      while (ip < per && ip < g.item_points) ip <<= 1;
-      if (ip < g.item_points) g.item_points = ip;
-    }
-  }
+  size_items(g, n, use_2d_path(d, h_L, msp));  // the work items the spread used
   Arena ar(const_cast<void*>(d_spread_ws), spread_ws_bytes);
   SpreadWs w;
-  spread_layout(ar, d, n, g.ntiles, nchan, g.cells, 8, &w);
+  spread_layout(ar, d, n, g.ntiles, nchan, g.cells, &w);
   DepositGeom dg;
   memset(&dg, 0, sizeof(dg));
   int64_t M = 1;
@@ -1604,13 +1777,13 @@ int flpr_deposit_sorted(int d, int64_t n, const double* d_x, const int* h_L, int
     auto k = tile_deposit_kernel<2>;
     FLPR_CUDA(raise_dyn_smem(k, smem));
     k<<<(unsigned)nitems, kDepThreads, smem, s>>>(
-        g, dg, n, d_x, w.offsets, w.items, w.rec_idx, (const double*)w.rec_val, w.absum,
+        g, dg, n, d_x, w.offsets, w.items, w.rec_idx, w.rec, rec_stride(d, nchan), w.absum,
         reinterpret_cast<unsigned long long*>(d_Q), reinterpret_cast<unsigned long long*>(d_B));
   } else {
     auto k = tile_deposit_kernel<1>;
     FLPR_CUDA(raise_dyn_smem(k, smem));
     k<<<(unsigned)nitems, kDepThreads, smem, s>>>(
-        g, dg, n, d_x, w.offsets, w.items, w.rec_idx, (const double*)w.rec_val, w.absum,
+        g, dg, n, d_x, w.offsets, w.items, w.rec_idx, w.rec, rec_stride(d, nchan), w.absum,
         reinterpret_cast<unsigned long long*>(d_Q), reinterpret_cast<unsigned long long*>(d_B));
   }
   FLPR_LAUNCH_CHECK();
