@@ -7,12 +7,12 @@
 //   2. tile_scan   : exclusive scans of the histogram and of the number of
 //                    work items per tile (a tile is split into chunks of at
 //                    most FLPR_TUNE_SPREAD_ITEM_POINTS points).
-//   3. bin_scatter : point indices sorted by tile.
-//   4. tile_accumulate : one CTA per work item; every point of the chunk is
-//                    spread into a shared-memory copy of its tile plus a
-//                    halo of msp cells (one warp per point, lanes over taps),
-//                    then the tile is added to the global accumulator with
-//                    one atomic per non-zero cell.
+//   3. bin_scatter : one contiguous record per point, in tile order.
+//   4. accumulate  : every work item is spread into a copy of its tile plus a
+//                    halo of msp cells, in registers (2-D and 3-D) or in
+//                    shared memory (1-D, wide stencils, tiny grids), which
+//                    is then added to the global accumulator with one atomic
+//                    per non-zero cell.
 //   5. finalize    : accumulator -> real grid (float or double) times 1/n.
 //
 // FLPR_PREC_F32 accumulates 64-bit fixed point: integer addition is
@@ -127,7 +127,7 @@ __global__ void knot_map_kernel(int d, double nm1, const double* __restrict__ st
 
 __global__ void bin_count_kernel(SpreadGeom g, int64_t n, const double* __restrict__ x,
                                  const double* __restrict__ d_kmap,
-                                 int* __restrict__ point_tile_out, int* __restrict__ counts,
+                                 int* __restrict__ counts,
                                  int nchan, int ones_channel, ChanPtrs cp,
                                  double* __restrict__ absum) {
   __shared__ double sh_abs[FLPR_MAX_CHANNELS];
@@ -140,7 +140,6 @@ __global__ void bin_count_kernel(SpreadGeom g, int64_t n, const double* __restri
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     int t = point_tile(g, s_ax, x, i, nullptr, nullptr);
-    point_tile_out[i] = t;
     atomicAdd(&counts[t], 1);
   }
   if (absum != nullptr) {
@@ -168,72 +167,108 @@ __global__ void bin_count_kernel(SpreadGeom g, int64_t n, const double* __restri
   }
 }
 
-// Single-block exclusive scans over the tile histogram (points and work
-// items per tile): per 1024-tile chunk a warp-shuffle scan, the warp totals
-// scanned by warp 0, and a running carry.  Launched with 1024 threads.
-__global__ void tile_scan_kernel(int ntiles, int item_points, const int* __restrict__ counts,
-                                 int* __restrict__ offsets, int* __restrict__ items,
-                                 int* __restrict__ cursor) {
+// Exclusive scans over the tile histogram (points and work items per tile) in
+// two launches: blocks of kScanTiles tiles scan their own counts (four tiles
+// per thread, warp shuffles, the warp totals scanned by warp 0) and leave
+// their totals, then every block adds the totals before it.  One block alone
+// took 1.4 us per 1024 tiles, 22 us for a 2-D grid and 350 us for a 3-D grid
+// of 256^3 in its one-cell slabs.  A histogram of one block needs one launch.
+constexpr int kScanTiles = 4096;
+
+__global__ void __launch_bounds__(1024)
+tile_scan_kernel(int ntiles, int item_points, const int* __restrict__ counts,
+                 int* __restrict__ offsets, int* __restrict__ items, int* __restrict__ cursor,
+                 int2* __restrict__ totals) {
   __shared__ int wa[32], wb[32];
-  __shared__ int carry_a, carry_b;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) {
-    carry_a = 0;
-    carry_b = 0;
+  const int t0 = blockIdx.x * kScanTiles + 4 * threadIdx.x;
+  int a[4], b[4], sa = 0, sb = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int c = t0 + k < ntiles ? counts[t0 + k] : 0;
+    a[k] = sa;
+    b[k] = sb;
+    sa += c;
+    sb += (c + item_points - 1) / item_points;
+  }
+  int ia = sa, ib = sb;  // inclusive warp scans
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int va = __shfl_up_sync(0xffffffffu, ia, o);
+    const int vb = __shfl_up_sync(0xffffffffu, ib, o);
+    if (lane >= o) {
+      ia += va;
+      ib += vb;
+    }
+  }
+  if (lane == 31) {
+    wa[warp] = ia;
+    wb[warp] = ib;
   }
   __syncthreads();
-  for (int base = 0; base < ntiles; base += blockDim.x) {
-    const int t = base + threadIdx.x;
-    const int c = t < ntiles ? counts[t] : 0;
-    const int a = c;
-    const int b = (c + item_points - 1) / item_points;
-    int ia = a, ib = b;  // inclusive warp scans
+  if (warp == 0) {
+    int xa = wa[lane], xb = wb[lane];  // 32 warps
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int va = __shfl_up_sync(0xffffffffu, ia, o);
-      const int vb = __shfl_up_sync(0xffffffffu, ib, o);
+      const int va = __shfl_up_sync(0xffffffffu, xa, o);
+      const int vb = __shfl_up_sync(0xffffffffu, xb, o);
       if (lane >= o) {
-        ia += va;
-        ib += vb;
+        xa += va;
+        xb += vb;
       }
     }
-    if (lane == 31) {
-      wa[warp] = ia;
-      wb[warp] = ib;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      int xa = wa[lane], xb = wb[lane];  // 32 warps of 32 threads
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int va = __shfl_up_sync(0xffffffffu, xa, o);
-        const int vb = __shfl_up_sync(0xffffffffu, xb, o);
-        if (lane >= o) {
-          xa += va;
-          xb += vb;
-        }
-      }
-      wa[lane] = xa;  // inclusive warp totals
-      wb[lane] = xb;
-    }
-    __syncthreads();
-    const int pa = carry_a + (warp ? wa[warp - 1] : 0) + ia - a;
-    const int pb = carry_b + (warp ? wb[warp - 1] : 0) + ib - b;
-    if (t < ntiles) {
-      offsets[t] = pa;
-      items[t] = pb;
-      cursor[t] = 0;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      carry_a += wa[31];
-      carry_b += wb[31];
-    }
-    __syncthreads();
+    wa[lane] = xa;  // inclusive warp totals
+    wb[lane] = xb;
   }
+  __syncthreads();
+  const int pa = (warp ? wa[warp - 1] : 0) + ia - sa, pb = (warp ? wb[warp - 1] : 0) + ib - sb;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (t0 + k < ntiles) {
+      offsets[t0 + k] = pa + a[k];
+      items[t0 + k] = pb + b[k];
+      cursor[t0 + k] = 0;
+    }
   if (threadIdx.x == 0) {
-    offsets[ntiles] = carry_a;
-    items[ntiles] = carry_b;
+    totals[blockIdx.x] = make_int2(wa[31], wb[31]);
+    if (gridDim.x == 1) {
+      offsets[ntiles] = wa[31];
+      items[ntiles] = wb[31];
+    }
+  }
+}
+
+__global__ void __launch_bounds__(1024)
+tile_scan_add_kernel(int ntiles, const int2* __restrict__ totals, int* __restrict__ offsets,
+                     int* __restrict__ items) {
+  __shared__ int s_a, s_b;
+  if (threadIdx.x == 0) s_a = s_b = 0;
+  __syncthreads();
+  int sa = 0, sb = 0;
+  for (int k = threadIdx.x; k < (int)blockIdx.x; k += blockDim.x) {
+    sa += totals[k].x;
+    sb += totals[k].y;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    sa += __shfl_xor_sync(0xffffffffu, sa, o);
+    sb += __shfl_xor_sync(0xffffffffu, sb, o);
+  }
+  if ((threadIdx.x & 31) == 0 && (sa | sb)) {
+    atomicAdd(&s_a, sa);
+    atomicAdd(&s_b, sb);
+  }
+  __syncthreads();
+  const int pa = s_a, pb = s_b;
+  for (int k = threadIdx.x; k < kScanTiles; k += blockDim.x) {
+    const int t = blockIdx.x * kScanTiles + k;
+    if (t < ntiles) {
+      offsets[t] += pa;
+      items[t] += pb;
+    }
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    offsets[ntiles] = pa + totals[blockIdx.x].x;
+    items[ntiles] = pb + totals[blockIdx.x].y;
   }
 }
 
@@ -468,8 +503,8 @@ tile_accumulate_kernel(SpreadGeom g, int nchan, int cgroup,
   }
 }
 
-// ---- 2-D path: one or two warps per work item -------------------------------
-// Tiles of 8 x 8 cells.  The warps of a CTA (one, or two that split the
+// ---- 2-D and 3-D path: one or two warps per work item ------------------------
+// Tiles of 8 x 8 cells of the last two axes.  The warps of a CTA (one, or two that split the
 // channels) take the points of one work item: they sort them by cell
 // (counting sort of their indices), then walk them row of cells by row of
 // cells, 32 points at a time staged in shared memory (per-axis tap weights
@@ -483,10 +518,20 @@ tile_accumulate_kernel(SpreadGeom g, int nchan, int cgroup,
 // accumulator every product is rounded to an integer as it is added, so sums
 // are exact and the grid does not depend on the order of the points.
 //
+// In 3-D a tile is one cell thick on the first axis, and the NT1 taps of that
+// axis take the place of the channels: tap plane j of a point has the value
+// e0[j] v, and a warp takes one channel (27 lanes, three planes each, for 9
+// taps).  A point so costs 30 multiply-adds per lane where a thread for each
+// halo column of an 8 x 8 x 8 tile, rounding every product by two additions,
+// took 37 operations and left more than half of its lanes idle.
+//
 // Bound by the FP64 pipe (UC (NT1 + 1) multiply-adds per point and warp,
 // about 2.2 cycles each) and by latency: the multiply-add takes 23 cycles,
 // so the next point's values are read and scaled beside this point's sums,
 // and UC stays at 3 or less, which leaves registers for 12 to 16 warps.
+// Measured: 1e6 points, 12 channels, grid 512^2: 527 -> 220 us (UC = 4 in one
+// warp: 266 us; the multiply-adds alone: 90 us); 1e7 points, one channel,
+// grid 128^3: 7.63 -> 1.90 ms.
 constexpr int kT2 = 8;            // tile edge of the 2-D path
 constexpr int kItem2 = 1024;      // most points of a work item
 
@@ -524,13 +569,13 @@ struct RegSum<double> {
 
 // Tap weights of one axis from the knot's offset f to its cell:
 // exp(-(f - hx j)^2 / ft) = exp(-f^2 / ft) r^j C_|j|, r = exp(2 f hx / ft),
-// C_j = exp(-(hx j)^2 / ft), for j = -MSP .. MSP into w (two exponentials
+// C_j = exp(-(hx j)^2 / ft), times val for j = -MSP .. MSP into w (two exponentials
 // and one reciprocal per axis instead of an exponential and a division per tap).
 template <int NT1>
-__device__ __forceinline__ void tap_weights(double f, double hx, double inv_ft,
+__device__ __forceinline__ void tap_weights(double f, double val, double hx, double inv_ft,
                                             const double* __restrict__ cj, double* __restrict__ w) {
   constexpr int MSP = (NT1 - 1) / 2;
-  const double e0 = exp(-(f * f) * inv_ft);
+  const double e0 = val * exp(-(f * f) * inv_ft);
   w[MSP] = e0;
   if constexpr (MSP > 0) {
     const double b = 2.0 * f * hx * inv_ft;
@@ -563,9 +608,13 @@ __device__ __forceinline__ int item_tile(const int* __restrict__ items, int ntil
   return lo;
 }
 
-__device__ __forceinline__ void copy16_async(double* dst, const double* src) {
+template <int BYTES>
+__device__ __forceinline__ void copy_async(double* dst, const double* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
 }
 __device__ __forceinline__ void copies_wait() {
   asm volatile("cp.async.wait_all;" ::: "memory");
@@ -581,20 +630,24 @@ __host__ __device__ constexpr int warps2(int nt1, int uc) {
 }
 
 // Shared memory of one CTA.  The rows that the lanes still hold at the end
-// go through the space of the staged points.
-template <int NT1, int UC, int NW>
+// go through the space of the staged points.  A warp's NCW "channels" are its
+// value channels in 2-D and the tap planes of its one channel in 3-D.
+template <int D, int NT1, int UC, int NW>
 struct Stage2 {
   static constexpr int W = kT2 + NT1 - 1;     // halo cells per axis
   static constexpr int GPL = groups2(NT1);    // channel groups of a warp
   static constexpr int NCW = UC * GPL;        // channels of a warp
   static constexpr int NCB = NCW * NW;        // channels of the CTA
-  static constexpr int WXS = (NT1 + 1) & ~1;  // even row stride: two axis-1 weights per load
-  static constexpr int RS = (2 + NCB + 1) & ~1;  // staged record: 2 knot offsets, the values
+  static constexpr int NVB = D == 2 ? NCB : NW;  // value channels of the CTA
+  static constexpr int WXS = (NT1 + 1) & ~1;  // even row stride: two weights per load
+  static constexpr int RS = D == 2 ? (2 + NVB + 1) & ~1 : 3 + NVB;  // staged record
+  static constexpr int VS = D == 2 ? RS : NCB;  // stride of the values the lanes read
   static constexpr int WR = W | 1;            // row-buffer stride of one channel
   struct Points {
     double rec[2][33 * RS];  // records of this batch and of the next (and one read ahead)
-    double wx[32 * WXS];
-    double wy[33 * NT1];
+    double wx[32 * WXS];     // weights of the last axis
+    double wy[33 * NT1];     // weights of the axis before it
+    double val[D == 3 ? 33 * VS : 1];  // 3-D: axis-0 weights times the channels' values
     double row[NCB * WR];
     unsigned short order[kItem2];
     unsigned char cell[kItem2];
@@ -603,36 +656,39 @@ struct Stage2 {
     Points st;
     double rows[NT1 * NCB * WR];
   };
-  double scale[NCB], zero[NCB];
-  double cj[2][(NT1 - 1) / 2 + 1];
+  double scale[NVB], zero[NVB];
+  double cj[D][(NT1 - 1) / 2 + 1];
   int off[kT2 * kT2 + 1];
   int cur[kT2 * kT2];
   int col[W];  // grid columns of the halo
+  int64_t plane[D == 3 ? NT1 : 1];  // 3-D: start of the grid planes of the tap planes
 };
 
 // Adds `nrows` halo rows from grid row gr0 on, (rows, NCW, WR) registers of
-// one warp's lanes for its channels c_w .. c_w + nc of the CTA's, to the
-// global accumulator: one atomic per non-zero cell.
-template <typename Acc, typename S>
+// one warp's lanes for its first nc channels, to the global accumulator: one
+// atomic per non-zero cell.  v_w: its first value channel in the CTA.
+template <typename Acc, int D, typename S>
 __device__ __forceinline__ void add_rows(const SpreadGeom& g, const S& sh, const double* buf,
-                                         int nrows, int gr0, int c_begin, int c_w, int nc,
+                                         int nrows, int gr0, int c_begin, int v_w, int nc,
                                          int lane, Acc* __restrict__ gacc) {
   constexpr int W = S::W, N = S::NCW * W, U = (N + 31) / 32;
+  const int Lr = g.L[D - 2], Lc = g.L[D - 1];
   for (int r = 0; r < nrows; ++r) {
-    int gr = (gr0 + r) % g.L[0];
-    if (gr < 0) gr += g.L[0];
-    Acc* grow = gacc + (int64_t)(c_begin + c_w) * g.cells + (int64_t)gr * g.L[1];
+    int gr = (gr0 + r) % Lr;
+    if (gr < 0) gr += Lr;
+    Acc* grow = gacc + (int64_t)(c_begin + v_w) * g.cells + (int64_t)gr * Lc;
     const double* rb = buf + r * S::NCW * S::WR;
     Acc v[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int idx = u * 32 + lane, c = idx / W, j = idx - c * W;
-      v[u] = c < nc ? RegSum<Acc>::value(rb[c * S::WR + j], sh.scale[c_w + c]) : Acc(0);
+      v[u] = c < nc ? RegSum<Acc>::value(rb[c * S::WR + j], sh.scale[D == 2 ? v_w + c : v_w]) : Acc(0);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int idx = u * 32 + lane, c = idx / W, j = idx - c * W;
-      if (v[u] != Acc(0)) AccOps<Acc>::add_global(grow + (int64_t)c * g.cells + sh.col[j], v[u]);
+      if (v[u] != Acc(0))
+        AccOps<Acc>::add_global(grow + (D == 2 ? (int64_t)c * g.cells : sh.plane[c]) + sh.col[j], v[u]);
     }
   }
 }
@@ -645,350 +701,214 @@ __device__ __forceinline__ void sync2() {
     __syncthreads();
 }
 
-template <typename Acc, int NT1, int UC, int NW>
+template <typename Acc, int D, int NT1, int UC, int NW>
 __global__ void __launch_bounds__(32 * NW, warps2(NT1, UC) / NW)
-tile_accumulate_2d_kernel(SpreadGeom g, int nchan, const int* __restrict__ offsets,
-                          const int* __restrict__ items, const int* __restrict__ rec_base,
-                          const double* __restrict__ rec, int stride,
-                          const double* __restrict__ absum, int margin_bits,
-                          Acc* __restrict__ gacc) {
-  using S = Stage2<NT1, UC, NW>;
+tile_accumulate_reg_kernel(SpreadGeom g, int nchan, const int* __restrict__ offsets,
+                           const int* __restrict__ items, const int* __restrict__ rec_base,
+                           const double* __restrict__ rec, int stride,
+                           const double* __restrict__ absum, int margin_bits,
+                           Acc* __restrict__ gacc) {
+  using S = Stage2<D, NT1, UC, NW>;
   constexpr int MSP = (NT1 - 1) / 2;
   constexpr int NLC = kT2 * kT2;
   constexpr int NT = 32 * NW;
-  constexpr int W = S::W, GPL = S::GPL, NCW = S::NCW, NCB = S::NCB, WXS = S::WXS, RS = S::RS,
-                WR = S::WR;
+  constexpr int W = S::W, GPL = S::GPL, NCW = S::NCW, NVB = S::NVB, WXS = S::WXS, RS = S::RS,
+                VS = S::VS, WR = S::WR;
   __shared__ __align__(16) unsigned char s_raw[sizeof(S)];
   S& sh = *reinterpret_cast<S*>(s_raw);
   int* const off = sh.off;
   int* const cur = sh.cur;
-
-  const int item = blockIdx.x;
-  if (item >= items[g.ntiles]) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int tile = item_tile(items, g.ntiles, item, lane);
-  const int p_begin = offsets[tile] + (item - items[tile]) * g.item_points;
-  const int np = min(offsets[tile + 1] - p_begin, g.item_points);
-  const int tc0 = tile / g.ntile[1], tc1 = tile - tc0 * g.ntile[1];
-  const int c_begin = blockIdx.y * NCB;
-  const int nc = min(nchan - c_begin, NCB);
-  const int c_w = warp * NCW, nc_w = min(max(nc - c_w, 0), NCW);
+  const int c_begin = blockIdx.y * NVB;
+  const int nv = min(nchan - c_begin, NVB);  // value channels here
+  const int v_w = D == 2 ? warp * NCW : warp;                        // this warp's first one
+  const int nc_w = D == 2 ? min(max(nv - v_w, 0), NCW) : (warp < nv ? NT1 : 0);
   const int jm = lane % NT1, grp = lane / NT1;
   const bool active = grp < GPL && grp * UC < nc_w;
-
-  const double hx0 = g.ax[0].hx, hx1 = g.ax[1].hx;
-  const double if0 = 1.0 / g.four_tau[0], if1 = 1.0 / g.four_tau[1];
-  for (int c = tid; c < NCB; c += NT) {
-    const double sc = (c < nc && absum != nullptr) ? fixed_scale(absum[c_begin + c], margin_bits) : 1.0;
+  const double hy = g.ax[D - 2].hx, hx = g.ax[D - 1].hx;
+  const double ify = 1.0 / g.four_tau[D - 2], ifx = 1.0 / g.four_tau[D - 1];
+  for (int c = tid; c < NVB; c += NT) {
+    const double sc = (c < nv && absum != nullptr) ? fixed_scale(absum[c_begin + c], margin_bits) : 1.0;
     sh.scale[c] = sc;
     sh.zero[c] = RegSum<Acc>::zero(1.0 / sc);
   }
-  if (tid < 2 * (MSP + 1)) {
-    const int ax = tid / (MSP + 1), j = tid - ax * (MSP + 1);
-    const double t = (ax == 0 ? hx0 : hx1) * (double)j;
-    sh.cj[ax][j] = exp(-(t * t) * (ax == 0 ? if0 : if1));
+  for (int k = tid; k < D * (MSP + 1); k += NT) {
+    const int ax = k / (MSP + 1), j = k - ax * (MSP + 1);
+    const double t = g.ax[ax].hx * (double)j;
+    sh.cj[ax][j] = exp(-(t * t) / g.four_tau[ax]);
   }
-  if (tid < W) {
-    const int gc = (tc1 * kT2 + tid - MSP) % g.L[1];
-    sh.col[tid] = gc < 0 ? gc + g.L[1] : gc;
-  }
-  // counting sort by cell
-  for (int i = tid; i < NLC; i += NT) cur[i] = 0;
-  sync2<NW>();
+  // items in a grid-stride loop: most CTAs of a launch sized by the tiles of
+  // the whole (padded) grid would find none
+  const int nitems = items[g.ntiles];
+  for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+    const int tile = item_tile(items, g.ntiles, item, lane);
+    const int p_begin = offsets[tile] + (item - items[tile]) * g.item_points;
+    const int np = min(offsets[tile + 1] - p_begin, g.item_points);
+    const int tcx = tile % g.ntile[D - 1], tcy = tile / g.ntile[D - 1] % g.ntile[D - 2];
+    sync2<NW>();  // the last item's readers are done
+    if (tid < W) {
+      const int gc = (tcx * kT2 + tid - MSP) % g.L[D - 1];
+      sh.col[tid] = gc < 0 ? gc + g.L[D - 1] : gc;
+    }
+    if (D == 3 && tid < NT1) {
+      int gp = (tile / (g.ntile[D - 1] * g.ntile[D - 2]) + tid - MSP) % g.L[0];
+      if (gp < 0) gp += g.L[0];
+      sh.plane[tid] = (int64_t)gp * g.L[1] * g.L[D - 1];
+    }
+    // counting sort by cell
+    for (int i = tid; i < NLC; i += NT) cur[i] = 0;
+    sync2<NW>();
 #pragma unroll 4
-  for (int i = tid; i < np; i += NT) {
-    const int packed = rec_base[p_begin + i];
-    const int lc = (packed & 1023) * kT2 + ((packed >> 10) & 1023);
-    sh.st.cell[i] = (unsigned char)lc;
-    atomicAdd(&cur[lc], 1);
-  }
-  sync2<NW>();
-  if (warp == 0) {
-    const int a0 = cur[2 * lane], a1 = cur[2 * lane + 1];
-    int incl = a0 + a1;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    const int excl = incl - a0 - a1;
-    off[2 * lane] = excl;
-    off[2 * lane + 1] = excl + a0;
-    if (lane == 31) off[NLC] = incl;
-    __syncwarp();
-    cur[2 * lane] = excl;
-    cur[2 * lane + 1] = excl + a0;
-  }
-  sync2<NW>();
-  for (int i = tid; i < np; i += NT)
-    sh.st.order[atomicAdd(&cur[sh.st.cell[i]], 1)] = (unsigned short)i;
-  sync2<NW>();
-
-  // records of the 32 points from b0 on, copied in the background in pieces
-  // of 16 bytes: the knot offsets, then this CTA's channels
-  const int npc = 1 + (nc + 1) / 2, dpt = NT / npc, dpc = NT - dpt * npc;
-  const int pt0 = tid / npc, pc0 = tid - pt0 * npc;
-  const double* rec_t = rec + (int64_t)p_begin * stride;
-  auto fetch = [&](int b0, int half) {
-    const int cnt = min(32, np - b0);
-    for (int pt = pt0, pc = pc0; pt < cnt;) {
-      copy16_async(&sh.st.rec[half][pt * RS + 2 * pc],
-                   rec_t + (int64_t)sh.st.order[b0 + pt] * stride + (pc ? c_begin : 0) + 2 * pc);
-      pc += dpc;
-      pt += dpt;
-      if (pc >= npc) {
-        pc -= npc;
-        ++pt;
-      }
-    }
-  };
-  fetch(0, 0);
-
-  const int vofs = c_w + (active ? grp * UC : 0);  // idle lanes repeat group 0 and drop it
-  double a[UC][W];
-#pragma unroll
-  for (int k = 0; k < UC; ++k)
-#pragma unroll
-    for (int j = 0; j < W; ++j) a[k][j] = sh.zero[vofs + k];
-  int row = 0, half = 0;
-  for (int b0 = 0; b0 < np; b0 += 32, half ^= 1) {
-    const int b1 = min(b0 + 32, np);
-    copies_wait();
-    sync2<NW>();  // this batch's records are there, the last one's readers done
-    if (b0 + lane < b1) {
-      const double2 f = *reinterpret_cast<const double2*>(&sh.st.rec[half][lane * RS]);
-      if (NW == 1 || warp == 0) tap_weights<NT1>(f.x, hx0, if0, sh.cj[0], sh.st.wy + lane * NT1);
-      if (NW == 1 || warp == 1) tap_weights<NT1>(f.y, hx1, if1, sh.cj[1], sh.st.wx + lane * WXS);
+    for (int i = tid; i < np; i += NT) {
+      const int packed = rec_base[p_begin + i];
+      const int lc = ((packed >> (10 * (D - 2))) & 1023) * kT2 + ((packed >> (10 * (D - 1))) & 1023);
+      sh.st.cell[i] = (unsigned char)lc;
+      atomicAdd(&cur[lc], 1);
     }
     sync2<NW>();
-    fetch(b1, half ^ 1);
-    for (;;) {
-      int jy = jm - row % NT1;
-      if (jy < 0) jy += NT1;
-      const int* ro = off + row * kT2;
-      int pp = max(ro[0], b0) - b0;
-      const double* yp = sh.st.wy + pp * NT1 + jy;
-      const double* vp = sh.st.rec[half] + pp * RS + 2 + vofs;
-      const double2* xp = reinterpret_cast<const double2*>(sh.st.wx + pp * WXS);
-      double v[UC];  // the next point's values times its axis-0 weight
+    if (warp == 0) {
+      const int a0 = cur[2 * lane], a1 = cur[2 * lane + 1];
+      int incl = a0 + a1;
 #pragma unroll
-      for (int k = 0; k < UC; ++k) v[k] = RegSum<Acc>::factor(*yp * vp[k]);
-#pragma unroll
-      for (int cr = 0; cr < kT2; ++cr) {
-        const int pe = min(ro[cr + 1], b1) - b0;
-#pragma unroll 1
-        for (; pp < pe; ++pp) {
-          yp += NT1;
-          vp += RS;
-          const double wyn = *yp;
-          double u[UC], w[WXS];
-#pragma unroll
-          for (int k = 0; k < UC; ++k) u[k] = vp[k];
-#pragma unroll
-          for (int jx = 0; jx < NT1; jx += 2) {
-            const double2 q = xp[jx / 2];
-            w[jx] = q.x;
-            w[jx + 1] = q.y;
-          }
-          xp += WXS / 2;
-#pragma unroll
-          for (int jx = 0; jx < NT1; ++jx)
-#pragma unroll
-            for (int k = 0; k < UC; ++k) a[k][cr + jx] = __fma_rn(v[k], w[jx], a[k][cr + jx]);
-#pragma unroll
-          for (int k = 0; k < UC; ++k) v[k] = RegSum<Acc>::factor(wyn * u[k]);
-        }
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
       }
-      if (ro[kT2] > b1) break;      // the row goes on in the next batch
-      if (row >= W - NT1) break;    // every lane on its last row
-      // halo row `row` is complete: its lanes hand it over and start row + NT1
-      double* rb = sh.st.row + c_w * WR;
-      if (active && jm == row % NT1) {
-        double* rp = rb + grp * UC * WR;
-#pragma unroll
-        for (int k = 0; k < UC; ++k) {
-          const double z = sh.zero[vofs + k];
-#pragma unroll
-          for (int j = 0; j < W; ++j) {
-            rp[k * WR + j] = a[k][j];
-            a[k][j] = z;
-          }
-        }
-      }
+      const int excl = incl - a0 - a1;
+      off[2 * lane] = excl;
+      off[2 * lane + 1] = excl + a0;
+      if (lane == 31) off[NLC] = incl;
       __syncwarp();
-      add_rows<Acc, S>(g, sh, rb, 1, tc0 * kT2 + row - MSP, c_begin, c_w, nc_w, lane, gacc);
-      __syncwarp();
-      ++row;
+      cur[2 * lane] = excl;
+      cur[2 * lane + 1] = excl + a0;
     }
-  }
-  // the last NT1 rows, each in its own lanes
-  sync2<NW>();
-  double* rb = sh.rows + (size_t)warp * NT1 * NCW * WR;
-  if (active) {
-    int r = (jm - (W - NT1)) % NT1;  // position of this lane's row among W - NT1 .. W - 1
-    if (r < 0) r += NT1;
-    double* rp = rb + (r * NCW + grp * UC) * WR;
+    sync2<NW>();
+    for (int i = tid; i < np; i += NT)
+      sh.st.order[atomicAdd(&cur[sh.st.cell[i]], 1)] = (unsigned short)i;
+    sync2<NW>();
+
+    // records of the 32 points from b0 on, copied in the background: the knot
+    // offsets, then this CTA's channels, in pieces of 16 bytes (3-D: three
+    // offsets, so 8 bytes)
+    constexpr int PC = D == 2 ? 2 : 1;
+    const int npc = D == 2 ? 1 + (nv + 1) / 2 : 3 + nv;
+    const int dpt = NT / npc, dpc = NT - dpt * npc;
+    const int pt0 = tid / npc, pc0 = tid - pt0 * npc;
+    const double* rec_t = rec + (int64_t)p_begin * stride;
+    auto fetch = [&](int b0, int half) {
+      const int cnt = min(32, np - b0);
+      for (int pt = pt0, pc = pc0; pt < cnt;) {
+        copy_async<8 * PC>(&sh.st.rec[half][pt * RS + PC * pc],
+                           rec_t + (int64_t)sh.st.order[b0 + pt] * stride +
+                               (PC * pc >= D ? c_begin : 0) + PC * pc);
+        pc += dpc;
+        pt += dpt;
+        if (pc >= npc) {
+          pc -= npc;
+          ++pt;
+        }
+      }
+    };
+    fetch(0, 0);
+
+    // idle lanes repeat group 0 and drop it
+    const int c_w = warp * NCW, vofs = c_w + (active ? grp * UC : 0);
+    auto zero_of = [&](int k) { return sh.zero[D == 2 ? vofs + k : v_w]; };
+    double a[UC][W];
 #pragma unroll
     for (int k = 0; k < UC; ++k)
 #pragma unroll
-      for (int j = 0; j < W; ++j) rp[k * WR + j] = a[k][j];
-  }
-  __syncwarp();
-  add_rows<Acc, S>(g, sh, rb, NT1, tc0 * kT2 + (W - NT1) - MSP, c_begin, c_w, nc_w, lane, gacc);
-}
-
-// Register accumulators of the 3-D path hold doubles in both precisions.
-// Fixed point: each product is rounded to the nearest integer (ties to even,
-// like __double2ll_rn) by adding and subtracting 1.5 * 2^52 (exact for
-// |v| < 2^51), and the integer sums stay below 2^50, so every addition is
-// exact; the flush converts the exact integer sum once.
-template <typename Acc>
-__device__ __forceinline__ void reg_add(double& a, double v);
-template <>
-__device__ __forceinline__ void reg_add<long long>(double& a, double v) {
-  constexpr double kRound = 6755399441055744.0;  // 1.5 * 2^52
-  a = __dadd_rn(a, __dsub_rn(__dadd_rn(v, kRound), kRound));
-}
-template <>
-__device__ __forceinline__ void reg_add<double>(double& a, double v) {
-  a += v;
-}
-
-template <typename Acc>
-__device__ __forceinline__ Acc reg_value(double a);
-template <>
-__device__ __forceinline__ long long reg_value<long long>(double a) {
-  return __double2ll_rn(a);
-}
-template <>
-__device__ __forceinline__ double reg_value<double>(double a) {
-  return a;
-}
-
-// ---- 3-D path: column ownership ------------------------------------------
-// Tiles of 8 x 8 x 8 cells, halo width W = 7 + NT1 (16 for 9 taps).  Thread
-// t of a CTA owns the halo column (x0, x1) = (t / W, t % W) and holds its W
-// cells along the last axis in registers.  The points of the work item go in
-// batches of kBatch3: their base cells and per-axis tap weights are staged
-// in shared memory, the last axis's already times the channel value and the
-// fixed-point scale; then every thread walks the batch and adds, for each
-// point whose tap footprint covers its column, the NT1 taps along the last
-// axis into its registers: (e0 e1) (e2 v scale), rounded to an integer and
-// summed exactly, so the grid does not depend on the order of the points
-// (no shared atomics).  The lanes of a warp take the same point, so the
-// footprint's offset along the last axis is the same for the whole warp.
-// One channel at a time (blockIdx.y).
-constexpr int kBatch3 = 128;
-constexpr int kThreads3 = 256;
-
-inline size_t smem_3d(int nt1) {
-  return (size_t)kBatch3 * 3 * nt1 * sizeof(double) + (size_t)kBatch3 * sizeof(int);
-}
-
-template <typename Acc, int NT1, int BZ>
-__device__ __forceinline__ void column_taps(double (&acc)[7 + NT1], double wxy,
-                                            const double* __restrict__ e2v) {
-#pragma unroll
-  for (int k = 0; k < NT1; ++k) reg_add<Acc>(acc[BZ + k], __dmul_rn(wxy, e2v[k]));
-}
-
-template <typename Acc, int NT1, int BZ = 0>
-__device__ __forceinline__ void column_dispatch(int bz, double (&acc)[7 + NT1], double wxy,
-                                                const double* e2v) {
-  if constexpr (BZ < 8) {
-    if (bz == BZ)
-      column_taps<Acc, NT1, BZ>(acc, wxy, e2v);
-    else
-      column_dispatch<Acc, NT1, BZ + 1>(bz, acc, wxy, e2v);
-  }
-}
-
-template <typename Acc, int NT1>
-__global__ void __launch_bounds__(kThreads3)
-tile_columns_3d_kernel(SpreadGeom g, int ones_channel, const int* __restrict__ offsets,
-                       const int* __restrict__ items, const int* __restrict__ rec_base,
-                       const double* __restrict__ rec, int stride,
-                       const double* __restrict__ absum, int margin_bits,
-                       Acc* __restrict__ gacc) {
-  constexpr int MSP = (NT1 - 1) / 2;
-  constexpr int W = 7 + NT1;
-  constexpr int PP = 3 * NT1;  // per-axis weights of one point
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* s_w = reinterpret_cast<double*>(smem_raw);  // [kBatch3][PP]
-  int* s_base = reinterpret_cast<int*>(s_w + kBatch3 * PP);
-  const int ch = blockIdx.y;
-  const int item = blockIdx.x;
-  if (item >= items[g.ntiles]) return;
-  int lo = 0, hi = g.ntiles;  // tile owning this item: largest t with items[t] <= item
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (items[mid] <= item) lo = mid; else hi = mid;
-  }
-  const int tile = lo;
-  const int p_begin = offsets[tile] + (item - items[tile]) * g.item_points;
-  const int p_end = min(offsets[tile + 1], p_begin + g.item_points);
-  const double sc = absum ? (double)fixed_scale(absum[ch], margin_bits) : 1.0;
-  const bool ones = ones_channel && ch == 0;
-
-  const int t = threadIdx.x;
-  const bool owner = t < W * W;
-  const int c0 = t / W, c1 = t - (t / W) * W;
-  double acc[W];
-#pragma unroll
-  for (int z = 0; z < W; ++z) acc[z] = 0.0;
-
-  for (int b0 = p_begin; b0 < p_end; b0 += kBatch3) {
-    const int nb = min(kBatch3, p_end - b0);
-    for (int i = t; i < nb * PP; i += blockDim.x) {
-      const int pp = i / PP;
-      const int r = i - pp * PP;
-      const int a = r / NT1, j = r - a * NT1;
-      const double fr = rec[(int64_t)(b0 + pp) * stride + a];
-      const double diff = fr - g.ax[a].hx * (double)(j - MSP);
-      double e = fexp(-(diff * diff) / g.four_tau[a]);
-      if (a == 2) {
-        // last axis: times the channel value and the fixed-point scale
-        if (!ones) e = __dmul_rn(e, rec[(int64_t)(b0 + pp) * stride + 3 + ch]);
-        if (sc != 1.0) e = __dmul_rn(e, sc);
+      for (int j = 0; j < W; ++j) a[k][j] = zero_of(k);
+    int row = 0, half = 0;
+    for (int b0 = 0; b0 < np; b0 += 32, half ^= 1) {
+      const int b1 = min(b0 + 32, np);
+      copies_wait();
+      sync2<NW>();  // this batch's records are there, the last one's readers done
+      if (b0 + lane < b1) {
+        const double* r = &sh.st.rec[half][lane * RS];
+        if (NW == 1 || warp == 0)
+          tap_weights<NT1>(r[D - 2], 1.0, hy, ify, sh.cj[D - 2], sh.st.wy + lane * NT1);
+        if (NW == 1 || warp == 1)
+          tap_weights<NT1>(r[D - 1], 1.0, hx, ifx, sh.cj[D - 1], sh.st.wx + lane * WXS);
+        if (D == 3 && warp < nv)
+          tap_weights<NT1>(r[0], r[3 + warp], g.ax[0].hx, 1.0 / g.four_tau[0], sh.cj[0],
+                           sh.st.val + lane * VS + c_w);
       }
-      s_w[i] = e;
-    }
-    for (int i = t; i < nb; i += blockDim.x) s_base[i] = rec_base[b0 + i];
-    __syncthreads();
-    if (owner) {
-      for (int pp = 0; pp < nb; ++pp) {
-        const int packed = s_base[pp];
-        const int d0 = c0 - (packed & 1023);
-        const int d1 = c1 - ((packed >> 10) & 1023);
-        if (d0 >= 0 && d0 < NT1 && d1 >= 0 && d1 < NT1) {
-          const double* wp = s_w + pp * PP;
-          const double wxy = __dmul_rn(wp[d0], wp[NT1 + d1]);
-          column_dispatch<Acc, NT1>((packed >> 20) & 1023, acc, wxy, wp + 2 * NT1);
+      sync2<NW>();
+      fetch(b1, half ^ 1);
+      for (;;) {
+        int jy = jm - row % NT1;
+        if (jy < 0) jy += NT1;
+        const int* ro = off + row * kT2;
+        int pp = max(ro[0], b0) - b0;
+        const double* yp = sh.st.wy + pp * NT1 + jy;
+        const double* vp = (D == 2 ? sh.st.rec[half] + 2 : sh.st.val) + pp * VS + vofs;
+        const double2* xp = reinterpret_cast<const double2*>(sh.st.wx + pp * WXS);
+        double v[UC];  // the next point's values times its axis-0 weight
+#pragma unroll
+        for (int k = 0; k < UC; ++k) v[k] = RegSum<Acc>::factor(*yp * vp[k]);
+#pragma unroll
+        for (int cr = 0; cr < kT2; ++cr) {
+          const int pe = min(ro[cr + 1], b1) - b0;
+#pragma unroll 1
+          for (; pp < pe; ++pp) {
+            yp += NT1;
+            vp += VS;
+            const double wyn = *yp;
+            double u[UC], w[WXS];
+#pragma unroll
+            for (int k = 0; k < UC; ++k) u[k] = vp[k];
+#pragma unroll
+            for (int jx = 0; jx < NT1; jx += 2) {
+              const double2 q = xp[jx / 2];
+              w[jx] = q.x;
+              w[jx + 1] = q.y;
+            }
+            xp += WXS / 2;
+#pragma unroll
+            for (int jx = 0; jx < NT1; ++jx)
+#pragma unroll
+              for (int k = 0; k < UC; ++k) a[k][cr + jx] = __fma_rn(v[k], w[jx], a[k][cr + jx]);
+#pragma unroll
+            for (int k = 0; k < UC; ++k) v[k] = RegSum<Acc>::factor(wyn * u[k]);
+          }
         }
+        if (ro[kT2] > b1) break;      // the row goes on in the next batch
+        if (row >= W - NT1) break;    // every lane on its last row
+        // halo row `row` is complete: its lanes hand it over and start row + NT1
+        double* rb = sh.st.row + c_w * WR;
+        if (active && jm == row % NT1) {
+          double* rp = rb + grp * UC * WR;
+#pragma unroll
+          for (int k = 0; k < UC; ++k) {
+            const double z = zero_of(k);
+#pragma unroll
+            for (int j = 0; j < W; ++j) {
+              rp[k * WR + j] = a[k][j];
+              a[k][j] = z;
+            }
+          }
+        }
+        __syncwarp();
+        add_rows<Acc, D, S>(g, sh, rb, 1, tcy * kT2 + row - MSP, c_begin, v_w, nc_w, lane, gacc);
+        __syncwarp();
+        ++row;
       }
     }
-    __syncthreads();  // the next batch overwrites the staged points
-  }
-  if (!owner) return;
-  int tcoord[3];
-  {
-    int r = tile;
-    for (int a = 2; a >= 0; --a) {
-      tcoord[a] = r % g.ntile[a];
-      r /= g.ntile[a];
-    }
-  }
-  int gc0 = (tcoord[0] * g.T[0] + c0 - g.msp) % g.L[0];
-  if (gc0 < 0) gc0 += g.L[0];
-  int gc1 = (tcoord[1] * g.T[1] + c1 - g.msp) % g.L[1];
-  if (gc1 < 0) gc1 += g.L[1];
-  Acc* base = gacc + (int64_t)ch * g.cells + ((int64_t)gc0 * g.L[1] + gc1) * g.L[2];
+    // the last NT1 rows, each in its own lanes
+    sync2<NW>();
+    double* rb = sh.rows + (size_t)warp * NT1 * NCW * WR;
+    if (active) {
+      int r = (jm - (W - NT1)) % NT1;  // position of this lane's row among W - NT1 .. W - 1
+      if (r < 0) r += NT1;
+      double* rp = rb + (r * NCW + grp * UC) * WR;
 #pragma unroll
-  for (int z = 0; z < W; ++z) {
-    if (acc[z] == 0.0) continue;
-    int gc2 = (tcoord[2] * g.T[2] + z - g.msp) % g.L[2];
-    if (gc2 < 0) gc2 += g.L[2];
-    AccOps<Acc>::add_global(base + gc2, reg_value<Acc>(acc[z]));
+      for (int k = 0; k < UC; ++k)
+#pragma unroll
+        for (int j = 0; j < W; ++j) rp[k * WR + j] = a[k][j];
+    }
+    __syncwarp();
+    add_rows<Acc, D, S>(g, sh, rb, NT1, tcy * kT2 + (W - NT1) - MSP, c_begin, v_w, nc_w, lane, gacc);
   }
 }
 
@@ -1012,15 +932,18 @@ __global__ void finalize_kernel(int nchan, int64_t cells, const Acc* __restrict_
   }
 }
 
-// 2-D grids of at least 8 x 8 cells take the per-cell register path.
-static bool use_2d_path(int d, const int* L, int msp) {
-  return d == 2 && L[0] >= kT2 && L[1] >= kT2 && 2 * msp + 1 <= 13;
+// 2-D and 3-D grids of at least 8 x 8 cells on their last two axes take the
+// register path, with up to 13 taps per axis in 2-D and 9 in 3-D (what the
+// lanes hold; the wider stencils of the oversampled accuracies go through
+// shared-memory atomics).
+static bool use_reg_path(int d, const int* L, int msp) {
+  return d >= 2 && L[d - 2] >= kT2 && L[d - 1] >= kT2 && 2 * msp + 1 <= (d == 2 ? 13 : 9);
 }
 
 static void make_geom(SpreadGeom& g, int d, const int* L, int msp, const double* tau,
                       const double* kmap) {
   memset(&g, 0, sizeof(g));
-  const bool path2 = use_2d_path(d, L, msp);
+  const bool reg = use_reg_path(d, L, msp);
   g.d = d;
   g.msp = msp;
   g.ntaps1 = 2 * msp + 1;
@@ -1033,8 +956,8 @@ static void make_geom(SpreadGeom& g, int d, const int* L, int msp, const double*
   for (int a = 0; a < 3; ++a) {
     if (a < d) {
       g.L[a] = L[a];
-      int T = d == 1 ? 256 : (d == 2 ? (path2 ? kT2 : tile2[a]) : tile3[a]);
-      if (d == 3) {
+      int T = d == 1 ? 256 : (reg ? (a < d - 2 ? 1 : kT2) : (d == 2 ? tile2[a] : tile3[a]));
+      if (d == 3 && !reg) {
         // wide stencils (oversampled accuracies): smaller tiles, so that one
         // channel's tile plus halo fits shared memory
         const size_t kMax3 = (size_t)200 * 1024;
@@ -1063,10 +986,10 @@ static void make_geom(SpreadGeom& g, int d, const int* L, int msp, const double*
 
 // Points per work item, the same for the spread and for the deposits that
 // read its records.  Grids with few tiles (small 1-D grids): about four items
-// per SM.  2-D path, one warp per item: at least 24 warps' worth of items per
+// per SM.  Register path, one or two warps per item: at least 24 warps' worth of items per
 // SM (two rounds of the resident ones), 256 to 1024 points.
-static void size_items(SpreadGeom& g, int64_t n, bool path2) {
-  if (path2) {
+static void size_items(SpreadGeom& g, int64_t n, bool reg) {
+  if (reg) {
     const int64_t per = n / (24LL * sm_count());
     int ip = 256;
     while (ip < per && ip < kItem2) ip <<= 1;
@@ -1101,13 +1024,13 @@ static int channel_group(const SpreadGeom& g, int nchan, size_t acc_bytes) {
 }
 
 struct SpreadWs {
-  int* point_tile;
   int* counts;
   int* offsets;
   int* items;
   int* cursor;
   int* rec_base;
   int* rec_idx;
+  int2* totals;
   double* rec;
   double* absum;
   void* gacc;
@@ -1116,7 +1039,6 @@ struct SpreadWs {
 template <typename A>
 static void spread_layout(A& ar, int d, int64_t n, int ntiles, int nchan, int64_t cells,
                           SpreadWs* w) {
-  auto p0 = ar.template take<int>(n);
   auto p1 = ar.template take<int>(ntiles);
   auto p2 = ar.template take<int>(ntiles + 1);
   auto p3 = ar.template take<int>(ntiles + 1);
@@ -1126,8 +1048,8 @@ static void spread_layout(A& ar, int d, int64_t n, int ntiles, int nchan, int64_
   auto p8 = ar.template take<double>(FLPR_MAX_CHANNELS);
   auto p9 = ar.template take<double>((size_t)nchan * cells);
   auto p10 = ar.template take<int>(n);
+  auto p11 = ar.template take<int2>((ntiles + kScanTiles - 1) / kScanTiles);
   if (w) {
-    w->point_tile = (int*)p0;
     w->counts = (int*)p1;
     w->offsets = (int*)p2;
     w->items = (int*)p3;
@@ -1137,6 +1059,7 @@ static void spread_layout(A& ar, int d, int64_t n, int ntiles, int nchan, int64_
     w->absum = (double*)p8;
     w->gacc = (void*)p9;
     w->rec_idx = (int*)p10;
+    w->totals = (int2*)p11;
   }
 }
 
@@ -1174,19 +1097,28 @@ static int launch_accumulate(const SpreadGeom& g, int nchan, int cg,
   return FLPR_OK;
 }
 
-template <typename Acc, int NT1, int UC, int NW>
-static int launch_2d_k(const SpreadGeom& g, int nchan, const SpreadWs& w, const double* absum,
-                       int margin, int64_t max_items, cudaStream_t s) {
-  auto k = tile_accumulate_2d_kernel<Acc, NT1, UC, NW>;
+template <typename Acc, int D, int NT1, int UC, int NW>
+static int launch_reg_k(const SpreadGeom& g, int nchan, const SpreadWs& w, const double* absum,
+                        int margin, int64_t max_items, cudaStream_t s) {
+  auto k = tile_accumulate_reg_kernel<Acc, D, NT1, UC, NW>;
   FLPR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared));
-  constexpr int NCB = Stage2<NT1, UC, NW>::NCB;
-  k<<<dim3((unsigned)max_items, (unsigned)((nchan + NCB - 1) / NCB)), 32 * NW, 0, s>>>(
-      g, nchan, w.offsets, w.items, w.rec_base, w.rec, rec_stride(2, nchan), absum, margin,
+  constexpr int NVB = Stage2<D, NT1, UC, NW>::NVB;
+  // a CTA per item in 2-D (dealing them out in turn cost 5% there); in 3-D
+  // the slabs of the padded grid are 8 times the occupied ones and more: four
+  // rounds of the resident CTAs, each taking items in turn
+  const int64_t cap = D == 2 ? max_items : 4LL * sm_count() * (warps2(NT1, UC) / NW);
+  const unsigned nb = (unsigned)(max_items < cap ? max_items : cap);
+  k<<<dim3(nb, (unsigned)((nchan + NVB - 1) / NVB)), 32 * NW, 0, s>>>(
+      g, nchan, w.offsets, w.items, w.rec_base, w.rec, rec_stride(D, nchan), absum, margin,
       (Acc*)w.gacc);
   FLPR_LAUNCH_CHECK();
   return FLPR_OK;
 }
+
+#define FLPR_REG(D, U, N)                                                                         \
+  return fixed ? launch_reg_k<long long, D, NT1, U, N>(g, nchan, w, w.absum, margin, max_items, s) \
+               : launch_reg_k<double, D, NT1, U, N>(g, nchan, w, nullptr, margin, max_items, s);
 
 // Channels per lane and warps per item: the channels spread over the lane
 // groups of one warp while that needs at most three per lane, else of two
@@ -1196,45 +1128,22 @@ static int launch_accumulate_2d(const SpreadGeom& g, int nchan, const SpreadWs& 
                                 int margin, int64_t max_items, cudaStream_t s) {
   constexpr int GPL = groups2(NT1);
   const int uc = (nchan + GPL - 1) / GPL;
-#define FLPR_UC2(U, N)                                                                         \
-  return fixed ? launch_2d_k<long long, NT1, U, N>(g, nchan, w, w.absum, margin, max_items, s) \
-               : launch_2d_k<double, NT1, U, N>(g, nchan, w, nullptr, margin, max_items, s);
-  if (uc <= 1) FLPR_UC2(1, 1)
-  if (uc == 2) FLPR_UC2(2, 1)
-  if (uc == 3) FLPR_UC2(3, 1)
-  if (uc == 4) FLPR_UC2(2, 2)
-  FLPR_UC2(3, 2)
-#undef FLPR_UC2
+  if (uc <= 1) FLPR_REG(2, 1, 1)
+  if (uc == 2) FLPR_REG(2, 2, 1)
+  if (uc == 3) FLPR_REG(2, 3, 1)
+  if (uc == 4) FLPR_REG(2, 2, 2)
+  FLPR_REG(2, 3, 2)
 }
 
-// The column kernel covers 3-D tiles of 8^3 with at most 9 taps per axis
-// (halo columns fit one CTA of 256 threads).
-static bool use_3d_columns(const SpreadGeom& g) {
-  if (g.d != 3 || g.ntaps1 > 9) return false;
-  for (int a = 0; a < 3; ++a)
-    if (g.T[a] != 8 || g.W[a] != 7 + g.ntaps1) return false;
-  return true;
-}
-
+// 3-D: one channel per warp, two warps when there is more than one.
 template <int NT1>
-static int launch_columns_3d(const SpreadGeom& g, int nchan, int ones_channel,
-                             const SpreadWs& w, bool fixed, int margin, dim3 grid,
-                             cudaStream_t s) {
-  const size_t smem = smem_3d(NT1);
-  if (fixed) {
-    auto k = tile_columns_3d_kernel<long long, NT1>;
-    FLPR_CUDA(raise_dyn_smem(k, smem));
-    k<<<grid, kThreads3, smem, s>>>(g, ones_channel, w.offsets, w.items, w.rec_base, w.rec,
-                                    rec_stride(3, nchan), w.absum, margin, (long long*)w.gacc);
-  } else {
-    auto k = tile_columns_3d_kernel<double, NT1>;
-    FLPR_CUDA(raise_dyn_smem(k, smem));
-    k<<<grid, kThreads3, smem, s>>>(g, ones_channel, w.offsets, w.items, w.rec_base, w.rec,
-                                    rec_stride(3, nchan), nullptr, margin, (double*)w.gacc);
-  }
-  FLPR_LAUNCH_CHECK();
-  return FLPR_OK;
+static int launch_accumulate_3d(const SpreadGeom& g, int nchan, const SpreadWs& w, bool fixed,
+                                int margin, int64_t max_items, cudaStream_t s) {
+  constexpr int UC = (NT1 + groups2(NT1) - 1) / groups2(NT1);
+  if (nchan == 1) FLPR_REG(3, UC, 1)
+  FLPR_REG(3, UC, 2)
 }
+#undef FLPR_REG
 
 static int finalize(const SpreadGeom& g, int64_t n, int nchan, bool fixed, int margin,
                     const SpreadWs& w, void* d_grid_out, cudaStream_t s);
@@ -1275,7 +1184,7 @@ static int spread_impl(int d, int64_t n, const double* d_x, const double* h_kmap
   cudaStream_t s = as_stream(stream);
   SpreadGeom g;
   make_geom(g, d, h_L, msp, h_tau, h_kmap);
-  size_items(g, n, use_2d_path(d, h_L, msp));
+  size_items(g, n, use_reg_path(d, h_L, msp));
   ChanPtrs cp;
   memset(&cp, 0, sizeof(cp));
   for (int c = 0; c < nchan - ones_channel; ++c) cp.col[c] = h_cols[c];
@@ -1292,12 +1201,17 @@ static int spread_impl(int d, int64_t n, const double* d_x, const double* h_kmap
   if (nb > 8 * sm_count()) nb = 8 * sm_count();
   // per-channel sums of |v|: the fixed-point scales of the FP32 grid and of
   // the sorted adjoint deposits (flpr_deposit_sorted) in either precision
-  bin_count_kernel<<<nb, 256, 0, s>>>(g, n, d_x, d_kmap, w.point_tile, w.counts, nchan, ones_channel, cp,
+  bin_count_kernel<<<nb, 256, 0, s>>>(g, n, d_x, d_kmap, w.counts, nchan, ones_channel, cp,
                                       w.absum);
   FLPR_LAUNCH_CHECK();
-  tile_scan_kernel<<<1, 1024, 0, s>>>(g.ntiles, g.item_points, w.counts, w.offsets, w.items,
-                                      w.cursor);
+  const int nsb = (g.ntiles + kScanTiles - 1) / kScanTiles;
+  tile_scan_kernel<<<nsb, 1024, 0, s>>>(g.ntiles, g.item_points, w.counts, w.offsets, w.items,
+                                        w.cursor, w.totals);
   FLPR_LAUNCH_CHECK();
+  if (nsb > 1) {
+    tile_scan_add_kernel<<<nsb, 1024, 0, s>>>(g.ntiles, w.totals, w.offsets, w.items);
+    FLPR_LAUNCH_CHECK();
+  }
   // records and tap weights are float64 in both precisions: FP32 weights
   // lose ~1e-6 on the far taps (exponents near 8), which ill-conditioned
   // local systems in sparse corners amplify; only the accumulator differs
@@ -1310,7 +1224,7 @@ static int spread_impl(int d, int64_t n, const double* d_x, const double* h_kmap
   FLPR_LAUNCH_CHECK();
 
   int64_t max_items = (int64_t)g.ntiles + (n + g.item_points - 1) / g.item_points;
-  if (use_2d_path(d, h_L, msp)) {
+  if (d == 2 && use_reg_path(d, h_L, msp)) {
     int st = FLPR_OK;
     switch (g.ntaps1) {
       case 1: st = launch_accumulate_2d<1>(g, nchan, w, fixed, margin, max_items, s); break;
@@ -1325,15 +1239,14 @@ static int spread_impl(int d, int64_t n, const double* d_x, const double* h_kmap
     if (st != FLPR_OK) return st;
     return finalize(g, n, nchan, fixed, margin, w, d_grid_out, s);
   }
-  if (use_3d_columns(g)) {
-    dim3 grid3((unsigned)max_items, (unsigned)nchan);
+  if (d == 3 && use_reg_path(d, h_L, msp)) {
     int st = FLPR_OK;
     switch (g.ntaps1) {
-      case 1: st = launch_columns_3d<1>(g, nchan, ones_channel, w, fixed, margin, grid3, s); break;
-      case 3: st = launch_columns_3d<3>(g, nchan, ones_channel, w, fixed, margin, grid3, s); break;
-      case 5: st = launch_columns_3d<5>(g, nchan, ones_channel, w, fixed, margin, grid3, s); break;
-      case 7: st = launch_columns_3d<7>(g, nchan, ones_channel, w, fixed, margin, grid3, s); break;
-      case 9: st = launch_columns_3d<9>(g, nchan, ones_channel, w, fixed, margin, grid3, s); break;
+      case 1: st = launch_accumulate_3d<1>(g, nchan, w, fixed, margin, max_items, s); break;
+      case 3: st = launch_accumulate_3d<3>(g, nchan, w, fixed, margin, max_items, s); break;
+      case 5: st = launch_accumulate_3d<5>(g, nchan, w, fixed, margin, max_items, s); break;
+      case 7: st = launch_accumulate_3d<7>(g, nchan, w, fixed, margin, max_items, s); break;
+      case 9: st = launch_accumulate_3d<9>(g, nchan, w, fixed, margin, max_items, s); break;
       default: set_error("spread: msp=%d not supported by the 3-D path", g.msp); return FLPR_ERR_ARG;
     }
     if (st != FLPR_OK) return st;
@@ -1745,7 +1658,7 @@ int flpr_deposit_sorted(int d, int64_t n, const double* d_x, const int* h_L, int
   SpreadGeom g;
   double tau[3] = {1, 1, 1}, kmap[27] = {0};
   make_geom(g, d, h_L, msp, tau, kmap);
-  size_items(g, n, use_2d_path(d, h_L, msp));  // the work items the spread used
+  size_items(g, n, use_reg_path(d, h_L, msp));  // the work items the spread used
   Arena ar(const_cast<void*>(d_spread_ws), spread_ws_bytes);
   SpreadWs w;
   spread_layout(ar, d, n, g.ntiles, nchan, g.cells, &w);

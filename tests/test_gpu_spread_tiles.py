@@ -1,0 +1,91 @@
+"""The register-accumulating spread kernels at the sizes where their work
+changes shape: batches of 32 points, items of at most 1024, channels per lane
+and per warp, footprints from one tap up, grids of a single tile."""
+import numpy as np
+import pytest
+
+import oracle.lpr as oracle
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+# FP64: the sums of n products in another order; FP32: half an ulp of the
+# float grid (6e-8) and the fixed-point quantum, both of the largest cell
+TOL = {1: 1e-12, 0: 2e-7}
+
+
+def _spread(x, vals, G, msp, prec, ones=1, geom=None):
+    import torch
+    from fastlpr_b200 import _lib, api
+    n, d = x.shape
+    ctx = api._Ctx(torch.device("cuda", 0))
+    dx = ctx.upload(x)
+    if geom is None:
+        geom = api._make_geom(api._point_stats(ctx, dx, n, d), n, d, np.asarray(G), msp, True)
+    cols = [ctx.upload(np.ascontiguousarray(c)) for c in vals.T]
+    C = ones + len(cols)
+    grid = ctx.empty((C, int(np.prod(geom.L))), dtype=torch.float64 if prec else torch.float32)
+    ws = ctx.ws(ctx.lib.flpr_spread_ws(d, n, _lib.ivec(geom.L), msp, C, prec))
+    _lib.check(ctx.lib.flpr_spread(d, n, dx.data_ptr(), _lib.dvec(geom.kmap.ravel()),
+                                   _lib.ivec(geom.L), msp, _lib.dvec(geom.tau), C, ones,
+                                   _lib.pvec([c.data_ptr() for c in cols]), grid.data_ptr(), prec,
+                                   ws.data_ptr(), ws.numel(), ctx.stream), "spread")
+    torch.cuda.synchronize()
+    return grid.double().cpu().numpy().reshape((C,) + tuple(geom.L)) * n, geom
+
+
+def _reference(x, vals, G, geom, msp):
+    xs = (x - geom.mean) / geom.std - geom.center
+    xmod = oracle.knot_coordinates(xs, geom.L, np.asarray(G), geom.qin)
+    return oracle.spread_grid(xmod, vals, geom.L, msp, geom.tau)
+
+
+def _points(n, d, seed, clustered):
+    rng = np.random.default_rng(seed)
+    x = rng.random((n, d))
+    if clustered:
+        x[2:] = 0.4 + 0.02 * x[2:]     # a few cells hold nearly all points
+        x[0], x[1] = 0.0, 1.0
+    return x, rng
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("d,n,G,msp,nval,clustered", [
+    (2, 2, [4, 4], 4, 0, False), (2, 31, [9, 40], 4, 1, False), (2, 33, [16, 16], 4, 3, False),
+    (2, 1025, [33, 20], 4, 5, True), (2, 9000, [40, 24], 4, 8, True), (2, 4000, [64, 48], 4, 11, False),
+    (2, 4000, [64, 48], 4, 12, True), (2, 3000, [30, 31], 4, 18, False), (2, 700, [17, 30], 4, 40, False),
+    (2, 900, [20, 20], 0, 4, False), (2, 900, [20, 21], 1, 11, False), (2, 900, [21, 20], 2, 12, False),
+    (2, 900, [5, 20], 3, 7, False), (2, 900, [20, 20], 5, 9, False), (2, 900, [20, 6], 6, 11, True),
+    (3, 2, [4, 4, 4], 4, 0, False), (3, 33, [5, 9, 7], 4, 1, False), (3, 5000, [12, 16, 10], 4, 2, True),
+    (3, 1025, [3, 20, 8], 3, 3, False), (3, 800, [9, 6, 12], 2, 0, False), (3, 800, [9, 9, 9], 1, 4, False),
+    (3, 800, [10, 8, 9], 0, 1, False), (3, 300, [2, 9, 2], 4, 1, False), (3, 300, [6, 6, 6], 5, 1, False)])
+def test_tiles_match_oracle(cuda_ok, d, n, G, msp, nval, clustered, prec):
+    x, rng = _points(n, d, 7 * n + nval, clustered)
+    vals = rng.standard_normal((n, nval)) * 10.0 ** rng.integers(-3, 4, nval)
+    g, geom = _spread(x, vals, G, msp, prec)
+    ref = _reference(x, np.column_stack([np.ones(n), vals]), G, geom, msp)
+    for c in range(1 + nval):
+        assert rel_err(g[c], ref[c]) < TOL[prec], c
+
+
+@pytest.mark.parametrize("d,G", [(2, [32, 32]), (3, [12, 12, 12])])
+def test_fixed_point_sums_do_not_depend_on_the_order(cuda_ok, d, G):
+    """Knots on the cells and values of few bits: products that would round by
+    the parity of the sum if ties could occur."""
+    rng = np.random.default_rng(5)
+    x = rng.integers(0, G[0], (6000, d)) / (G[0] - 1.0)
+    x[0], x[1] = 0.0, 1.0
+    vals = np.column_stack([rng.integers(-4, 5, 6000) * 0.5, np.where(np.arange(6000) == 7, 2.0 ** 51, 1.0)])
+    a, geom = _spread(x, vals, G, 4, 0)
+    p = np.concatenate([[0, 1], 2 + rng.permutation(5998)])
+    b, _ = _spread(x[p], vals[p], G, 4, 0, geom=geom)
+    np.testing.assert_array_equal(a, b)
+
+
+def test_constant_channel_may_be_left_out(cuda_ok):
+    x, rng = _points(2000, 2, 3, False)
+    vals = rng.standard_normal((2000, 3))
+    g, geom = _spread(x, vals, [30, 30], 4, 1, ones=0)
+    ref = _reference(x, vals, [30, 30], geom, 4)
+    for c in range(3):
+        assert rel_err(g[c], ref[c]) < TOL[1]
