@@ -89,3 +89,46 @@ def test_constant_channel_may_be_left_out(cuda_ok):
     ref = _reference(x, vals, [30, 30], geom, 4)
     for c in range(3):
         assert rel_err(g[c], ref[c]) < TOL[1]
+
+
+@pytest.mark.parametrize("d,n,G,C,narrow", [
+    (2, 2, [4, 4], 1, False), (2, 255, [9, 40], 10, False), (2, 257, [40, 9], 11, False),
+    (2, 3000, [30, 31], 12, True), (2, 1500, [64, 48], 23, False), (2, 700, [5, 20], 32, True),
+    (2, 5000, [16, 16], 2, True), (1, 300, [40], 11, False)])
+def test_sorted_deposits_at_the_edges(cuda_ok, d, n, G, C, narrow):
+    """Sorted deposits against one FP64 atomic per point, corner and channel;
+    `narrow`: a raw grid inside the data, so points lie beyond it."""
+    import torch
+    from fastlpr_b200 import _lib, api
+    x, rng = _points(n, d, 11 * n + C, n == 5000)
+    cols = rng.standard_normal((n, C)) * 10.0 ** rng.integers(-3, 4, C)
+    ctx = api._Ctx(torch.device("cuda", 0))
+    dx = ctx.upload(x)
+    geom = api._make_geom(api._point_stats(ctx, dx, n, d), n, d, np.asarray(G), 4, True)
+    dc = [ctx.upload(np.ascontiguousarray(c)) for c in cols.T]
+    ptrs = _lib.pvec([c.data_ptr() for c in dc])
+    L, Gv = _lib.ivec(geom.L), _lib.ivec(G)
+    grid = ctx.empty((1 + C, int(np.prod(geom.L))), dtype=torch.float32)
+    ws = ctx.ws(ctx.lib.flpr_spread_ws(d, n, L, 4, 1 + C, 0))
+    _lib.check(ctx.lib.flpr_spread(d, n, dx.data_ptr(), _lib.dvec(geom.kmap.ravel()), L, 4,
+                                   _lib.dvec(geom.tau), 1 + C, 1, ptrs, grid.data_ptr(), 0,
+                                   ws.data_ptr(), ws.numel(), ctx.stream), "spread")
+    ax = _lib.dvec(api._axes_arg(api._raw_axes(geom, {"xrange": [[0.2, 0.7]] * d} if narrow else {})))
+    M, NP = int(np.prod(G)), (2 ** d) * (2 ** d + 1) // 2
+
+    def outputs():
+        return ctx.empty((M, C)), ctx.empty((M, NP)), ctx.empty(C)
+
+    a, b = outputs(), outputs()
+    ws2 = ctx.ws(ctx.lib.flpr_deposit_sorted_ws(d, n, L, 4, 1 + C))
+    _lib.check(ctx.lib.flpr_deposit_sorted(d, n, dx.data_ptr(), L, 4, 1 + C, 1, ptrs, ws.data_ptr(),
+                                           ws.numel(), ax, Gv, _lib.ivec(api._node0_cells(geom)),
+                                           a[0].data_ptr(), a[1].data_ptr(), a[2].data_ptr(),
+                                           ws2.data_ptr(), ws2.numel(), ctx.stream), "deposit_sorted")
+    _lib.check(ctx.lib.flpr_deposit(d, n, dx.data_ptr(), ax, Gv, C, ptrs, b[0].data_ptr(),
+                                    b[1].data_ptr(), b[2].data_ptr(), ctx.stream), "deposit")
+    torch.cuda.synchronize()
+    for c in range(C):
+        assert rel_err(a[0][:, c].cpu().numpy(), b[0][:, c].cpu().numpy()) < 1e-12
+    for u, v in zip(a[1:], b[1:]):
+        assert rel_err(u.cpu().numpy(), v.cpu().numpy()) < 1e-12
