@@ -27,6 +27,7 @@ streams, no capture).
 from __future__ import annotations
 
 import collections
+import gc
 import os
 import time
 from concurrent.futures import ThreadPoolExecutor
@@ -227,8 +228,16 @@ class LprPlan:
             graph = torch.cuda.CUDAGraph()
             cap = torch.cuda.Stream(self.device)
             cap.wait_stream(torch.cuda.current_stream(self.device))
-            with torch.cuda.graph(graph, stream=cap):
-                outs = self._issue(idx)
+            # a collection inside the capture could free an earlier plan's
+            # graphs and buffers, a call that ends the capture
+            collecting = gc.isenabled()
+            gc.disable()
+            try:
+                with torch.cuda.graph(graph, stream=cap):
+                    outs = self._issue(idx)
+            finally:
+                if collecting:
+                    gc.enable()
             self.segs.append(_Segment(idx, graph, outs, self._finite,
                                       torch.cuda.Stream(self.device)))
         torch.cuda.synchronize(self.device)
