@@ -32,6 +32,8 @@ SIGNATURES = [
     ("flpr_destroy", _I, [_VP]),
     ("flpr_point_stats_ws", _SZ, [_I, _I64]),
     ("flpr_point_stats", _I, [_I, _I64, _VP, _VP, _VP, _SZ, _VP]),
+    ("flpr_input_stats_ws", _SZ, [_I, _I64]),
+    ("flpr_input_stats", _I, [_I, _I64, _VP, _I, _PVP, _VP, _VP, _SZ, _VP]),
     ("flpr_point_stats_noalloc", _I, [_I, _I64, _VP, _VP, _VP]),
     ("flpr_spread_ws", _SZ, [_I, _I64, _PI, _I, _I, _I]),
     ("flpr_spread", _I, [_I, _I64, _VP, _PD, _PI, _I, _PD, _I, _I, _PVP, _VP, _I, _VP, _SZ, _VP]),
@@ -89,6 +91,8 @@ SIGNATURES = [
     ("flpr_spline_prefilter", _I, [_I, _PI, _I64, _I, _VP, _VP, _VP]),
     ("flpr_gcv_select", _I, [_I, _I, _I, _I, _I, _I, _D, _D, _VP, _VP, _VP, _VP, _VP]),
     ("flpr_select_grid", _I, [_I64, _I, _I, _I, _VP, _VP, _I, _VP, _VP, _VP, _VP]),
+    ("flpr_fit_outputs", _I, [_I, _I64, _VP, _PD, _PI, _I, _I, _I, _VP, _VP, _I, _VP, _PVP, _VP,
+                              _VP, _VP, _VP, _VP, _VP]),
     ("flpr_spline_reduce", _I, [_I, _I64, _VP, _VP, _PI, _I, _I, _I, _VP, _PVP, _PVP, _VP, _VP,
                                 _VP, _VP]),
     ("flpr_spline_eval", _I, [_I, _I64, _VP, _VP, _PI, _I, _VP, _VP, _VP]),

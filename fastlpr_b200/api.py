@@ -73,15 +73,6 @@ def _as_column_matrix(x) -> np.ndarray:
     return arr.astype(float, copy=False)
 
 
-def _finite_flags(tensors) -> torch.Tensor:
-    """Device-side NaN/Inf scan: [any NaN, any Inf] per tensor, in order."""
-    out = []
-    for t in tensors:
-        out.append(torch.isnan(t).any())
-        out.append(torch.isinf(t).any())
-    return torch.stack(out)
-
-
 def _raise_nonfinite(flags: np.ndarray, names, fn: str) -> None:
     """ValueError for the first NaN, then Inf, per input (api.py:310-323)."""
     for k, (what, _) in enumerate(names):
@@ -349,6 +340,24 @@ def _point_stats_dev(ctx: _Ctx, dx: torch.Tensor, n: int, d: int) -> torch.Tenso
     ctx.check(ctx.lib.flpr_point_stats(d, n, dx.data_ptr(), out.data_ptr(), ws.data_ptr(),
                                        ws.numel(), ctx.stream), "flpr_point_stats")
     return out
+
+
+def _input_stats_dev(ctx: _Ctx, dx: torch.Tensor, n: int, d: int,
+                     ycols: Sequence[torch.Tensor]) -> torch.Tensor:
+    """The (4 d) device statistics followed by four flags (0 or 1): any NaN,
+    any Inf in the points, any NaN, any Inf in the response columns."""
+    out = ctx.empty(4 * d + 4)
+    ws = ctx.ws(ctx.lib.flpr_input_stats_ws(d, n))
+    ctx.check(ctx.lib.flpr_input_stats(d, n, dx.data_ptr(), len(ycols),
+                                       _lib.pvec([c.data_ptr() for c in ycols]), out.data_ptr(),
+                                       ws.data_ptr(), ws.numel(), ctx.stream), "flpr_input_stats")
+    return out
+
+
+def _split_stats(v: np.ndarray, d: int) -> Tuple[np.ndarray, np.ndarray]:
+    """((4, d) statistics, flags) of a downloaded _input_stats_dev (or of the
+    statistics alone)."""
+    return v[:4 * d].reshape(4, d), v[4 * d:]
 
 
 def _point_stats(ctx: _Ctx, dx: torch.Tensor, n: int, d: int) -> np.ndarray:
@@ -1035,11 +1044,11 @@ def _prepare_lpr(ctx, x_arr, y_arr, dy, opts, order, prec, variance, y_is_comple
             else:
                 ycols.append(ctx.upload(np.ascontiguousarray(col, dtype=float)))
     y_raw_dev = None
-    flags_h = None
-    if dev_inputs is None and stats is None:
-        # NaN/Inf checks of the inputs (api.py:310-323) run on the device; the
-        # flags come back with the point statistics' synchronisation
-        flags_h = _to_host(_finite_flags([dx, torch.stack(ycols)]))
+    # NaN/Inf checks of the inputs (api.py:310-323) run on the device, with the
+    # point statistics; the flags come back with them
+    checked = dev_inputs is None and stats is None
+    st_dev = _input_stats_dev(ctx, dx, n, d, ycols) if checked else None
+    flags = None
     ev.mark("upload")
     if variance:
         y_raw_dev = ycols[0]
@@ -1072,7 +1081,8 @@ def _prepare_lpr(ctx, x_arr, y_arr, dy, opts, order, prec, variance, y_is_comple
         # device from the statistics, so the spread and the transform are
         # enqueued before the statistics reach the host (the host geometry
         # below repeats the same arithmetic)
-        st_dev = _point_stats_dev(ctx, dx, n, d)
+        if st_dev is None:
+            st_dev = _point_stats_dev(ctx, dx, n, d)
         st_host = _to_host(st_dev)
         st_ready = torch.cuda.Event()
         st_ready.record()
@@ -1087,11 +1097,13 @@ def _prepare_lpr(ctx, x_arr, y_arr, dy, opts, order, prec, variance, y_is_comple
         pre = SimpleNamespace(n=n, d=d, L=L, accuracy=accuracy, kmap=None)
         spec = _spread_fft(ctx, pre, dx, ycols + pcols, prec, ev, kmap_dev=kmap_dev, keep=kept)
         st_ready.synchronize()
-        stats = st_host.numpy().reshape(4, d)
+        stats, flags = _split_stats(st_host.numpy(), d)
+    elif checked:
+        stats, flags = _split_stats(st_dev.cpu().numpy(), d)
     elif stats is None:
         stats = _point_stats(ctx, dx, n, d)
-    if flags_h is not None:
-        _raise_nonfinite(flags_h.numpy(), [("Input x", 0), ("Response y", 1)], "cv_fastlpr")
+    if checked:
+        _raise_nonfinite(flags, [("Input x", 0), ("Response y", 1)], "cv_fastlpr")
     geom = _make_geom(stats, n, d, G, accuracy, flag_power2)
     ev.mark("setup")
     if spec is None:
@@ -1520,14 +1532,22 @@ def _finalize_enqueue(ctx, st: _LprState, r: dict, ev, device_select: bool = Fal
     geom = st.geom
     m, S = r["m"], r["S"]
     H, ns, M = r["H"], r["ns"], geom.M
-    gcv_dev = sel_dev = None
+    gcv_dev = sel_dev = pack = None
     if device_select:
+        if not st.variance and st.methods["output"] != "cubic" and ny <= 32:
+            # every output in one buffer: one launch forms them in the layouts
+            # of the result, one copy brings them down
+            pack = ctx.empty(2 * n * ny + M * (ny + 1) + 4 * H + 1)
         sel_dev = ctx.empty(1, dtype=torch.int32)
         if st.calc_dof:
             if hsum_dev is None:
                 hs = torch.from_numpy(np.ascontiguousarray(np.sum(r["bw_k"], axis=1))).pin_memory()
                 hsum_dev = hs.to(ctx.device, non_blocking=True)
-            gcv_dev = ctx.empty(4 * H)
+            if pack is not None:
+                gcv_ptr = pack.data_ptr() + 8 * (pack.numel() - 1 - 4 * H)
+            else:
+                gcv_dev = ctx.empty(4 * H)
+                gcv_ptr = gcv_dev.data_ptr()
             agg = {"first": 0, "average": 1, "sum": 2}.get(str(st.opts.get("gcv_selection",
                                                                             "first")))
             if agg is None:
@@ -1536,13 +1556,29 @@ def _finalize_enqueue(ctx, st: _LprState, r: dict, ev, device_select: bool = Fal
             ctx.check(lib.flpr_gcv_select(H, ny, st.R, 1 if r["dual"] else 0,
                                           1 if st.y_is_complex else 0, agg, float(n),
                                           float(st.opts.get("dstd", 0.0)), r["packed"].data_ptr(),
-                                          hsum_dev.data_ptr(), gcv_dev.data_ptr(),
+                                          hsum_dev.data_ptr(), gcv_ptr,
                                           sel_dev.data_ptr(), ctx.stream), "flpr_gcv_select")
         else:
             sel_dev.zero_()
+        s_prec = _lib.FLPR_PREC_F32 if S.dtype == torch.float32 else _lib.FLPR_PREC_F64
+        if pack is not None:
+            p0 = pack.data_ptr()
+            p1, p2, p3 = p0 + 8 * n * ny, p0 + 16 * n * ny, p0 + 16 * n * ny + 8 * M * ny
+            ctx.check(lib.flpr_fit_outputs(d, n, st.dx.data_ptr(), st.ax_arg, st.G_arg, ny,
+                                           r["mstride"], m.shape[0], m.data_ptr(), S.data_ptr(),
+                                           s_prec, sel_dev.data_ptr(),
+                                           _lib.pvec([c.data_ptr() for c in st.ycols[:ny]]), p0,
+                                           p1, p2, p3, p0 + 8 * (pack.numel() - 1), ctx.stream),
+                      "flpr_fit_outputs")
+            ev.mark("final_interp")
+            if bufs is None:
+                return {"pack": _to_host(pack)}
+            if bufs.get("pack") is None:
+                return {"pack": pack}
+            bufs["pack"].copy_(pack, non_blocking=True)
+            return {"pack": bufs["pack"]}
         gv_dev = ctx.empty((ny, M))
         s0_dev = ctx.empty(M)
-        s_prec = _lib.FLPR_PREC_F32 if S.dtype == torch.float32 else _lib.FLPR_PREC_F64
         ctx.check(lib.flpr_select_grid(M, ny, r["mstride"], m.shape[0], m.data_ptr(),
                                        S.data_ptr(), s_prec, sel_dev.data_ptr(),
                                        gv_dev.data_ptr(), s0_dev.data_ptr(), ctx.stream),
@@ -1624,6 +1660,24 @@ def _output_bufs(st: _LprState, H: int) -> dict:
             "gcv": pin(4 * H) if st.calc_dof else None, "sel": pin(1, torch.int32)}
 
 
+def _unpack_outputs(st: _LprState, r: dict, pack: torch.Tensor) -> dict:
+    """The outputs of _finalize_enqueue as views of the downloaded buffer
+    {fitted values (n, ny), residuals (n, ny), surface (M, ny), s0 (M), GCV
+    arrays (4 H), index}."""
+    n, ny, M, H = st.n, st.ny, st.geom.M, r["H"]
+
+    def shaped(t, k):
+        if st.y_is_complex:
+            t = torch.view_as_complex(t.view(k, st.dy, 2))
+            return t[:, 0] if st.dy == 1 else t
+        return t if ny == 1 else t.view(k, ny)
+
+    a, b, c = n * ny, 2 * n * ny, 2 * n * ny + M * ny
+    return {"yh": shaped(pack[:a], n), "rh": shaped(pack[a:b], n), "gvh": shaped(pack[b:c], M),
+            "s0h": pack[c:c + M], "dn": None,
+            "gcv": pack[c + M:c + M + 4 * H] if st.calc_dof else None, "sel": pack[-1:]}
+
+
 def _finalize_build(ctx, st: _LprState, r: dict, pend: dict, ev, search,
                     copy: bool = False) -> RegressionOutput:
     """Result structure from the downloaded outputs of _finalize_enqueue
@@ -1631,6 +1685,8 @@ def _finalize_build(ctx, st: _LprState, r: dict, pend: dict, ev, search,
     d, dy = st.d, st.dy
     geom, opts = st.geom, st.opts
     bw_k = r["bw_k"]
+    if "pack" in pend:
+        pend = _unpack_outputs(st, r, pend["pack"])
     if pend.get("sel") is not None:
         sel = int(pend["sel"].numpy()[0])
         if st.calc_dof:
@@ -1807,6 +1863,8 @@ def _learned_finish(ctx, st: _LprState, bandwidths: np.ndarray, r: dict, pend: d
     r["bw_k"] = bandwidths[window]
     record = {"mode": "learned", "proposal_index": t, "windows": [[int(i) for i in window]],
               "nlist": nlist, "accepted": False}
+    if "pack" in pend:
+        pend = _unpack_outputs(st, r, pend["pack"])
     gcv_m = pend["gcv"].numpy()[:R]
     for walk in range(_MAX_WALKS + 1):
         pos = int(np.argmin(gcv_m))
@@ -1961,9 +2019,8 @@ def _fit_kde(ctx, x_arr, bandwidths, opts, G, prec):
     lib = ctx.lib
     n, d = x_arr.shape
     dx = ctx.upload(x_arr)
-    flags_h = _to_host(_finite_flags([dx]))
-    stats = _point_stats(ctx, dx, n, d)
-    _raise_nonfinite(flags_h.numpy(), [("Input x", 0)], "cv_fastkde")
+    stats, flags = _split_stats(_input_stats_dev(ctx, dx, n, d, []).cpu().numpy(), d)
+    _raise_nonfinite(flags, [("Input x", 0)], "cv_fastkde")
     geom = _make_geom(stats, n, d, G, int(opts["accuracy"]), bool(opts.get("flag_power2", True)))
     kern, bw, keep, ihbad = _filter_bandwidths(ctx, geom, bandwidths, 1, _kernel_id(opts))
     if len(keep) != bandwidths.shape[0] or bw.shape[0] != bandwidths.shape[0]:

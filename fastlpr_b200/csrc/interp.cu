@@ -210,6 +210,42 @@ __global__ void interp_eval_kernel(InterpGeom g, int64_t n, const double* __rest
   }
 }
 
+// Outputs of a fit at bandwidth *sel: fitted values and residuals (n, ny) at
+// the points, the surface (M, ny) and the zeroth moment plane s0 (M), in one
+// launch and in the layouts of the result.  NaN when *sel is out of range.
+template <int D, typename SReal>
+__global__ void __launch_bounds__(256)
+fit_outputs_kernel(InterpGeom g, int64_t n, const double* __restrict__ x, int ny, int mstride,
+                   int H, const double* __restrict__ m, const SReal* __restrict__ S,
+                   const int* __restrict__ sel, ColPtrs yc, double* __restrict__ yhat,
+                   double* __restrict__ res, double* __restrict__ surf, double* __restrict__ s0,
+                   double* __restrict__ sel_out) {
+  const int s = *sel;
+  const bool ok = s >= 0 && s < H;
+  const double* ms = m + (int64_t)(ok ? s : 0) * g.M * mstride;
+  const int64_t total = n > g.M ? n : g.M;
+  if (blockIdx.x == 0 && threadIdx.x == 0) sel_out[0] = (double)s;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    if (i < n) {
+      StencilD<D> st;
+      make_stencil_d<D>(g, x, i, st);
+      for (int c = 0; c < ny; ++c) {
+        double r = 0.0;
+#pragma unroll
+        for (int k = 0; k < (1 << D); ++k) r += st.w[k] * ms[st.base[k] * mstride + c];
+        if (!ok) r = NAN;
+        yhat[i * ny + c] = r;
+        res[i * ny + c] = yc.col[c][i] - r;
+      }
+    }
+    if (i < g.M) {
+      for (int c = 0; c < ny; ++c) surf[i * ny + c] = ok ? ms[i * mstride + c] : NAN;
+      s0[i] = ok ? (double)S[(int64_t)s * g.M + i] : NAN;
+    }
+  }
+}
+
 // ---- KDE -----------------------------------------------------------------
 __global__ void plane_sum_kernel(int64_t M, const double* __restrict__ s, double* __restrict__ sums) {
   __shared__ double sh[32];
@@ -504,6 +540,20 @@ static int pt_blocks(int64_t n, int per_sm) {
   return (int)b;
 }
 
+template <int D>
+static void launch_outputs(const InterpGeom& g, int64_t n, const double* x, int ny, int mstride,
+                           int H, const double* m, const void* S, int s_prec, const int* sel,
+                           const ColPtrs& yc, double* yhat, double* res, double* surf, double* s0,
+                           double* sel_out, cudaStream_t s) {
+  const int nb = pt_blocks(n > g.M ? n : g.M, 8);
+  if (s_prec == FLPR_PREC_F32)
+    fit_outputs_kernel<D, float><<<nb, 256, 0, s>>>(g, n, x, ny, mstride, H, m, (const float*)S,
+                                                    sel, yc, yhat, res, surf, s0, sel_out);
+  else
+    fit_outputs_kernel<D, double><<<nb, 256, 0, s>>>(g, n, x, ny, mstride, H, m, (const double*)S,
+                                                     sel, yc, yhat, res, surf, s0, sel_out);
+}
+
 }  // namespace flpr
 
 using namespace flpr;
@@ -559,6 +609,33 @@ int flpr_interp_eval(int d, int64_t n, const double* d_x, const double* h_ax, co
   FLPR_CHECK_ARG(n >= 1 && nval >= 1, "interp_eval: n=%lld nval=%d", (long long)n, nval);
   interp_eval_kernel<false><<<pt_blocks(n, 8), 256, 0, as_stream(stream)>>>(g, n, d_x, nval,
                                                                              d_vals, d_out);
+  FLPR_LAUNCH_CHECK();
+  return FLPR_OK;
+}
+
+int flpr_fit_outputs(int d, int64_t n, const double* d_x, const double* h_ax, const int* h_G,
+                     int ny, int mstride, int H, const double* d_m, const void* d_S, int s_prec,
+                     const int* d_sel, const double* const* h_ycols, double* d_yhat,
+                     double* d_res, double* d_surface, double* d_s0, double* d_sel_out,
+                     void* stream) {
+  InterpGeom g;
+  FLPR_TRY(make_geom(g, d, h_ax, h_G));
+  FLPR_CHECK_ARG(n >= 1 && H >= 1 && ny >= 1 && ny <= kMaxRed && mstride >= ny,
+                 "fit_outputs: n=%lld H=%d ny=%d mstride=%d", (long long)n, H, ny, mstride);
+  FLPR_CHECK_ARG(s_prec == FLPR_PREC_F32 || s_prec == FLPR_PREC_F64, "fit_outputs: precision");
+  ColPtrs yc;
+  memset(&yc, 0, sizeof(yc));
+  for (int c = 0; c < ny; ++c) yc.col[c] = h_ycols[c];
+  cudaStream_t s = as_stream(stream);
+#define FLPR_OUT(D)                                                                          \
+  launch_outputs<D>(g, n, d_x, ny, mstride, H, d_m, d_S, s_prec, d_sel, yc, d_yhat, d_res, \
+                    d_surface, d_s0, d_sel_out, s)
+  switch (d) {
+    case 1: FLPR_OUT(1); break;
+    case 2: FLPR_OUT(2); break;
+    default: FLPR_OUT(3); break;
+  }
+#undef FLPR_OUT
   FLPR_LAUNCH_CHECK();
   return FLPR_OK;
 }

@@ -25,15 +25,28 @@ __device__ __forceinline__ Moments merge(const Moments& a, const Moments& b) {
 
 constexpr int kStatThreads = 256;
 
-// One block-partial per (block, axis): Welford per thread, Chan merge.
+struct StatCols {
+  const double* col[FLPR_MAX_CHANNELS];
+};
+
+// 1: NaN, 2: infinite
+__device__ __forceinline__ int unfit(double v) { return isnan(v) ? 1 : (isinf(v) ? 2 : 0); }
+
+// One block-partial per (block, axis): Welford per thread, Chan merge.  With
+// `bad`, the pass over the points also looks for NaN and infinities (bits 0
+// and 1 of bad[block]) and so does one over ncol response columns (bits 2
+// and 3): the checks cost no launch and no further read of the points.
 __global__ void point_stats_partial(int d, int64_t n, const double* __restrict__ x,
-                                    Moments* __restrict__ part) {
+                                    Moments* __restrict__ part, int ncol, StatCols cols,
+                                    int* __restrict__ bad) {
   __shared__ Moments sh[kStatThreads];
+  int flags = 0;
   for (int ax = 0; ax < d; ++ax) {
     Moments m{0.0, 0.0, 0.0, INFINITY, -INFINITY};
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
       double v = x[i * d + ax];
+      flags |= unfit(v);
       m.n += 1.0;
       double delta = v - m.mean;
       m.mean += delta / m.n;
@@ -50,10 +63,21 @@ __global__ void point_stats_partial(int d, int64_t n, const double* __restrict__
     if (threadIdx.x == 0) part[blockIdx.x * d + ax] = sh[0];
     __syncthreads();
   }
+  if (bad == nullptr) return;
+  int yf = 0;
+  for (int c = 0; c < ncol; ++c)
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x)
+      yf |= unfit(cols.col[c][i]);
+  flags |= yf << 2;
+  int any = 0;
+  for (int k = 0; k < 4; ++k) any |= __syncthreads_or(flags & (1 << k)) ? 1 << k : 0;
+  if (threadIdx.x == 0) bad[blockIdx.x] = any;
 }
 
+// out: the 4 d statistics, then (with `bad`) the four flags as 0 or 1
 __global__ void point_stats_final(int d, int nblocks, const Moments* __restrict__ part,
-                                  double* __restrict__ out) {
+                                  const int* __restrict__ bad, double* __restrict__ out) {
   __shared__ Moments sh[kStatThreads];
   for (int ax = 0; ax < d; ++ax) {
     Moments m{0.0, 0.0, 0.0, INFINITY, -INFINITY};
@@ -71,6 +95,13 @@ __global__ void point_stats_final(int d, int nblocks, const Moments* __restrict_
       out[3 * d + ax] = sh[0].m2;
     }
     __syncthreads();
+  }
+  if (bad == nullptr) return;
+  int flags = 0;
+  for (int b = threadIdx.x; b < nblocks; b += blockDim.x) flags |= bad[b];
+  for (int k = 0; k < 4; ++k) {
+    const int any = __syncthreads_or(flags & (1 << k));
+    if (threadIdx.x == 0) out[4 * d + k] = any ? 1.0 : 0.0;
   }
 }
 
@@ -186,9 +217,10 @@ int flpr_point_stats_noalloc(int d, int64_t n, const double* d_x, double* d_stat
   FLPR_TRY(noalloc_scratch(&part));
   // every block writes its record for every axis before point_stats_final
   // reads it, so nothing in the scratch has to start at zero
-  point_stats_partial<<<nb, kStatThreads, 0, as_stream(stream)>>>(d, n, d_x, part);
+  point_stats_partial<<<nb, kStatThreads, 0, as_stream(stream)>>>(d, n, d_x, part, 0, StatCols{},
+                                                                   nullptr);
   FLPR_LAUNCH_CHECK();
-  point_stats_final<<<1, kStatThreads, 0, as_stream(stream)>>>(d, nb, part, d_stats);
+  point_stats_final<<<1, kStatThreads, 0, as_stream(stream)>>>(d, nb, part, nullptr, d_stats);
   FLPR_LAUNCH_CHECK();
   return FLPR_OK;
 }
@@ -207,9 +239,36 @@ int flpr_point_stats(int d, int64_t n, const double* d_x, double* d_stats, void*
   }
   int nb = stat_blocks(n);
   Moments* part = static_cast<Moments*>(d_ws);
-  point_stats_partial<<<nb, kStatThreads, 0, as_stream(stream)>>>(d, n, d_x, part);
+  point_stats_partial<<<nb, kStatThreads, 0, as_stream(stream)>>>(d, n, d_x, part, 0, StatCols{},
+                                                                   nullptr);
   FLPR_LAUNCH_CHECK();
-  point_stats_final<<<1, kStatThreads, 0, as_stream(stream)>>>(d, nb, part, d_stats);
+  point_stats_final<<<1, kStatThreads, 0, as_stream(stream)>>>(d, nb, part, nullptr, d_stats);
+  FLPR_LAUNCH_CHECK();
+  return FLPR_OK;
+}
+
+size_t flpr_input_stats_ws(int d, int64_t n) {
+  return flpr_point_stats_ws(d, n) + align_up(sizeof(int) * (size_t)stat_blocks(n));
+}
+
+int flpr_input_stats(int d, int64_t n, const double* d_x, int ncol, const double* const* h_cols,
+                     double* d_out, void* d_ws, size_t ws_bytes, void* stream) {
+  FLPR_CHECK_ARG(d >= 1 && d <= 16, "input_stats: bad d=%d", d);
+  FLPR_CHECK_ARG(n >= 1, "input_stats: n=%lld", (long long)n);
+  FLPR_CHECK_ARG(ncol >= 0 && ncol <= FLPR_MAX_CHANNELS, "input_stats: ncol=%d", ncol);
+  if (ws_bytes < flpr_input_stats_ws(d, n)) {
+    set_error("input_stats: workspace too small");
+    return FLPR_ERR_WORKSPACE;
+  }
+  const int nb = stat_blocks(n);
+  Moments* part = static_cast<Moments*>(d_ws);
+  int* bad = reinterpret_cast<int*>(static_cast<char*>(d_ws) + flpr_point_stats_ws(d, n));
+  StatCols cols{};
+  for (int c = 0; c < ncol; ++c) cols.col[c] = h_cols[c];
+  point_stats_partial<<<nb, kStatThreads, 0, as_stream(stream)>>>(d, n, d_x, part, ncol, cols,
+                                                                   bad);
+  FLPR_LAUNCH_CHECK();
+  point_stats_final<<<1, kStatThreads, 0, as_stream(stream)>>>(d, nb, part, bad, d_out);
   FLPR_LAUNCH_CHECK();
   return FLPR_OK;
 }

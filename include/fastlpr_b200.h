@@ -70,6 +70,13 @@ int flpr_destroy(flpr_handle_t handle);
 size_t flpr_point_stats_ws(int d, int64_t n);
 int flpr_point_stats(int d, int64_t n, const double* d_x, double* d_stats,
                      void* d_ws, size_t ws_bytes, void* stream);
+/* The same statistics with the input checks of a fit (api.py:310-323): d_out
+ * receives the 4*d statistics and then four flags (0 or 1): any NaN, any
+ * infinity in x, any NaN, any infinity in the ncol response columns h_cols
+ * (device float64 arrays of n; ncol may be 0). */
+size_t flpr_input_stats_ws(int d, int64_t n);
+int flpr_input_stats(int d, int64_t n, const double* d_x, int ncol, const double* const* h_cols,
+                     double* d_out, void* d_ws, size_t ws_bytes, void* stream);
 
 /* (1b) The same point statistics without any device allocation by the
  * caller or the library.  This entry point has no counterpart in the
@@ -469,6 +476,17 @@ int flpr_gcv_select(int H, int ny, int R, int dual, int y_complex, int agg, doub
                     void* stream);
 int flpr_select_grid(int64_t M, int ny, int mstride, int H, const double* d_m, const void* d_S,
                      int s_prec, const int* d_sel, double* d_gv, double* d_s0, void* stream);
+/* Outputs of a fit at bandwidth *d_sel in one launch: fitted values and
+ * residuals (n, ny) at the points (clamped multilinear interpolation, as
+ * flpr_interp_eval), the surface (M, ny) and s0 (M), NaN when *d_sel is not
+ * in [0, H); d_sel_out[0] receives the index as a double.  d_m: (H, M,
+ * mstride); d_S and s_prec as for flpr_select_grid; h_ycols: ny device
+ * columns.  api.py:743-832. */
+int flpr_fit_outputs(int d, int64_t n, const double* d_x, const double* h_ax, const int* h_G,
+                     int ny, int mstride, int H, const double* d_m, const void* d_S, int s_prec,
+                     const int* d_sel, const double* const* h_ycols, double* d_yhat,
+                     double* d_res, double* d_surface, double* d_s0, double* d_sel_out,
+                     void* stream);
 
 /* ---------------------------------------------------------------------
  * (9) KDE normalisation and LCV.  Replaces api.py:1059-1133.

@@ -132,3 +132,59 @@ def test_sorted_deposits_at_the_edges(cuda_ok, d, n, G, C, narrow):
         assert rel_err(a[0][:, c].cpu().numpy(), b[0][:, c].cpu().numpy()) < 1e-12
     for u, v in zip(a[1:], b[1:]):
         assert rel_err(u.cpu().numpy(), v.cpu().numpy()) < 1e-12
+
+
+@pytest.mark.parametrize("d,n,G,ny,mstride,f32", [(1, 2, [2], 1, 1, True), (1, 5000, [40], 2, 12, False),
+                                                  (2, 257, [30, 7], 3, 3, True), (3, 900, [4, 5, 6], 1, 1, False),
+                                                  (2, 50, [60, 50], 4, 5, False)])
+def test_fit_outputs_match_their_parts(cuda_ok, d, n, G, ny, mstride, f32):
+    import torch
+    from fastlpr_b200 import _lib, api
+    rng = np.random.default_rng(n)
+    ctx = api._Ctx(torch.device("cuda", 0))
+    M, H = int(np.prod(G)), 3
+    x = ctx.upload(rng.random((n, d)) * 1.2 - 0.1)
+    m, y = ctx.upload(rng.standard_normal((H, M, mstride))), ctx.upload(rng.standard_normal((ny, n)))
+    S = ctx.upload(rng.random((H, M))).to(torch.float32 if f32 else torch.float64)
+    ax, Gv = _lib.dvec([0.0, 1.0 / 40] * d), _lib.ivec(G)
+    for pick in (0, 2, -1):
+        sel = torch.tensor([pick], dtype=torch.int32, device=x.device)
+        yh, res, surf, s0, so = (ctx.empty(s) for s in ((n, ny), (n, ny), (M, ny), (M,), (1,)))
+        _lib.check(ctx.lib.flpr_fit_outputs(
+            d, n, x.data_ptr(), ax, Gv, ny, mstride, H, m.data_ptr(), S.data_ptr(), 0 if f32 else 1,
+            sel.data_ptr(), _lib.pvec([y[c].data_ptr() for c in range(ny)]), yh.data_ptr(),
+            res.data_ptr(), surf.data_ptr(), s0.data_ptr(), so.data_ptr(), ctx.stream), "outputs")
+        assert float(so[0]) == pick
+        if pick < 0:
+            assert all(bool(torch.isnan(t).all()) for t in (yh, res, surf, s0))
+            continue
+        vals, ref = m[pick][:, :ny].t().contiguous(), ctx.empty((ny, n))
+        _lib.check(ctx.lib.flpr_interp_eval(d, n, x.data_ptr(), ax, Gv, ny, vals.data_ptr(),
+                                            ref.data_ptr(), ctx.stream), "interp_eval")
+        assert torch.equal(yh, ref.t()) and torch.equal(res, y.t() - ref.t())
+        assert torch.equal(surf, vals.t()) and torch.equal(s0, S[pick].double())
+
+
+@pytest.mark.parametrize("n", [1, 255, 257, 700000])
+def test_input_stats_flags(cuda_ok, n):
+    import torch
+    from fastlpr_b200 import api
+    rng = np.random.default_rng(n)
+    ctx = api._Ctx(torch.device("cuda", 0))
+    x, y = rng.random((n, 2)), rng.random((2, n))
+
+    def flags(x, y):
+        dx, dy = ctx.upload(x), ctx.upload(y)
+        v = api._input_stats_dev(ctx, dx, n, 2, [dy[0], dy[1]]).cpu().numpy()
+        return v[:8], list(v[8:])
+
+    st, fl = flags(x, y)
+    assert fl == [0, 0, 0, 0]
+    np.testing.assert_array_equal(st, api._point_stats(ctx, ctx.upload(x), n, 2).ravel())
+    for k, (bad, where) in enumerate([(np.nan, 0), (-np.inf, 0), (np.nan, 1), (np.inf, 1)]):
+        xx, yy = x.copy(), y.copy()
+        if where == 0:
+            xx[n - 1, 1] = bad
+        else:
+            yy[1, n - 1] = bad
+        assert flags(xx, yy)[1] == [float(j == k) for j in range(4)]
