@@ -13,6 +13,7 @@ CUDA library through its C ABI (``_lib``):
 from __future__ import annotations
 
 import copy
+import functools
 import math
 import time
 import warnings
@@ -153,9 +154,15 @@ def _one_se_rule(scores, errs, bandwidths, prefer_smaller: bool, dstd: float = 1
 # ---------------------------------------------------------------------------
 # Device context
 # ---------------------------------------------------------------------------
+_have_cuda = False
+
+
 def _device(options) -> torch.device:
-    if not torch.cuda.is_available():
-        raise RuntimeError("fastlpr_b200 needs a CUDA device (no CPU fallback)")
+    global _have_cuda
+    if not _have_cuda:
+        if not torch.cuda.is_available():
+            raise RuntimeError("fastlpr_b200 needs a CUDA device (no CPU fallback)")
+        _have_cuda = True
     dev = options.get("device", None) if options else None
     if dev is None:
         return torch.device("cuda", torch.cuda.current_device())
@@ -170,7 +177,8 @@ class _Ctx:
         self.index = device.index if device.index is not None else torch.cuda.current_device()
         self.lib = _lib.load()
         self.handle = _lib.handle(self.index)
-        self.stream = torch.cuda.current_stream(device).cuda_stream
+        torch.cuda.init()
+        self.stream = torch._C._cuda_getCurrentRawStream(self.index)
 
     def empty(self, shape, dtype=torch.float64):
         return torch.empty(shape, dtype=dtype, device=self.device)
@@ -312,10 +320,11 @@ class _Geom:
     xmin: np.ndarray
     xmax: np.ndarray
     accuracy: int = 4
+    tab: Optional["_GridTables"] = None
 
     @property
     def M(self) -> int:
-        return int(np.prod(self.G))
+        return int(np.prod(self.G)) if self.tab is None else self.tab.M
 
 
 def _grid_params(G: np.ndarray, flag_power2: bool):
@@ -331,6 +340,33 @@ def _grid_params(G: np.ndarray, flag_power2: bool):
     qout[0] = np.ceil((L - G) / 2).astype(int)
     qout[1] = qout[0] + G - 1
     return L, qin, qout
+
+
+class _GridTables:
+    """What depends on the grid's shape alone: padding, crop windows, knot
+    constants, and the arguments of the library calls made from them."""
+
+    def __init__(self, G: np.ndarray, flag_power2: bool):
+        self.G = np.array(G)
+        self.L, self.qin, self.qout = _grid_params(self.G, flag_power2)
+        self.ks, self.r0, self.hx = _knot_consts(self.G, self.L, self.qin)
+        for v in (self.G, self.L, self.qin, self.qout, self.ks, self.r0, self.hx):
+            v.setflags(write=False)
+        self.M = int(np.prod(self.G))
+        self.cells = int(np.prod(self.L))
+        self.half = self.cells // int(self.L[-1]) * (int(self.L[-1]) // 2 + 1)
+        self.G_c, self.L_c, self.q_c = _lib.ivec(self.G), _lib.ivec(self.L), _lib.ivec(self.qout[0])
+        self.lq = (self.G_c, self.L_c, self.q_c)
+        self.knot_c = (_lib.dvec(self.ks), _lib.dvec(self.r0), _lib.dvec(self.hx))
+
+
+@functools.lru_cache(maxsize=256)
+def _tables_of(shape: Tuple[int, ...], flag_power2: bool) -> _GridTables:
+    return _GridTables(np.array(shape), flag_power2)
+
+
+def _grid_tables(G, flag_power2: bool) -> _GridTables:
+    return _tables_of(tuple(int(v) for v in G), bool(flag_power2))
 
 
 def _point_stats_dev(ctx: _Ctx, dx: torch.Tensor, n: int, d: int) -> torch.Tensor:
@@ -384,37 +420,34 @@ def _knot_consts(G: np.ndarray, L: np.ndarray, qin: np.ndarray):
 
 def _make_geom(stats: np.ndarray, n: int, d: int, G: np.ndarray, accuracy: int,
                flag_power2: bool) -> _Geom:
+    tab = _grid_tables(G, flag_power2)
     xmin, xmax, mean, m2 = stats[0].copy(), stats[1].copy(), stats[2].copy(), stats[3].copy()
-    std = np.sqrt(m2 / (n - 1)) if n > 1 else np.full(d, np.nan)
-    std[std == 0] = 1.0
-    xs_min = (xmin - mean) / std                        # model.py:58-68
-    xs_max = (xmax - mean) / std
-    center = (xs_max + xs_min) / 2
-    lo = xs_min - center
-    hi = xs_max - center
-    L, qin, qout = _grid_params(G, flag_power2)
-    kmap = np.zeros((d, 9))
-    ks_all, r0_all, hx_all = _knot_consts(G, L, qin)       # convolution.py:190-208
+    rows = []
     for a in range(d):
-        scale = hi[a] - lo[a]
+        # float arithmetic on the scalars of one axis (the operations and the
+        # order of the device's flpr_knot_map)
+        mu = float(mean[a])
+        sd = math.sqrt(float(m2[a]) / (n - 1)) if n > 1 else math.nan
+        if sd == 0:
+            sd = 1.0
+        xs_min = (float(xmin[a]) - mu) / sd                 # model.py:58-68
+        xs_max = (float(xmax[a]) - mu) / sd
+        center = (xs_max + xs_min) / 2
+        lo, hi = xs_min - center, xs_max - center
+        scale = hi - lo
         if scale == 0:
             scale = 1.0
-        ks, r0 = ks_all[a], r0_all[a]
-
-        def chain(v):
-            xn = (np.float64(v) - lo[a]) / scale * ks + r0
-            xn = xn + 0.5
-            xn = np.mod(xn, 1.0)
-            return xn - 0.5
-
-        kmin = (chain(lo[a]) + chain(hi[a])) * 0.5 - 0.5       # nufftn_type1.py:164-166
-        shift = -0.5 - kmin
-        hx = 2 * np.pi / L[a]
-        kmap[a] = [mean[a], std[a], center[a], lo[a], scale, ks, r0, shift, hx]
-    msp, tau, _, _ = _spread_params(L, kmap, accuracy)
-    return _Geom(n=n, d=d, G=G, L=L, qin=qin, qout=qout, msp=msp, tau=tau, kmap=kmap, lo=lo,
-                 hi=hi, mean=mean, std=std, center=center, xmin=xmin, xmax=xmax,
-                 accuracy=int(accuracy))
+        ks, r0 = float(tab.ks[a]), float(tab.r0[a])        # convolution.py:190-208
+        c0 = ((lo - lo) / scale * ks + r0 + 0.5) % 1.0 - 0.5
+        c1 = ((hi - lo) / scale * ks + r0 + 0.5) % 1.0 - 0.5
+        kmin = (c0 + c1) * 0.5 - 0.5                        # nufftn_type1.py:164-166
+        rows.append((mu, sd, center, lo, scale, ks, r0, -0.5 - kmin, float(tab.hx[a]), hi))
+    r = np.array(rows)
+    msp, tau, _, kmap = _spread_params(tab.L, r[:, :9], accuracy)
+    kmap[:, 8] = tab.hx                    # no oversampling
+    return _Geom(n=n, d=d, G=tab.G, L=tab.L, qin=tab.qin, qout=tab.qout, msp=msp, tau=tau,
+                 kmap=kmap, lo=r[:, 3].copy(), hi=r[:, 9].copy(), mean=mean, std=r[:, 1].copy(),
+                 center=r[:, 2].copy(), xmin=xmin, xmax=xmax, accuracy=int(accuracy), tab=tab)
 
 
 def _design_powers(d: int, order: int) -> List[Tuple[int, ...]]:
@@ -444,21 +477,28 @@ def _element_powers(d: int, order: int) -> List[Tuple[int, ...]]:
     return [tuple(a + b for a, b in zip(pw[i], pw[j])) for j in range(nt) for i in range(j, nt)]
 
 
+def _upload_bandwidths(ctx: _Ctx, bw: np.ndarray) -> Tuple[torch.Tensor, torch.Tensor]:
+    """The (H, d) bandwidths and their sums over the axes, in one upload."""
+    H, d = bw.shape
+    v = ctx.upload(np.concatenate([bw.ravel(), np.sum(bw, axis=1)]))
+    return v, v[H * d:]
+
+
 def _kernel_factors(ctx: _Ctx, geom: _Geom, bw: np.ndarray, npow: int):
-    """Per-axis kernel spectra F and the a=0 grid sums (convolution.py:318-652)."""
+    """Per-axis kernel spectra F and the a=0 grid sums (convolution.py:318-652),
+    and the bandwidths' sums over the axes."""
     H = bw.shape[0]
-    d = geom.d
-    dh = ctx.upload(np.ascontiguousarray(bw))
-    nF = int(sum(H * npow * int(geom.L[a]) for a in range(d)))
-    F = ctx.empty((nF, 2))
+    d, tab = geom.d, geom.tab
+    dh, hsum = _upload_bandwidths(ctx, bw)
+    F = ctx.empty((H * npow * int(sum(tab.L)), 2))
     sum0 = ctx.empty((d, H))
-    ws = ctx.ws(ctx.lib.flpr_kernel_factors_ws(ctx.handle, d, _lib.ivec(geom.L), H, npow))
-    ctx.check(ctx.lib.flpr_kernel_factors(ctx.handle, d, _lib.ivec(geom.G), _lib.ivec(geom.L),
+    ws = ctx.ws(ctx.lib.flpr_kernel_factors_ws(ctx.handle, d, tab.L_c, H, npow))
+    ctx.check(ctx.lib.flpr_kernel_factors(ctx.handle, d, tab.G_c, tab.L_c,
                                           _lib.dvec(geom.lo), _lib.dvec(geom.hi), H,
                                           dh.data_ptr(), npow, F.data_ptr(), sum0.data_ptr(),
                                           ws.data_ptr(), ws.numel(), ctx.stream),
               "flpr_kernel_factors")
-    return F, sum0
+    return F, sum0, hsum
 
 
 def _kernel_sums_host(geom: _Geom, bw: np.ndarray) -> np.ndarray:
@@ -483,8 +523,11 @@ def _separable_kernel_sums(geom: _Geom, bw: np.ndarray, norm: float) -> np.ndarr
     get the exact sums."""
     peak = np.ones(bw.shape[0])
     for a in range(geom.d):
-        g = np.linspace(geom.lo[a], geom.hi[a], int(geom.G[a]))
-        u = np.min(np.abs(g)) / bw[:, a]
+        # the grid point nearest to zero (of the data's mid-range)
+        lo, cells = float(geom.lo[a]), int(geom.G[a]) - 1
+        step = (float(geom.hi[a]) - lo) / cells if cells else 0.0
+        at = min(max(int(round(-lo / step)), 0), cells) if step > 0 else 0
+        u = abs(lo + at * step) / bw[:, a]
         peak = peak * (np.exp(-0.5 * (u * u)) / bw[:, a])
     sums = peak / norm
     low = np.where(sums < EPS * 20)[0]
@@ -500,9 +543,11 @@ class _Kernel:
     of the convolutions that use them."""
 
     def __init__(self, kid: int, data: torch.Tensor, H: int, npow: int, scale: float,
-                 elems: Optional[Dict[Tuple[int, ...], int]] = None):
+                 elems: Optional[Dict[Tuple[int, ...], int]] = None,
+                 hsum: Optional[torch.Tensor] = None):
         self.kid, self.data, self.H, self.npow, self.scale = kid, data, H, npow, scale
         self.elems = elems
+        self.hsum = hsum           # the bandwidths' sums over the axes, on the device
 
     @property
     def separable(self) -> bool:
@@ -512,13 +557,14 @@ class _Kernel:
         return self.data.data_ptr()
 
 
-def _kernel_spectra_full(ctx, geom, bw, powers, kid):
+def _kernel_spectra_full(ctx, geom, bw, powers, kid, dh=None):
     """(len(powers), H, half) complex128 spectra of the radial kernel's
     moment planes (convolution.py:318-652 with kernel.py:159-431)."""
     H, d = bw.shape[0], geom.d
     L = geom.L
     half = int(np.prod(L[:-1])) * (int(L[-1]) // 2 + 1)
-    dh = ctx.upload(np.ascontiguousarray(bw))
+    if dh is None:
+        dh, _ = _upload_bandwidths(ctx, bw)
     K = ctx.empty((len(powers), H, half, 2))
     nitems = len(powers) * H
     ws = ctx.ws(ctx.lib.flpr_kernel_spectra_ws(ctx.handle, d, _lib.ivec(L), nitems))
@@ -534,16 +580,18 @@ def _kernel_spectra_full(ctx, geom, bw, powers, kid):
 def _make_kernel(ctx, geom, bw, npow, kid) -> Tuple[_Kernel, Optional[np.ndarray]]:
     """Kernel spectra for bw; for radial kernels also the order-0 plane sums
     (the DC terms of their spectra), else None."""
-    Lprod = float(np.prod(geom.L.astype(float)))
+    Lprod = float(geom.tab.cells)
     if kid in (0, 1):
-        F, _ = _kernel_factors(ctx, geom, bw, npow)
+        F, _, hsum = _kernel_factors(ctx, geom, bw, npow)
         scale = (1.0 / SQRT_2PI if kid == 0 else 1.0) / Lprod
-        return _Kernel(kid, F, bw.shape[0], npow, scale), None
+        return _Kernel(kid, F, bw.shape[0], npow, scale, hsum=hsum), None
     powers = _element_powers(geom.d, (npow - 1) // 2)
     uniq = sorted(set(powers), key=powers.index)
-    K = _kernel_spectra_full(ctx, geom, bw, uniq, kid)
+    dh, hsum = _upload_bandwidths(ctx, bw)
+    K = _kernel_spectra_full(ctx, geom, bw, uniq, kid, dh)
     sums = K[uniq.index((0,) * geom.d), :, 0, 0].cpu().numpy()
-    return _Kernel(kid, K, bw.shape[0], npow, 1.0 / Lprod, {p: i for i, p in enumerate(uniq)}), sums
+    return _Kernel(kid, K, bw.shape[0], npow, 1.0 / Lprod, {p: i for i, p in enumerate(uniq)},
+                   hsum=hsum), sums
 
 
 def _filter_bandwidths(ctx, geom, bw, npow, kid: int = 0):
@@ -590,6 +638,26 @@ def _spread_params(L: np.ndarray, kmap: np.ndarray, accuracy: int):
     return msp, tau, ratio, kmap
 
 
+class _Column:
+    """One row of a device matrix, by address (the matrix outlives it)."""
+
+    __slots__ = ("ptr",)
+
+    def __init__(self, ptr: int):
+        self.ptr = ptr
+
+    def data_ptr(self) -> int:
+        return self.ptr
+
+
+class _Columns(list):
+    """Device columns with their addresses as one call argument."""
+
+    def __init__(self, cols):
+        super().__init__(cols)
+        self.args = _lib.pvec([c.data_ptr() for c in self])
+
+
 def _spread_fft(ctx: _Ctx, geom: _Geom, dx: torch.Tensor, cols: List[torch.Tensor], prec: int,
                 ev=None, accuracy: Optional[int] = None, ones: bool = True,
                 kmap_dev: Optional[torch.Tensor] = None, keep: Optional[dict] = None):
@@ -604,36 +672,38 @@ def _spread_fft(ctx: _Ctx, geom: _Geom, dx: torch.Tensor, cols: List[torch.Tenso
     acc = geom.accuracy if accuracy is None else int(accuracy)
     msp, tau, ratio, kmap = _spread_params(geom.L, None if kmap_dev is not None else geom.kmap,
                                            acc)
-    Lsp = (geom.L * ratio).astype(int)
     C = (1 if ones else 0) + len(cols)
-    cells = int(np.prod(Lsp))
+    if ratio == 1:
+        Lsp, Lsp_c, cells, half = geom.L, geom.tab.L_c, geom.tab.cells, geom.tab.half
+    else:
+        Lsp = (geom.L * ratio).astype(int)
+        Lsp_c, cells = _lib.ivec(Lsp), int(np.prod(Lsp))
+        half = cells // int(Lsp[-1]) * (int(Lsp[-1]) // 2 + 1)
     real_dt = torch.float32 if prec == _lib.FLPR_PREC_F32 else torch.float64
     grid = ctx.empty((C, cells), dtype=real_dt)
-    ws = ctx.ws(ctx.lib.flpr_spread_ws(d, n, _lib.ivec(Lsp), msp, C, prec))
-    chans = _lib.pvec([c.data_ptr() for c in cols])
+    ws = ctx.ws(ctx.lib.flpr_spread_ws(d, n, Lsp_c, msp, C, prec))
+    chans = cols.args if isinstance(cols, _Columns) else _lib.pvec([c.data_ptr() for c in cols])
     if kmap_dev is not None:
         if ratio != 1:
             raise ValueError("device knot maps serve accuracies up to 6")
-        hx = 2 * np.pi / (ratio * np.asarray(geom.L, dtype=float))
         ctx.check(ctx.lib.flpr_spread_dkmap(d, n, dx.data_ptr(), kmap_dev.data_ptr(),
-                                            _lib.dvec(hx), _lib.ivec(Lsp), msp, _lib.dvec(tau),
+                                            geom.tab.knot_c[2], Lsp_c, msp, _lib.dvec(tau),
                                             C, 1 if ones else 0, chans, grid.data_ptr(), prec,
                                             ws.data_ptr(), ws.numel(), ctx.stream),
                   "flpr_spread_dkmap")
     else:
         ctx.check(ctx.lib.flpr_spread(d, n, dx.data_ptr(), _lib.dvec(kmap.ravel()),
-                                      _lib.ivec(Lsp), msp, _lib.dvec(tau), C, 1 if ones else 0,
-                                      chans, grid.data_ptr(), prec, ws.data_ptr(), ws.numel(),
+                                      Lsp_c, msp, _lib.dvec(tau), C, 1 if ones else 0, chans,
+                                      grid.data_ptr(), prec, ws.data_ptr(), ws.numel(),
                                       ctx.stream), "flpr_spread")
     if keep is not None and ratio == 1:
-        keep.update(ws=ws, d=d, n=n, L=Lsp.copy(), msp=msp, C=C, prec=prec)
+        keep.update(ws=ws, d=d, n=n, L=Lsp, L_c=Lsp_c, cells=cells, msp=msp, C=C, prec=prec)
     del ws
     if ev is not None:
         ev.mark("spread")
-    half = cells // int(Lsp[-1]) * (int(Lsp[-1]) // 2 + 1)
     spec = ctx.empty((C, half, 2), dtype=real_dt)
-    ws = ctx.ws(ctx.lib.flpr_forward_fft_ws(ctx.handle, d, _lib.ivec(Lsp), C, prec))
-    ctx.check(ctx.lib.flpr_forward_fft(ctx.handle, d, _lib.ivec(Lsp), C, grid.data_ptr(),
+    ws = ctx.ws(ctx.lib.flpr_forward_fft_ws(ctx.handle, d, Lsp_c, C, prec))
+    ctx.check(ctx.lib.flpr_forward_fft(ctx.handle, d, Lsp_c, C, grid.data_ptr(),
                                        spec.data_ptr(), prec, ws.data_ptr(), ws.numel(),
                                        ctx.stream), "flpr_forward_fft")
     if ratio > 1:
@@ -667,11 +737,11 @@ def _grid64(ctx: _Ctx, kept: dict, nout: Optional[int] = None) -> torch.Tensor:
     """(nout, cells) FP64 grid of the first nout channels (default all) from
     the exact fixed-point sums of an FP32 spread (flpr_spread_grid64_channels;
     `kept` from _spread_fft)."""
-    cells = int(np.prod(kept["L"]))
+    cells = kept["cells"]
     nout = kept["C"] if nout is None else int(nout)
     out = ctx.empty((nout, cells))
     ws = kept["ws"]
-    ctx.check(ctx.lib.flpr_spread_grid64_channels(kept["d"], kept["n"], _lib.ivec(kept["L"]),
+    ctx.check(ctx.lib.flpr_spread_grid64_channels(kept["d"], kept["n"], kept["L_c"],
                                                   kept["msp"], kept["C"], nout, ws.data_ptr(),
                                                   ws.numel(), out.data_ptr(), ctx.stream),
               "flpr_spread_grid64_channels")
@@ -682,13 +752,11 @@ def _spectra64(ctx: _Ctx, st) -> torch.Tensor:
     """FP64 spectra of every channel (D2Z of the FP64 grid), formed once."""
     if getattr(st, "spec64", None) is None:
         geom, d = st.geom, st.geom.d
-        cells = int(np.prod(geom.L))
-        half = cells // int(geom.L[-1]) * (int(geom.L[-1]) // 2 + 1)
         C = st.grid64.shape[0]
-        spec = ctx.empty((C, half, 2))
-        ws = ctx.ws(ctx.lib.flpr_forward_fft_ws(ctx.handle, d, _lib.ivec(geom.L), C,
+        spec = ctx.empty((C, geom.tab.half, 2))
+        ws = ctx.ws(ctx.lib.flpr_forward_fft_ws(ctx.handle, d, geom.tab.L_c, C,
                                                 _lib.FLPR_PREC_F64))
-        ctx.check(ctx.lib.flpr_forward_fft(ctx.handle, d, _lib.ivec(geom.L), C,
+        ctx.check(ctx.lib.flpr_forward_fft(ctx.handle, d, geom.tab.L_c, C,
                                            st.grid64.data_ptr(), spec.data_ptr(),
                                            _lib.FLPR_PREC_F64, ws.data_ptr(), ws.numel(),
                                            ctx.stream), "flpr_forward_fft")
@@ -715,63 +783,78 @@ def _sparse_bandwidths(geom, n: int, bw: np.ndarray) -> np.ndarray:
 _CONV_FULL_2D = False
 
 
-def _conv(ctx: _Ctx, geom: _Geom, spec, kern: _Kernel, prods, prec: int, add_eps: bool):
-    """Planes for a product list [(chan, hidx, pow tuple)] -> (nprod, M)."""
-    d = geom.d
-    nprod = len(prods)
+class _Products:
+    """A list of (channel, bandwidth index, exponents) products and the call
+    arguments made from it."""
+
+    def __init__(self, prods):
+        self.prods = tuple(prods)
+        self.n = len(self.prods)
+        self.chan = _lib.ivec([p[0] for p in self.prods])
+        self.hidx = _lib.ivec([p[1] for p in self.prods])
+        self.pw = _lib.ivec([v for p in self.prods for v in p[2]])
+
+
+@functools.lru_cache(maxsize=64)
+def _s_products(d: int, order: int, H: int) -> Tuple[_Products, Tuple[int, ...]]:
+    """The distinct moment planes of the ones channel for H bandwidths, element
+    major, and which of them each packed S element is."""
+    epw = [tuple(e) for e in _element_powers(d, order)]
+    uniq = sorted(set(epw), key=epw.index)
+    return (_Products((0, h, u) for u in uniq for h in range(H)),
+            tuple(uniq.index(e) for e in epw))
+
+
+@functools.lru_cache(maxsize=64)
+def _t_products(d: int, order: int, Cv: int, H: int) -> _Products:
+    """The products of Cv value channels (1 .. Cv of the spectra) with every
+    design term for H bandwidths: (term, channel, bandwidth)."""
+    terms = [(0,) * d] if order == 0 else _design_powers(d, order)
+    return _Products((1 + c, h, tuple(u)) for u in terms for c in range(Cv) for h in range(H))
+
+
+def _conv(ctx: _Ctx, geom: _Geom, spec, kern: _Kernel, prods: _Products, prec: int,
+          add_eps: bool):
+    """Planes for a list of products -> (nprod, M)."""
+    d, tab = geom.d, geom.tab
+    nprod = prods.n
     real_dt = torch.float32 if prec == _lib.FLPR_PREC_F32 else torch.float64
     out = ctx.empty((nprod, geom.M), dtype=real_dt)
-    chan = [p[0] for p in prods]
     if kern.separable and d == 2 and not _CONV_FULL_2D:
-        hidx = [p[1] for p in prods]
-        pw = [v for p in prods for v in p[2]]
-        ws = ctx.ws(ctx.lib.flpr_conv2d_sep_ws(ctx.handle, _lib.ivec(geom.G), _lib.ivec(geom.L),
-                                               nprod, prec))
-        ctx.check(ctx.lib.flpr_conv2d_sep(ctx.handle, _lib.ivec(geom.G), _lib.ivec(geom.L),
-                                          _lib.ivec(geom.qout[0]), kern.H, kern.npow,
-                                          spec.data_ptr(), kern.data_ptr(), nprod,
-                                          _lib.ivec(chan), _lib.ivec(hidx), _lib.ivec(pw),
-                                          kern.scale, 1 if add_eps else 0, out.data_ptr(), prec,
-                                          ws.data_ptr(), ws.numel(), ctx.stream),
-                  "flpr_conv2d_sep")
+        ws = ctx.ws(ctx.lib.flpr_conv2d_sep_ws(ctx.handle, tab.G_c, tab.L_c, nprod, prec))
+        ctx.check(ctx.lib.flpr_conv2d_sep(ctx.handle, *tab.lq, kern.H, kern.npow,
+                                          spec.data_ptr(), kern.data_ptr(), nprod, prods.chan,
+                                          prods.hidx, prods.pw, kern.scale, 1 if add_eps else 0,
+                                          out.data_ptr(), prec, ws.data_ptr(), ws.numel(),
+                                          ctx.stream), "flpr_conv2d_sep")
         return out
-    ws = ctx.ws(ctx.lib.flpr_conv_ws(ctx.handle, d, _lib.ivec(geom.L), nprod, prec))
+    ws = ctx.ws(ctx.lib.flpr_conv_ws(ctx.handle, d, tab.L_c, nprod, prec))
     if kern.separable:
-        hidx = [p[1] for p in prods]
-        pw = [v for p in prods for v in p[2]]
-        ctx.check(ctx.lib.flpr_conv(ctx.handle, d, _lib.ivec(geom.G), _lib.ivec(geom.L),
-                                    _lib.ivec(geom.qout[0]), kern.H, kern.npow, spec.data_ptr(),
-                                    kern.data_ptr(), nprod, _lib.ivec(chan), _lib.ivec(hidx),
-                                    _lib.ivec(pw), kern.scale, 1 if add_eps else 0,
-                                    out.data_ptr(), prec, ws.data_ptr(), ws.numel(), ctx.stream),
-                  "flpr_conv")
+        ctx.check(ctx.lib.flpr_conv(ctx.handle, d, *tab.lq, kern.H, kern.npow, spec.data_ptr(),
+                                    kern.data_ptr(), nprod, prods.chan, prods.hidx, prods.pw,
+                                    kern.scale, 1 if add_eps else 0, out.data_ptr(), prec,
+                                    ws.data_ptr(), ws.numel(), ctx.stream), "flpr_conv")
     else:
-        kidx = [kern.elems[tuple(p[2])] * kern.H + int(p[1]) for p in prods]
-        ctx.check(ctx.lib.flpr_conv_full(ctx.handle, d, _lib.ivec(geom.G), _lib.ivec(geom.L),
-                                         _lib.ivec(geom.qout[0]), len(kern.elems) * kern.H,
-                                         spec.data_ptr(), kern.data_ptr(), nprod,
-                                         _lib.ivec(chan), _lib.ivec(kidx), kern.scale,
-                                         1 if add_eps else 0, out.data_ptr(), prec,
-                                         ws.data_ptr(), ws.numel(), ctx.stream), "flpr_conv_full")
+        kidx = [kern.elems[p[2]] * kern.H + p[1] for p in prods.prods]
+        ctx.check(ctx.lib.flpr_conv_full(ctx.handle, d, *tab.lq, len(kern.elems) * kern.H,
+                                         spec.data_ptr(), kern.data_ptr(), nprod, prods.chan,
+                                         _lib.ivec(kidx), kern.scale, 1 if add_eps else 0,
+                                         out.data_ptr(), prec, ws.data_ptr(), ws.numel(),
+                                         ctx.stream), "flpr_conv_full")
     return out
 
 
-def _conv_s(ctx: _Ctx, geom: _Geom, spec, kern: _Kernel, hks, epw, prec: int,
+def _conv_s(ctx: _Ctx, geom: _Geom, spec, kern: _Kernel, H: int, order: int, prec: int,
             add_eps: bool) -> torch.Tensor:
-    """The moment planes S of the ones channel for the bandwidth rows `hks`
-    and every element power in `epw` -> (len(epw) * len(hks), M), element
+    """The moment planes S of the ones channel for the kernel's first H
+    bandwidths and every packed element -> (elements * H, M), element
     major.  Elements with the same power (order 2: 21 elements, 15 powers)
     are convolved once and their planes repeated."""
-    uniq = []
-    for e in epw:
-        if tuple(e) not in uniq:
-            uniq.append(tuple(e))
-    H = len(hks)
-    out = _conv(ctx, geom, spec, kern, [(0, hk, u) for u in uniq for hk in hks], prec, add_eps)
-    if len(uniq) == len(epw):
+    prods, which = _s_products(geom.d, order, H)
+    out = _conv(ctx, geom, spec, kern, prods, prec, add_eps)
+    if prods.n == len(which) * H:
         return out
-    blocks = [out[uniq.index(tuple(e)) * H:(uniq.index(tuple(e)) + 1) * H] for e in epw]
-    return torch.cat(blocks, dim=0)
+    return torch.cat([out[k * H:(k + 1) * H] for k in which], dim=0)
 
 
 def _precision(opts, dims: Optional[int] = None) -> int:
@@ -821,9 +904,10 @@ def _check_interp_methods(opts, dims: int, n: int) -> Dict[str, str]:
     out = {"gcv": spline.check_method("gcv_interp_method", opts.get("gcv_interp_method", default)),
            "dof": spline.check_method("dof_interp_method", opts.get("dof_interp_method", default)),
            "output": spline.check_method("interp_method", opts.get("interp_method", "linear"))}
-    G = _grid_shape(opts, n, dims)
-    if "cubic" in out.values() and np.any(G < 4):
-        raise ValueError(f"cubic interpolation needs at least 4 grid points per axis, got N={G}")
+    if "cubic" in out.values():
+        G = _grid_shape(opts, n, dims)
+        if np.any(G < 4):
+            raise ValueError(f"cubic interpolation needs at least 4 grid points per axis, got N={G}")
     return out
 
 
@@ -1060,16 +1144,19 @@ def _prepare_lpr(ctx, x_arr, y_arr, dy, opts, order, prec, variance, y_is_comple
     G = _grid_shape(opts, n, d)
     accuracy = int(opts["accuracy"])
     flag_power2 = bool(opts.get("flag_power2", True))
+    tab = _grid_tables(G, flag_power2)
     calc_dof = bool(opts.get("calc_dof", True))
     if calc_dof:
         if probes is None:
             probes = _probes(ctx, n, int(opts.get("num_dof_sample", 10)),
                              opts.get("dof_seed", 42), opts.get("random_matrix", None))
         ptens, R = probes
-        pcols = [ptens[r] for r in range(R)]
+        p0, pstep = ptens.data_ptr(), ptens.stride(0) * 8
+        pcols = [_Column(p0 + r * pstep) for r in range(R)]
     else:
         R = 0
         pcols = []
+    vcols = _Columns(ycols + pcols)
     # The user's accuracy applies to the response channels only (their
     # transform in nufft_regression_with_precomputed_kdf, api.py:640); the
     # design planes (compute_design_matrix, api.py:571) and the probes
@@ -1086,16 +1173,13 @@ def _prepare_lpr(ctx, x_arr, y_arr, dy, opts, order, prec, variance, y_is_comple
         st_host = _to_host(st_dev)
         st_ready = torch.cuda.Event()
         st_ready.record()
-        L, qin, _ = _grid_params(G, flag_power2)
-        ks, r0, hx = _knot_consts(G, L, qin)
         kmap_dev = ctx.empty(9 * d)
-        ctx.check(lib.flpr_knot_map(d, n, st_dev.data_ptr(), _lib.dvec(ks), _lib.dvec(r0),
-                                    _lib.dvec(hx), kmap_dev.data_ptr(), ctx.stream),
-                  "flpr_knot_map")
+        ctx.check(lib.flpr_knot_map(d, n, st_dev.data_ptr(), *tab.knot_c, kmap_dev.data_ptr(),
+                                    ctx.stream), "flpr_knot_map")
         if hook is not None:
             hook(dx, ycols, None, n, d, d_stats=st_dev[:2 * d])
-        pre = SimpleNamespace(n=n, d=d, L=L, accuracy=accuracy, kmap=None)
-        spec = _spread_fft(ctx, pre, dx, ycols + pcols, prec, ev, kmap_dev=kmap_dev, keep=kept)
+        pre = SimpleNamespace(n=n, d=d, L=tab.L, tab=tab, accuracy=accuracy, kmap=None)
+        spec = _spread_fft(ctx, pre, dx, vcols, prec, ev, kmap_dev=kmap_dev, keep=kept)
         st_ready.synchronize()
         stats, flags = _split_stats(st_host.numpy(), d)
     elif checked:
@@ -1110,7 +1194,7 @@ def _prepare_lpr(ctx, x_arr, y_arr, dy, opts, order, prec, variance, y_is_comple
         if hook is not None:
             hook(dx, ycols, stats, n, d)
         if geom.accuracy == acc_default:
-            spec = _spread_fft(ctx, geom, dx, ycols + pcols, prec, ev, keep=kept)
+            spec = _spread_fft(ctx, geom, dx, vcols, prec, ev, keep=kept)
         else:
             spec_s = _spread_fft(ctx, geom, dx, pcols, prec, ev, accuracy=acc_default, ones=True)
             spec_y = _spread_fft(ctx, geom, dx, ycols, prec, ev, accuracy=geom.accuracy,
@@ -1125,7 +1209,7 @@ def _prepare_lpr(ctx, x_arr, y_arr, dy, opts, order, prec, variance, y_is_comple
         n=n, d=d, dx=dx, ycols=ycols, pcols=pcols, R=R, ny=ny, y_raw_dev=y_raw_dev,
         stats=stats, geom=geom, spec=spec, calc_dof=calc_dof, order=order, prec=prec,
         dy=dy, variance=variance, y_is_complex=y_is_complex, opts=opts,
-        axes_raw=axes_raw, ax_arg=_lib.dvec(_axes_arg(axes_raw)), G_arg=_lib.ivec(geom.G),
+        axes_raw=axes_raw, ax_arg=_lib.dvec(_axes_arg(axes_raw)), G_arg=tab.G_c, probes=probes if calc_dof else None,
         methods=methods, spl=None, kid=_kernel_id(opts),
         dual=(calc_dof and ny <= 4 and not opts.get("_direct_reduce", False)
               and methods["gcv"] == "linear" and methods["dof"] == "linear"), Q=None))
@@ -1134,7 +1218,7 @@ def _prepare_lpr(ctx, x_arr, y_arr, dy, opts, order, prec, variance, y_is_comple
         if order == 2 or sparse_any:
             # the exact FP64 grid for FP64 planes; the ones channel alone
             # when only the order-2 moment planes need it (_evaluate_device)
-            Lq = (_lib.ivec(geom.G), _lib.ivec(geom.L), _lib.ivec(geom.qout[0]))
+            Lq = geom.tab.lq
             ones_only = (order == 2 and not sparse_any and d == 2 and st.dual
                          and st.kid in (0, 1) and not opts.get("_no_fused", False)
                          and lib.flpr_lpr2d_fused_supported(*Lq, 1, 2, ny + R) == 1)
@@ -1151,11 +1235,11 @@ def _prepare_lpr(ctx, x_arr, y_arr, dy, opts, order, prec, variance, y_is_comple
         st.sq = ctx.empty(Cv)
         if kept and d <= 2 and kept["C"] == 1 + Cv:
             # from the spread's tile-sorted records: exact and order-free
-            ws2 = ctx.ws(lib.flpr_deposit_sorted_ws(d, n, _lib.ivec(kept["L"]), kept["msp"],
+            ws2 = ctx.ws(lib.flpr_deposit_sorted_ws(d, n, kept["L_c"], kept["msp"],
                                                     kept["C"]))
-            ctx.check(lib.flpr_deposit_sorted(d, n, dx.data_ptr(), _lib.ivec(kept["L"]),
+            ctx.check(lib.flpr_deposit_sorted(d, n, dx.data_ptr(), kept["L_c"],
                                               kept["msp"], kept["C"], 1,
-                                              _lib.pvec([c.data_ptr() for c in ycols + pcols]),
+                                              vcols.args,
                                               kept["ws"].data_ptr(),
                                               kept["ws"].numel(), st.ax_arg, st.G_arg,
                                               _lib.ivec(_node0_cells(geom)), st.Q.data_ptr(),
@@ -1165,7 +1249,7 @@ def _prepare_lpr(ctx, x_arr, y_arr, dy, opts, order, prec, variance, y_is_comple
             del ws2
         else:
             ctx.check(lib.flpr_deposit(d, n, dx.data_ptr(), st.ax_arg, st.G_arg, Cv,
-                                       _lib.pvec([c.data_ptr() for c in ycols + pcols]),
+                                       vcols.args,
                                        st.Q.data_ptr(), st.Bst.data_ptr(), st.sq.data_ptr(),
                                        ctx.stream), "flpr_deposit")
         ev.mark("deposit")
@@ -1198,7 +1282,7 @@ def _evaluate_device(ctx, st: _LprState, filt, ev) -> dict:
         leading = k64 < len(mask) and bool(np.all(mask[:k64]))
         if st.order == 2:
             # moment planes in FP64, value channels on the fused FP32 path
-            Lq = (_lib.ivec(st.geom.G), _lib.ivec(st.geom.L), _lib.ivec(st.geom.qout[0]))
+            Lq = st.geom.tab.lq
             if ((k64 == 0 or leading) and k64 < len(mask) and st.d == 2 and st.dual
                     and kern0.separable and not st.opts.get("_no_fused", False)
                     and ctx.lib.flpr_lpr2d_fused_supported(*Lq, len(mask) - k64, 2,
@@ -1222,23 +1306,19 @@ def _evaluate_device(ctx, st: _LprState, filt, ev) -> dict:
     geom, spec, opts, calc_dof = st.geom, st.spec, st.opts, st.calc_dof
     ycols, pcols = st.ycols, st.pcols
     npow = 2 * order + 1
-    kern, bw, keep, _ = filt
+    kern, bw, keep, _ = filt            # keep: every row of bw, in order
     H = len(keep)
-    epw = _element_powers(d, order)
-    ns = len(epw)
-    nt = 1 if order == 0 else len(_design_powers(d, order))
-    h_t = list(keep) if calc_dof else [int(keep[0])]
-    Ht = len(h_t)
+    nt = math.comb(d + order, order)
+    ns = nt * (nt + 1) // 2
+    Ht = H if calc_dof else 1
     Cv = ny + R
     M = geom.M
-    Lq = (_lib.ivec(geom.G), _lib.ivec(geom.L), _lib.ivec(geom.qout[0]))
+    Lq = geom.tab.lq
     use_fused = st.dual and kern.separable and _fused_ok(ctx, st, prec, H)
     if not use_fused:
-        S = _conv_s(ctx, geom, spec, kern, [int(hk) for hk in keep], epw, prec, order == 0)
+        S = _conv_s(ctx, geom, spec, kern, H, order, prec, order == 0)
         ev.mark("conv_S")
-        T = _conv(ctx, geom, spec, kern,
-                  [(1 + c, int(hk), epw[i]) for i in range(nt) for c in range(Cv) for hk in h_t],
-                  prec, False)
+        T = _conv(ctx, geom, spec, kern, _t_products(d, order, Cv, Ht), prec, False)
         ev.mark("conv_T")
     bw_k = bw[keep]
     scalar = ctx.empty(1)
@@ -1311,7 +1391,7 @@ def _evaluate_device(ctx, st: _LprState, filt, ev) -> dict:
                                 red[st.methods["dof"]][1].reshape(-1),
                                 red[st.methods["dof"]][2].reshape(-1)])
     return dict(keep=keep, bw_k=bw_k, H=H, m=m, S=S, ns=ns, mstride=mstride, packed=packed,
-                dual=st.dual)
+                dual=st.dual, hsum=kern.hsum)
 
 
 def _stencil_quad(ctx, st, H: int, ny: int, m: torch.Tensor, quad: torch.Tensor) -> None:
@@ -1345,7 +1425,7 @@ def _fused_ok(ctx, st, prec: int, H: int) -> bool:
     """Whether the fused 2-D passes serve this fit in `prec`."""
     if st.d != 2 or st.opts.get("_no_fused", False) or H < 1:
         return False
-    Lq = (_lib.ivec(st.geom.G), _lib.ivec(st.geom.L), _lib.ivec(st.geom.qout[0]))
+    Lq = st.geom.tab.lq
     return ctx.lib.flpr_lpr2d_fused_ex_supported(prec, *Lq, H, st.order, st.ny + st.R) == 1
 
 
@@ -1355,7 +1435,7 @@ def _fused_s_planes(ctx, st, spec, kern: "_Kernel", prec: int) -> torch.Tensor:
     geom, order = st.geom, st.order
     ns = len(_element_powers(st.d, order))
     Cv = st.ny + st.R
-    Lq = (_lib.ivec(geom.G), _lib.ivec(geom.L), _lib.ivec(geom.qout[0]))
+    Lq = geom.tab.lq
     S = ctx.empty((ns, kern.H, geom.M),
                   dtype=torch.float64 if prec == _lib.FLPR_PREC_F64 else torch.float32)
     ws = ctx.ws(ctx.lib.flpr_lpr2d_fused_ex_ws(prec, *Lq, kern.H, order, Cv))
@@ -1383,9 +1463,8 @@ def _evaluate_split(ctx, st: _LprState, filt, k64: int, ev, s64_all: bool = Fals
     H32 = H - k64
     npow = 2 * order + 1
     k32k = _kernel_rows(kern, keep[k64:], geom)
-    epw = _element_powers(d, order)
-    ns = len(epw)
-    nt = 1 if order == 0 else len(_design_powers(d, order))
+    nt = math.comb(d + order, order)
+    ns = nt * (nt + 1) // 2
     Cv = ny + R
     M = geom.M
     F32, F64 = _lib.FLPR_PREC_F32, _lib.FLPR_PREC_F64
@@ -1399,10 +1478,8 @@ def _evaluate_split(ctx, st: _LprState, filt, k64: int, ev, s64_all: bool = Fals
         if fused64:
             S64 = _fused_s_planes(ctx, st, spec64, k64k, F64)
         else:
-            S64 = _conv_s(ctx, geom, spec64, k64k, list(range(k64)), epw, F64, order == 0)
-            T64 = _conv(ctx, geom, spec64, k64k,
-                        [(1 + c, hk, epw[i]) for i in range(nt) for c in range(Cv)
-                         for hk in range(k64)], F64, False)
+            S64 = _conv_s(ctx, geom, spec64, k64k, k64, order, F64, order == 0)
+            T64 = _conv(ctx, geom, spec64, k64k, _t_products(d, order, Cv, k64), F64, False)
         scal64 = ctx.empty(1)
         ctx.check(lib.flpr_scalar_of(order, nt, k64, M, S64.data_ptr(), F64, None,
                                      scal64.data_ptr(), ctx.stream), "flpr_scalar_of")
@@ -1411,7 +1488,7 @@ def _evaluate_split(ctx, st: _LprState, filt, k64: int, ev, s64_all: bool = Fals
     m32 = m.data_ptr() + k64 * M * ny * 8
     dots32 = ctx.empty((Cv, H32))
     scalar = ctx.empty(1)
-    Lq = (_lib.ivec(geom.G), _lib.ivec(geom.L), _lib.ivec(geom.qout[0]))
+    Lq = geom.tab.lq
     use_fused = (d == 2 and not st.opts.get("_no_fused", False)
                  and lib.flpr_lpr2d_fused_supported(*Lq, H32, order, Cv) == 1)
     floor = scal64.data_ptr() if scal64 is not None else None
@@ -1419,7 +1496,7 @@ def _evaluate_split(ctx, st: _LprState, filt, k64: int, ev, s64_all: bool = Fals
         if fused64:
             S32 = _fused_s_planes(ctx, st, spec64, k32k, F64)
         else:
-            S32 = _conv_s(ctx, geom, spec64, k32k, list(range(H32)), epw, F64, order == 0)
+            S32 = _conv_s(ctx, geom, spec64, k32k, H32, order, F64, order == 0)
         ctx.check(lib.flpr_scalar_of(order, nt, H32, M, S32.data_ptr(), F64, floor,
                                      scalar.data_ptr(), ctx.stream), "flpr_scalar_of")
         ws = ctx.ws(lib.flpr_lpr2d_fused_ws(*Lq, H32, order, Cv))
@@ -1439,10 +1516,8 @@ def _evaluate_split(ctx, st: _LprState, filt, k64: int, ev, s64_all: bool = Fals
                                              ws.numel(), ctx.stream), "flpr_lpr2d_fused_floor")
         del ws
     else:
-        S32 = _conv_s(ctx, geom, st.spec, k32k, list(range(H32)), epw, F32, order == 0)
-        T32 = _conv(ctx, geom, st.spec, k32k,
-                    [(1 + c, hk, epw[i]) for i in range(nt) for c in range(Cv) for hk in range(H32)],
-                    F32, False)
+        S32 = _conv_s(ctx, geom, st.spec, k32k, H32, order, F32, order == 0)
+        T32 = _conv(ctx, geom, st.spec, k32k, _t_products(d, order, Cv, H32), F32, False)
         ctx.check(lib.flpr_scalar_of(order, nt, H32, M, S32.data_ptr(), F32, floor,
                                      scalar.data_ptr(), ctx.stream), "flpr_scalar_of")
         ctx.check(lib.flpr_solve_reduce_given(order, nt, H32, H32, M, Cv, S32.data_ptr(),
@@ -1477,7 +1552,8 @@ def _evaluate_split(ctx, st: _LprState, filt, k64: int, ev, s64_all: bool = Fals
     packed = torch.cat([st.sq.reshape(-1), dots.reshape(-1), quad.reshape(-1)])
     S0 = torch.cat(parts_s0 + [S32.view(ns, H32, M)[0].to(torch.float64)], dim=0)
     return dict(keep=keep, bw_k=bw_k, H=H, m=m, S=S0.view(1, H, M), ns=1, mstride=ny,
-                packed=packed, dual=True, fp64_bandwidths=k64, s_planes_fp64=bool(s64_all))
+                packed=packed, dual=True, fp64_bandwidths=k64, s_planes_fp64=bool(s64_all),
+                hsum=kern.hsum)
 
 
 def _evaluate_host(st: _LprState, r: dict, packed: Optional[np.ndarray]) -> dict:
@@ -1540,6 +1616,8 @@ def _finalize_enqueue(ctx, st: _LprState, r: dict, ev, device_select: bool = Fal
             pack = ctx.empty(2 * n * ny + M * (ny + 1) + 4 * H + 1)
         sel_dev = ctx.empty(1, dtype=torch.int32)
         if st.calc_dof:
+            if hsum_dev is None:
+                hsum_dev = r.get("hsum")
             if hsum_dev is None:
                 hs = torch.from_numpy(np.ascontiguousarray(np.sum(r["bw_k"], axis=1))).pin_memory()
                 hsum_dev = hs.to(ctx.device, non_blocking=True)
@@ -1665,17 +1743,17 @@ def _unpack_outputs(st: _LprState, r: dict, pack: torch.Tensor) -> dict:
     {fitted values (n, ny), residuals (n, ny), surface (M, ny), s0 (M), GCV
     arrays (4 H), index}."""
     n, ny, M, H = st.n, st.ny, st.geom.M, r["H"]
+    v = pack.numpy()
 
     def shaped(t, k):
         if st.y_is_complex:
-            t = torch.view_as_complex(t.view(k, st.dy, 2))
-            return t[:, 0] if st.dy == 1 else t
-        return t if ny == 1 else t.view(k, ny)
+            t = t.view(np.complex128)
+        return t if st.dy == 1 else t.reshape(k, st.dy)
 
     a, b, c = n * ny, 2 * n * ny, 2 * n * ny + M * ny
-    return {"yh": shaped(pack[:a], n), "rh": shaped(pack[a:b], n), "gvh": shaped(pack[b:c], M),
-            "s0h": pack[c:c + M], "dn": None,
-            "gcv": pack[c + M:c + M + 4 * H] if st.calc_dof else None, "sel": pack[-1:]}
+    return {"yh": shaped(v[:a], n), "rh": shaped(v[a:b], n), "gvh": shaped(v[b:c], M),
+            "s0h": v[c:c + M], "dn": None,
+            "gcv": v[c + M:c + M + 4 * H] if st.calc_dof else None, "sel": v[-1:]}
 
 
 def _finalize_build(ctx, st: _LprState, r: dict, pend: dict, ev, search,
@@ -1688,20 +1766,20 @@ def _finalize_build(ctx, st: _LprState, r: dict, pend: dict, ev, search,
     if "pack" in pend:
         pend = _unpack_outputs(st, r, pend["pack"])
     if pend.get("sel") is not None:
-        sel = int(pend["sel"].numpy()[0])
+        sel = int(np.asarray(pend["sel"])[0])
         if st.calc_dof:
             if sel < 0:
                 raise ValueError(
                     "All GCV scores are NaN or Inf. Regression failed for all bandwidths. "
                     "Try: (1) Use larger bandwidth h, (2) Increase grid points, "
                     "(3) Check for data quality issues")
-            g4 = pend["gcv"].numpy().reshape(4, r["H"]).copy()
+            g4 = np.asarray(pend["gcv"]).reshape(4, r["H"]).copy()
             gcv = {"gcv_m": g4[0], "gcv_sd": g4[1], "dof": g4[2], "dof_stderr": g4[3]}
         else:
             gcv = None
     else:
         sel, gcv = r["sel"], r["gcv"]
-    yh, rh, gvh = pend["yh"].numpy(), pend["rh"].numpy(), pend["gvh"].numpy()
+    yh, rh, gvh = np.asarray(pend["yh"]), np.asarray(pend["rh"]), np.asarray(pend["gvh"])
     if copy:
         yh, rh, gvh = yh.copy(), rh.copy(), gvh.copy()
     s0h = pend["s0h"]
@@ -1710,7 +1788,7 @@ def _finalize_build(ctx, st: _LprState, r: dict, pend: dict, ev, search,
     # already (n,) / (n, dy), complex where the response is (_result_layout)
     yhat, residuals = yh, rh
     grid_values = gvh.reshape(gshape if dy == 1 else gshape + (dy,))
-    s0 = s0h.numpy().reshape(gshape)
+    s0 = np.asarray(s0h).reshape(gshape)
     if copy:
         s0 = s0.copy()
     ev.mark("download")
@@ -1865,7 +1943,7 @@ def _learned_finish(ctx, st: _LprState, bandwidths: np.ndarray, r: dict, pend: d
               "nlist": nlist, "accepted": False}
     if "pack" in pend:
         pend = _unpack_outputs(st, r, pend["pack"])
-    gcv_m = pend["gcv"].numpy()[:R]
+    gcv_m = np.asarray(pend["gcv"])[:R]
     for walk in range(_MAX_WALKS + 1):
         pos = int(np.argmin(gcv_m))
         if _learned.accept_window(window, pos, nlist):
@@ -2019,16 +2097,35 @@ def _fit_kde(ctx, x_arr, bandwidths, opts, G, prec):
     lib = ctx.lib
     n, d = x_arr.shape
     dx = ctx.upload(x_arr)
-    stats, flags = _split_stats(_input_stats_dev(ctx, dx, n, d, []).cpu().numpy(), d)
+    accuracy, flag_power2 = int(opts["accuracy"]), bool(opts.get("flag_power2", True))
+    st_dev = _input_stats_dev(ctx, dx, n, d, [])
+    st_host = _to_host(st_dev)
+    spec = None
+    if accuracy <= 6:
+        # the knot maps are formed on the device, so the spread and the
+        # transform are enqueued before the statistics reach the host
+        st_ready = torch.cuda.Event()
+        st_ready.record()
+        tab = _grid_tables(G, flag_power2)
+        kmap_dev = ctx.empty(9 * d)
+        ctx.check(lib.flpr_knot_map(d, n, st_dev.data_ptr(), *tab.knot_c, kmap_dev.data_ptr(),
+                                    ctx.stream), "flpr_knot_map")
+        pre = SimpleNamespace(n=n, d=d, L=tab.L, tab=tab, accuracy=accuracy, kmap=None)
+        spec = _spread_fft(ctx, pre, dx, [], prec, kmap_dev=kmap_dev)
+        st_ready.synchronize()
+    else:
+        torch.cuda.current_stream(ctx.device).synchronize()
+    stats, flags = _split_stats(st_host.numpy(), d)
     _raise_nonfinite(flags, [("Input x", 0)], "cv_fastkde")
-    geom = _make_geom(stats, n, d, G, int(opts["accuracy"]), bool(opts.get("flag_power2", True)))
+    geom = _make_geom(stats, n, d, G, accuracy, flag_power2)
     kern, bw, keep, ihbad = _filter_bandwidths(ctx, geom, bandwidths, 1, _kernel_id(opts))
     if len(keep) != bandwidths.shape[0] or bw.shape[0] != bandwidths.shape[0]:
         # the reference indexes its density columns by the unfiltered list here
         raise ValueError("a bandwidth is too small for the KDE grid")
     H = len(keep)
-    spec = _spread_fft(ctx, geom, dx, [], prec)
-    S = _conv(ctx, geom, spec, kern, [(0, int(k), (0,) * d) for k in keep], prec, True)
+    if spec is None:
+        spec = _spread_fft(ctx, geom, dx, [], prec)
+    S = _conv_s(ctx, geom, spec, kern, H, 0, prec, True)
     S64 = S if S.dtype == torch.float64 else S.to(torch.float64)
     # raw grid axes by inverting centring and z-scoring (api.py:1038-1057)
     axes_raw = []
@@ -2044,7 +2141,7 @@ def _fit_kde(ctx, x_arr, bandwidths, opts, G, prec):
     lcv = ctx.empty((H, 2))
     ws = ctx.ws(lib.flpr_kde_ws(n, H, M))
     ctx.check(lib.flpr_kde_lcv(d, n, dx.data_ptr(), _lib.dvec(_axes_arg(axes_raw)),
-                               _lib.ivec(geom.G), H, S64.data_ptr(), dxg, _lib.dvec(k0),
+                               geom.tab.G_c, H, S64.data_ptr(), dxg, _lib.dvec(k0),
                                f.data_ptr(), lcv.data_ptr(), ws.data_ptr(), ws.numel(),
                                ctx.stream), "flpr_kde_lcv")
     # both results into pinned memory with one synchronisation (a pageable

@@ -45,7 +45,10 @@ class GridInterpolant:
         for a in self.grid_axes:
             ax += [float(a[0]), float(a[1] - a[0]) if len(a) > 1 else 1.0]
         self._ax = ax
-        self.bounds = [(a.min(), a.max()) for a in self.grid_axes]
+
+    @property
+    def bounds(self):
+        return [(a.min(), a.max()) for a in self.grid_axes]
 
     def __call__(self, points) -> np.ndarray:
         pts = np.atleast_2d(np.asarray(points, dtype=float))
