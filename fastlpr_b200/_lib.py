@@ -41,6 +41,7 @@ SIGNATURES = [
                                _SZ, _VP]),
     ("flpr_spread_grid64", _I, [_I, _I64, _PI, _I, _I, _VP, _SZ, _VP, _VP]),
     ("flpr_spread_grid64_channels", _I, [_I, _I64, _PI, _I, _I, _I, _VP, _SZ, _VP, _VP]),
+    ("flpr_spread_order", _I, [_I, _I64, _PI, _I, _I, _VP, _SZ, C.POINTER(_VP)]),
     ("flpr_knot_map", _I, [_I, _I64, _VP, _PD, _PD, _PD, _VP, _VP]),
     ("flpr_forward_fft_ws", _SZ, [_VP, _I, _PI, _I, _I]),
     ("flpr_forward_fft", _I, [_VP, _I, _PI, _I, _VP, _VP, _I, _VP, _SZ, _VP]),
@@ -98,6 +99,8 @@ SIGNATURES = [
     ("flpr_spline_eval", _I, [_I, _I64, _VP, _VP, _PI, _I, _VP, _VP, _VP]),
     ("flpr_kde_ws", _SZ, [_I64, _I, _I64]),
     ("flpr_kde_lcv", _I, [_I, _I64, _VP, _PD, _PI, _I, _VP, _D, _PD, _VP, _VP, _VP, _SZ, _VP]),
+    ("flpr_kde_density", _I, [_I, _I64, _PI, _I, _VP, _I, _D, _VP, _VP, _SZ, _VP]),
+    ("flpr_kde_scores", _I, [_I, _I64, _VP, _VP, _PD, _PI, _I, _PD, _VP, _VP, _SZ, _VP]),
     ("flpr_log_shift", _I, [_I64, _VP, _D, _VP, _VP]),
     ("flpr_exp_weighted_sum", _I, [_I64, _VP, _VP, _VP, _VP]),
     ("flpr_bin_moments", _I, [_I, _I64, _VP, _VP, _VP, _VP, _VP]),

@@ -2100,7 +2100,7 @@ def _fit_kde(ctx, x_arr, bandwidths, opts, G, prec):
     accuracy, flag_power2 = int(opts["accuracy"]), bool(opts.get("flag_power2", True))
     st_dev = _input_stats_dev(ctx, dx, n, d, [])
     st_host = _to_host(st_dev)
-    spec = None
+    spec, kept = None, {}
     if accuracy <= 6:
         # the knot maps are formed on the device, so the spread and the
         # transform are enqueued before the statistics reach the host
@@ -2111,7 +2111,7 @@ def _fit_kde(ctx, x_arr, bandwidths, opts, G, prec):
         ctx.check(lib.flpr_knot_map(d, n, st_dev.data_ptr(), *tab.knot_c, kmap_dev.data_ptr(),
                                     ctx.stream), "flpr_knot_map")
         pre = SimpleNamespace(n=n, d=d, L=tab.L, tab=tab, accuracy=accuracy, kmap=None)
-        spec = _spread_fft(ctx, pre, dx, [], prec, kmap_dev=kmap_dev)
+        spec = _spread_fft(ctx, pre, dx, [], prec, kmap_dev=kmap_dev, keep=kept)
         st_ready.synchronize()
     else:
         torch.cuda.current_stream(ctx.device).synchronize()
@@ -2126,7 +2126,6 @@ def _fit_kde(ctx, x_arr, bandwidths, opts, G, prec):
     if spec is None:
         spec = _spread_fft(ctx, geom, dx, [], prec)
     S = _conv_s(ctx, geom, spec, kern, H, 0, prec, True)
-    S64 = S if S.dtype == torch.float64 else S.to(torch.float64)
     # raw grid axes by inverting centring and z-scoring (api.py:1038-1057)
     axes_raw = []
     for a in range(d):
@@ -2140,14 +2139,32 @@ def _fit_kde(ctx, x_arr, bandwidths, opts, G, prec):
     f = ctx.empty((H, M))
     lcv = ctx.empty((H, 2))
     ws = ctx.ws(lib.flpr_kde_ws(n, H, M))
-    ctx.check(lib.flpr_kde_lcv(d, n, dx.data_ptr(), _lib.dvec(_axes_arg(axes_raw)),
-                               geom.tab.G_c, H, S64.data_ptr(), dxg, _lib.dvec(k0),
-                               f.data_ptr(), lcv.data_ptr(), ws.data_ptr(), ws.numel(),
-                               ctx.stream), "flpr_kde_lcv")
-    # both results into pinned memory with one synchronisation (a pageable
-    # copy of the (H, M) densities runs at a fraction of the link speed)
-    lc_h, f_h = _to_host(lcv), _to_host(f)
-    torch.cuda.current_stream(ctx.device).synchronize()
+    ctx.check(lib.flpr_kde_density(d, n, geom.tab.G_c, H, S.data_ptr(), prec, dxg, f.data_ptr(),
+                                   ws.data_ptr(), ws.numel(), ctx.stream), "flpr_kde_density")
+    main = torch.cuda.current_stream(ctx.device)
+    beside = None
+    if f.numel() * 8 >= _STAGE_MIN_BYTES:
+        # large densities go down (into pinned memory) beside the scores
+        beside = torch.cuda.Stream(ctx.device)
+        beside.wait_stream(main)
+        f.record_stream(beside)
+        with torch.cuda.stream(beside):
+            f_h = _to_host(f)
+    order = None
+    if kept:
+        order = _lib.C.c_void_p()
+        ctx.check(lib.flpr_spread_order(d, n, kept["L_c"], kept["msp"], kept["C"],
+                                        kept["ws"].data_ptr(), kept["ws"].numel(),
+                                        _lib.C.byref(order)), "flpr_spread_order")
+    ctx.check(lib.flpr_kde_scores(d, n, dx.data_ptr(), order, _lib.dvec(_axes_arg(axes_raw)),
+                                  geom.tab.G_c, H, _lib.dvec(k0), lcv.data_ptr(), ws.data_ptr(),
+                                  ws.numel(), ctx.stream), "flpr_kde_scores")
+    lc_h = _to_host(lcv)
+    if beside is None:
+        f_h = _to_host(f)
+    else:
+        beside.synchronize()
+    main.synchronize()
     lc = lc_h.numpy()
     lcv_m = lc[:, 0].copy()
     var_l = lc[:, 1] / n

@@ -247,21 +247,23 @@ fit_outputs_kernel(InterpGeom g, int64_t n, const double* __restrict__ x, int ny
 }
 
 // ---- KDE -----------------------------------------------------------------
-__global__ void plane_sum_kernel(int64_t M, const double* __restrict__ s, double* __restrict__ sums) {
+template <typename Real>
+__global__ void plane_sum_kernel(int64_t M, const Real* __restrict__ s, double* __restrict__ sums) {
   __shared__ double sh[32];
   const int h = blockIdx.y;
-  const double* p = s + (int64_t)h * M;
+  const Real* p = s + (int64_t)h * M;
   double a = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < M;
        i += (int64_t)gridDim.x * blockDim.x)
-    a += p[i];
+    a += (double)p[i];
   double t = block_sum(a, sh);
   if (threadIdx.x == 0) atomicAdd(&sums[h], t);
 }
 
 // f (H, M) and its bandwidth-fastest copy fT (M, H), through a 32 x 32 tile:
 // grid (ceil(M / 32), ceil(H / 32)), block (32, 8).
-__global__ void kde_normalize_kernel(int64_t M, int H, const double* __restrict__ s,
+template <typename Real>
+__global__ void kde_normalize_kernel(int64_t M, int H, const Real* __restrict__ s,
                                      const double* __restrict__ sums, double dxprod,
                                      double* __restrict__ f, double* __restrict__ fT) {
   __shared__ double tile[32][33];
@@ -273,8 +275,8 @@ __global__ void kde_normalize_kernel(int64_t M, int H, const double* __restrict_
     const int64_t m = m0 + tx;
     if (h < H && m < M) {
       const int64_t t = (int64_t)h * M + m;
-      const double tot = sums[h] * dxprod;
-      double v = tot > 0.0 ? s[t] / tot : s[t];
+      const double tot = sums[h] * dxprod, sv = (double)s[t];
+      double v = tot > 0.0 ? sv / tot : sv;
       v = v > 0.0 ? v : 0.0;
       f[t] = v;
       tile[hh][tx] = v;
@@ -288,83 +290,99 @@ __global__ void kde_normalize_kernel(int64_t M, int H, const double* __restrict_
   }
 }
 
-constexpr int kLcvGroup = 8;  // bandwidths per LCV pass
+constexpr int kLcvMaxH = 512;     // kernel constants of a launch
+constexpr int kLcvThreads = 256;
 
 struct K0g {
-  double k0[kLcvGroup];
+  double k0[kLcvMaxH];
 };
 
-// LCV terms l = log(max(n/(n-1) (f(x_i) - K0/n), 1e-10)) of a group of up to
-// kLcvGroup bandwidths h0.. from the bandwidth-fastest densities fT (M, H):
-// the trilinear stencil of a point is formed once and each corner's
-// densities of the group are contiguous.  Sums of (l - c) and (l - c)^2
-// with c = l at point 0: the shift keeps the variance free of cancellation
-// (exactly zero when every l is clamped).
-template <int D>
-__global__ void kde_lcv_group_kernel(InterpGeom g, int64_t n, const double* __restrict__ x,
-                                     const double* __restrict__ fT, int H, int h0, int hn, K0g k0,
-                                     double* __restrict__ part) {
-  __shared__ double sh[32];
-  __shared__ double s_c[kLcvGroup], s_k0n[kLcvGroup];
+// LCV terms l = log(max(n/(n-1) (f(x_i) - K0/n), 1e-10)) of LPP bandwidths
+// (chunk blockIdx.y of them) from the bandwidth-fastest densities fT (M, H).
+// A warp forms the stencils of 32 points, one per lane, in shared memory and
+// then takes 32 / LPP points at a time, lane = bandwidth: each corner is one
+// contiguous read of LPP densities (a thread per point with its own eight
+// corners of eight bandwidths touched 32 lines per load).  `order` (may be
+// null): the points in the tile order of the spread, so that the corners of
+// neighbouring points meet in L1.  Sums of (l - c) and (l - c)^2 with c = l
+// at point 0: the shift keeps the variance free of cancellation (exactly
+// zero when every l is clamped).
+template <int D, int LPP>
+__global__ void __launch_bounds__(kLcvThreads)
+kde_lcv_kernel(InterpGeom g, int64_t n, const double* __restrict__ x,
+               const int* __restrict__ order, const double* __restrict__ fT, int H, int h0, int hn,
+               K0g k0, double* __restrict__ part) {
+  constexpr int NC = 1 << D, PPW = 32 / LPP, NW = kLcvThreads / 32;
+  __shared__ __align__(16) double s_w[NW][32 * NC];
+  __shared__ int64_t s_base[NW][32];
+  __shared__ double sh1[NW][LPP], sh2[NW][LPP];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int sub = lane / LPP, j = lane - sub * LPP;
+  const int hl = blockIdx.y * LPP + j;  // among the hn bandwidths from h0 on
+  const bool act = hl < hn;
+  const int h = h0 + (act ? hl : 0);
   const double ratio = (double)n / (double)(n - 1);
-  if (threadIdx.x < kLcvGroup) {
-    const int j = threadIdx.x;
-    const double k0n = j < hn ? k0.k0[j] / (double)n : 0.0;
-    s_k0n[j] = k0n;
-    double c = 0.0;
-    if (j < hn) {
-      StencilD<D> st;
-      make_stencil_d<D>(g, x, 0, st);
-      double v = 0.0;
+  const double k0n = act ? k0.k0[hl] / (double)n : 0.0;
+  const double* fh = fT + h;
+  int64_t coff[NC];  // corner offsets in fT
 #pragma unroll
-      for (int k = 0; k < (1 << D); ++k) v += st.w[k] * fT[st.base[k] * H + h0 + j];
-      double fl = ratio * (v - k0n);
-      if (!(fl > 1e-10)) fl = 1e-10;
-      c = log(fl);
-    }
-    s_c[j] = c;
+  for (int k = 0; k < NC; ++k) {
+    int64_t o = 0;
+#pragma unroll
+    for (int a = 0; a < D; ++a) o = o * g.G[a] + (g.G[a] > 1 ? (k >> (D - 1 - a)) & 1 : 0);
+    coff[k] = o * H;
   }
-  __syncthreads();
-  double s1[kLcvGroup], s2[kLcvGroup];
+  auto term = [&](const double* w, int64_t base) {
+    const double* p = fh + base * H;
+    double v = 0.0;
 #pragma unroll
-  for (int j = 0; j < kLcvGroup; ++j) s1[j] = s2[j] = 0.0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
+    for (int k = 0; k < NC; ++k) v += w[k] * p[coff[k]];
+    double fl = ratio * (v - k0n);
+    if (!(fl > 1e-10)) fl = 1e-10;
+    return log(fl);
+  };
+  auto stage = [&](int64_t i) {  // point i's stencil into this lane's place
     StencilD<D> st;
     make_stencil_d<D>(g, x, i, st);
-    double v[kLcvGroup];
+    s_base[warp][lane] = st.base[0];
 #pragma unroll
-    for (int j = 0; j < kLcvGroup; ++j) v[j] = 0.0;
-#pragma unroll
-    for (int k = 0; k < (1 << D); ++k) {
-      const double* row = fT + st.base[k] * H + h0;
-      const double w = st.w[k];
-#pragma unroll
-      for (int j = 0; j < kLcvGroup; ++j)
-        if (j < hn) v[j] += w * row[j];
-    }
-#pragma unroll
-    for (int j = 0; j < kLcvGroup; ++j) {
-      if (j < hn) {
-        double fl = ratio * (v[j] - s_k0n[j]);
-        if (!(fl > 1e-10)) fl = 1e-10;
-        const double l = log(fl) - s_c[j];
-        s1[j] += l;
-        s2[j] += l * l;
-      }
+    for (int k = 0; k < NC; ++k) s_w[warp][lane * NC + k] = st.w[k];
+  };
+  if (lane == 0) stage(0);
+  __syncwarp();
+  const double c = term(s_w[warp], s_base[warp][0]);
+  double s1 = 0.0, s2 = 0.0;
+  const int64_t nwarp = (int64_t)gridDim.x * NW;
+  for (int64_t b = ((int64_t)blockIdx.x * NW + warp) * 32; b < n; b += nwarp * 32) {
+    const int cnt = (int)min((int64_t)32, n - b);
+    __syncwarp();
+    if (lane < cnt) stage(order ? order[b + lane] : b + lane);
+    __syncwarp();
+    for (int r = sub; r < cnt; r += PPW) {
+      const double l = term(s_w[warp] + r * NC, s_base[warp][r]) - c;
+      s1 += l;
+      s2 += l * l;
     }
   }
 #pragma unroll
-  for (int j = 0; j < kLcvGroup; ++j) {
-    if (j < hn) {  // hn is the same for the whole block
-      const double a = block_sum(s1[j], sh);
-      if (threadIdx.x == 0) atomicAdd(&part[3 * (h0 + j)], a);
-      const double b = block_sum(s2[j], sh);
-      if (threadIdx.x == 0) {
-        atomicAdd(&part[3 * (h0 + j) + 1], b);
-        if (blockIdx.x == 0) part[3 * (h0 + j) + 2] = s_c[j];
-      }
+  for (int o = 16; o >= LPP; o >>= 1) {
+    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+  }
+  if (lane < LPP) {
+    sh1[warp][j] = s1;
+    sh2[warp][j] = s2;
+  }
+  __syncthreads();
+  if (warp == 0 && lane < LPP && act) {
+    double a = 0.0, q = 0.0;
+    for (int w = 0; w < NW; ++w) {
+      a += sh1[w][j];
+      q += sh2[w][j];
     }
+    atomicAdd(&part[3 * h], a);
+    atomicAdd(&part[3 * h + 1], q);
+    if (blockIdx.x == 0) part[3 * h + 2] = c;
   }
 }
 
@@ -554,6 +572,12 @@ static void launch_outputs(const InterpGeom& g, int64_t n, const double* x, int 
                                                      sel, yc, yhat, res, surf, s0, sel_out);
 }
 
+// The bandwidth-fastest densities (M, H) in the workspace of flpr_kde_ws.
+static double* kde_transposed(void* ws, int H) {
+  return reinterpret_cast<double*>(static_cast<char*>(ws) + align_up(sizeof(double) * (size_t)H) +
+                                   align_up(sizeof(double) * 3 * (size_t)H));
+}
+
 }  // namespace flpr
 
 using namespace flpr;
@@ -740,42 +764,84 @@ size_t flpr_kde_ws(int64_t n, int H, int64_t M) {
 int flpr_kde_lcv(int d, int64_t n, const double* d_x, const double* h_ax, const int* h_G, int H,
                  const double* d_s, double dxprod, const double* h_k0, double* d_f, double* d_lcv,
                  void* d_ws, size_t ws_bytes, void* stream) {
+  FLPR_TRY(flpr_kde_density(d, n, h_G, H, d_s, FLPR_PREC_F64, dxprod, d_f, d_ws, ws_bytes, stream));
+  return flpr_kde_scores(d, n, d_x, nullptr, h_ax, h_G, H, h_k0, d_lcv, d_ws, ws_bytes, stream);
+}
+
+int flpr_kde_density(int d, int64_t n, const int* h_G, int H, const void* d_s, int s_prec,
+                     double dxprod, double* d_f, void* d_ws, size_t ws_bytes, void* stream) {
   InterpGeom g;
-  FLPR_TRY(make_geom(g, d, h_ax, h_G));
-  FLPR_CHECK_ARG(n >= 2 && H >= 1, "kde_lcv: n=%lld H=%d", (long long)n, H);
+  double ax[6] = {0, 1, 0, 1, 0, 1};
+  FLPR_TRY(make_geom(g, d, ax, h_G));
+  FLPR_CHECK_ARG(n >= 2 && H >= 1, "kde_density: n=%lld H=%d", (long long)n, H);
+  FLPR_CHECK_ARG(s_prec == FLPR_PREC_F32 || s_prec == FLPR_PREC_F64, "kde_density: precision");
   if (ws_bytes < flpr_kde_ws(n, H, g.M)) {
-    set_error("kde_lcv: workspace too small");
+    set_error("kde_density: workspace too small");
     return FLPR_ERR_WORKSPACE;
   }
   cudaStream_t s = as_stream(stream);
   double* sums = static_cast<double*>(d_ws);
-  double* part = reinterpret_cast<double*>(static_cast<char*>(d_ws) +
-                                           align_up(sizeof(double) * (size_t)H));
+  double* fT = kde_transposed(d_ws, H);
   FLPR_CUDA(cudaMemsetAsync(sums, 0, sizeof(double) * H, s));
-  FLPR_CUDA(cudaMemsetAsync(part, 0, sizeof(double) * 3 * H, s));
   int gb = pt_blocks(g.M, 2);
   gb = (gb + H - 1) / H;
   if (gb < 4) gb = 4;
-  plane_sum_kernel<<<dim3(gb, H), 256, 0, s>>>(g.M, d_s, sums);
+  FLPR_CHECK_ARG((g.M + 31) / 32 < ((int64_t)1 << 31), "kde_density: grid too large");
+  const dim3 ng((unsigned)((g.M + 31) / 32), (unsigned)((H + 31) / 32));
+  if (s_prec == FLPR_PREC_F32) {
+    plane_sum_kernel<float><<<dim3(gb, H), 256, 0, s>>>(g.M, (const float*)d_s, sums);
+    FLPR_LAUNCH_CHECK();
+    kde_normalize_kernel<float><<<ng, dim3(32, 8), 0, s>>>(g.M, H, (const float*)d_s, sums, dxprod,
+                                                           d_f, fT);
+  } else {
+    plane_sum_kernel<double><<<dim3(gb, H), 256, 0, s>>>(g.M, (const double*)d_s, sums);
+    FLPR_LAUNCH_CHECK();
+    kde_normalize_kernel<double><<<ng, dim3(32, 8), 0, s>>>(g.M, H, (const double*)d_s, sums,
+                                                            dxprod, d_f, fT);
+  }
   FLPR_LAUNCH_CHECK();
-  double* fT = reinterpret_cast<double*>(static_cast<char*>(d_ws) +
-                                         align_up(sizeof(double) * (size_t)H) +
-                                         align_up(sizeof(double) * 3 * (size_t)H));
-  FLPR_CHECK_ARG((g.M + 31) / 32 < ((int64_t)1 << 31), "kde_lcv: grid too large");
-  kde_normalize_kernel<<<dim3((unsigned)((g.M + 31) / 32), (unsigned)((H + 31) / 32)),
-                         dim3(32, 8), 0, s>>>(g.M, H, d_s, sums, dxprod, d_f, fT);
-  FLPR_LAUNCH_CHECK();
-  const int ngroups = (H + kLcvGroup - 1) / kLcvGroup;
-  const int per_g = (4 * sm_count() + ngroups - 1) / ngroups;
-  for (int h0 = 0; h0 < H; h0 += kLcvGroup) {
-    const int hn = H - h0 < kLcvGroup ? H - h0 : kLcvGroup;
+  return FLPR_OK;
+}
+
+int flpr_kde_scores(int d, int64_t n, const double* d_x, const int* d_order, const double* h_ax,
+                    const int* h_G, int H, const double* h_k0, double* d_lcv, void* d_ws,
+                    size_t ws_bytes, void* stream) {
+  InterpGeom g;
+  FLPR_TRY(make_geom(g, d, h_ax, h_G));
+  FLPR_CHECK_ARG(n >= 2 && H >= 1, "kde_scores: n=%lld H=%d", (long long)n, H);
+  if (ws_bytes < flpr_kde_ws(n, H, g.M)) {
+    set_error("kde_scores: workspace too small");
+    return FLPR_ERR_WORKSPACE;
+  }
+  cudaStream_t s = as_stream(stream);
+  double* part = reinterpret_cast<double*>(static_cast<char*>(d_ws) +
+                                           align_up(sizeof(double) * (size_t)H));
+  const double* fT = kde_transposed(d_ws, H);
+  FLPR_CUDA(cudaMemsetAsync(part, 0, sizeof(double) * 3 * H, s));
+  for (int h0 = 0; h0 < H; h0 += kLcvMaxH) {
+    const int hn = H - h0 < kLcvMaxH ? H - h0 : kLcvMaxH;
     K0g k0;
-    for (int j = 0; j < kLcvGroup; ++j) k0.k0[j] = j < hn ? h_k0[h0 + j] : 0.0;
+    for (int j = 0; j < hn; ++j) k0.k0[j] = h_k0[h0 + j];
+    // lanes per point: 16 bandwidths unless 8 leave fewer of them idle
+    const bool wide = (hn + 15) / 16 * 16 <= (hn + 7) / 8 * 8;
+    const int chunks = wide ? (hn + 15) / 16 : (hn + 7) / 8;
+    int64_t nb = (8LL * sm_count() + chunks - 1) / chunks;
+    const int64_t most = (n + kLcvThreads - 1) / kLcvThreads;
+    if (nb > most) nb = most;
+    const dim3 grid((unsigned)nb, (unsigned)chunks);
+#define FLPR_LCV(D)                                                                          \
+  if (wide)                                                                                  \
+    kde_lcv_kernel<D, 16><<<grid, kLcvThreads, 0, s>>>(g, n, d_x, d_order, fT, H, h0, hn, k0, \
+                                                       part);                                \
+  else                                                                                       \
+    kde_lcv_kernel<D, 8><<<grid, kLcvThreads, 0, s>>>(g, n, d_x, d_order, fT, H, h0, hn, k0,  \
+                                                      part);
     switch (d) {
-      case 1: kde_lcv_group_kernel<1><<<per_g, 256, 0, s>>>(g, n, d_x, fT, H, h0, hn, k0, part); break;
-      case 2: kde_lcv_group_kernel<2><<<per_g, 256, 0, s>>>(g, n, d_x, fT, H, h0, hn, k0, part); break;
-      default: kde_lcv_group_kernel<3><<<per_g, 256, 0, s>>>(g, n, d_x, fT, H, h0, hn, k0, part); break;
+      case 1: FLPR_LCV(1) break;
+      case 2: FLPR_LCV(2) break;
+      default: FLPR_LCV(3) break;
     }
+#undef FLPR_LCV
     FLPR_LAUNCH_CHECK();
   }
   kde_lcv_finish_kernel<<<(H + 127) / 128, 128, 0, s>>>(H, n, part, d_lcv);

@@ -1334,6 +1334,26 @@ int flpr_spread_grid64_channels(int d, int64_t n, const int* h_L, int msp, int n
   return FLPR_OK;
 }
 
+int flpr_spread_order(int d, int64_t n, const int* h_L, int msp, int nchan, const void* d_ws,
+                      size_t ws_bytes, const int** d_order) {
+  FLPR_CHECK_ARG(d >= 1 && d <= 3, "spread_order: d=%d not in [1,3]", d);
+  FLPR_CHECK_ARG(n >= 1 && nchan >= 1 && nchan <= FLPR_MAX_CHANNELS, "spread_order: n/nchan");
+  FLPR_CHECK_ARG(d_ws != nullptr && d_order != nullptr, "spread_order: null pointer");
+  for (int a = 0; a < d; ++a) FLPR_CHECK_ARG(h_L[a] >= 1, "spread_order: L[%d]=%d", a, h_L[a]);
+  if (ws_bytes < flpr_spread_ws(d, n, h_L, msp, nchan, FLPR_PREC_F32)) {
+    set_error("spread_order: workspace too small");
+    return FLPR_ERR_WORKSPACE;
+  }
+  SpreadGeom g;
+  double tau[3] = {1, 1, 1}, kmap[27] = {0};
+  make_geom(g, d, h_L, msp, tau, kmap);
+  Arena ar(const_cast<void*>(d_ws), ws_bytes);
+  SpreadWs w;
+  spread_layout(ar, d, n, g.ntiles, nchan, g.cells, &w);
+  *d_order = w.rec_idx;
+  return FLPR_OK;
+}
+
 int flpr_knot_map(int d, int64_t n, const double* d_stats, const double* h_ks,
                   const double* h_r0, const double* h_hx, double* d_kmap, void* stream) {
   FLPR_CHECK_ARG(d >= 1 && d <= 3, "knot_map: d=%d not in [1,3]", d);

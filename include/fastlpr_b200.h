@@ -149,6 +149,11 @@ int flpr_spread_grid64(int d, int64_t n, const int* h_L, int msp, int nchan, con
 int flpr_spread_grid64_channels(int d, int64_t n, const int* h_L, int msp, int nchan, int nout,
                                 const void* d_ws, size_t ws_bytes, double* d_grid64,
                                 void* stream);
+/* Where in this workspace the last spread (same d, n, L, msp, nchan) left the
+ * indices of the points in its tile order: *d_order points at n ints on the
+ * device, valid while the workspace is and no other spread uses it. */
+int flpr_spread_order(int d, int64_t n, const int* h_L, int msp, int nchan, const void* d_ws,
+                      size_t ws_bytes, const int** d_order);
 /* Knot maps d_kmap (d x 9) from the point statistics d_stats (4 x d:
  * minimum, maximum, mean, M2 as flpr_point_stats writes them) and the
  * host-known per-axis constants of the grid (ks, r0: the knot range of
@@ -504,6 +509,17 @@ size_t flpr_kde_ws(int64_t n, int H, int64_t M);
 int flpr_kde_lcv(int d, int64_t n, const double* d_x, const double* h_ax, const int* h_G,
                  int H, const double* d_s, double dxprod, const double* h_k0,
                  double* d_f, double* d_lcv, void* d_ws, size_t ws_bytes, void* stream);
+/* flpr_kde_lcv in its two parts, on the same workspace: the densities from
+ * sums in either precision (s_prec: float or double d_s), and the LCV sums
+ * from the densities of the last flpr_kde_density; d_order (n, device; may be
+ * NULL): an order of the points in which neighbours in the list are
+ * neighbours in space (flpr_spread_order), which the reads of the densities
+ * follow. */
+int flpr_kde_density(int d, int64_t n, const int* h_G, int H, const void* d_s, int s_prec,
+                     double dxprod, double* d_f, void* d_ws, size_t ws_bytes, void* stream);
+int flpr_kde_scores(int d, int64_t n, const double* d_x, const int* d_order, const double* h_ax,
+                    const int* h_G, int H, const double* h_k0, double* d_lcv, void* d_ws,
+                    size_t ws_bytes, void* stream);
 
 /* (10) Small elementwise helpers used by the variance mode of
  * api.py:390-396 and api.py:771-786. */

@@ -188,3 +188,18 @@ def test_input_stats_flags(cuda_ok, n):
         else:
             yy[1, n - 1] = bad
         assert flags(xx, yy)[1] == [float(j == k) for j in range(4)]
+
+
+@pytest.mark.parametrize("d,n,G,H", [(1, 40, [30], 1), (1, 3000, [50], 17), (2, 33, [9, 12], 7), (2, 2000, [20, 31], 9),
+                                     (3, 500, [6, 9, 7], 16), (3, 300, [5, 5, 6], 20), (1, 300, [16], 530)])
+def test_density_scores_at_the_edges(cuda_ok, d, n, G, H):
+    """Bandwidths that fill 8 or 16 lanes or not, a last batch of one point,
+    more bandwidths than one launch takes; FP64, so to 1e-9 of the oracle."""
+    import fastlpr_b200
+    rng = np.random.default_rng(13 * n + H)
+    x = rng.standard_normal((n, d))
+    h = np.column_stack([np.linspace(0.3, 1.2, H)] * d)
+    opts = {"N": G if d > 1 else G[0], "precision": "fp64"}
+    k, o = fastlpr_b200.cv_fastkde(x, h, dict(opts)), oracle.cv_fastkde(x, h, {"N": opts["N"]})
+    assert rel_err(k.metadata["fhat_all"], o["fhat_all"]) < 1e-9
+    assert rel_err(k.lcv["lcv_m"], o["lcv_m"]) < 1e-9 and rel_err(k.lcv["lcv_sd"], o["lcv_sd"]) < 1e-9
