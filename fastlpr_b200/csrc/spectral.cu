@@ -104,6 +104,10 @@ struct ConvArgs {
   // crop_kernel, and ceil(2^32 / row length) for the division by it
   int prow, crow;
   unsigned pmagic, cmagic;
+  // 3-D: products of the batch lie side by side within each plane of axis 0
+  // (L0, nb, L1, L2/2+1), and only the kept planes are transformed further
+  // (G0, nb, L1, L2); nb = 0: one product after the other
+  int nb;
 };
 
 // Rows of length `len` per block: about 2048 elements, at most kRowsMax; and
@@ -130,6 +134,7 @@ product_kernel(ConvArgs ca, ProdBatch desc, const typename Cplx<Real>::type* __r
                const double2* __restrict__ F, typename Cplx<Real>::type* __restrict__ out) {
   using C = typename Cplx<Real>::type;
   __shared__ double2 s_k[kRowsMax];
+  __shared__ int64_t s_dst[kRowsMax];
   const ProdDesc pd = desc.p[blockIdx.y];
   const int d = ca.d, Lh = ca.L[d - 1] / 2 + 1;
   const int rows = d == 1 ? 1 : (d == 2 ? ca.L[0] : ca.L[0] * ca.L[1]);
@@ -149,22 +154,24 @@ product_kernel(ConvArgs ca, ProdBatch desc, const typename Cplx<Real>::type* __r
       kr = nr_;
     }
     s_k[threadIdx.x] = make_double2(kr, ki);
+    s_dst[threadIdx.x] = ca.nb ? (((int64_t)om[0] * ca.nb + blockIdx.y) * ca.L[1] + om[1]) * Lh
+                               : (int64_t)blockIdx.y * ca.half + (int64_t)row * Lh;
   }
   __syncthreads();
   const double2* fl = F + ca.foff[d - 1] + ((int64_t)pd.hidx * ca.npow + pd.pw[d - 1]) * ca.L[d - 1];
   const C* src = spec + (int64_t)pd.chan * ca.half + (int64_t)row0 * Lh;
-  C* dst = out + (int64_t)blockIdx.y * ca.half + (int64_t)row0 * Lh;
   const int total = nr * Lh;
 #pragma unroll 4
   for (int e = threadIdx.x; e < total; e += 256) {
     const int r = ca.prow == 1 ? 0 : (int)__umulhi((unsigned)e, ca.pmagic);
-    const double2 k = s_k[r], f = fl[e - r * Lh];
+    const int w = e - r * Lh;
+    const double2 k = s_k[r], f = fl[w];
     const double kr = k.x * f.x - k.y * f.y, ki = k.x * f.y + k.y * f.x;
     const C s = src[e];
     C o;
     o.x = (Real)((double)s.x * kr - (double)s.y * ki);
     o.y = (Real)((double)s.x * ki + (double)s.y * kr);
-    dst[e] = o;
+    out[s_dst[r] + w] = o;
   }
 }
 
@@ -183,12 +190,13 @@ crop_kernel(ConvArgs ca, int p0, const Real* __restrict__ full, int add_eps,
     if (d == 2) src = row + ca.qout[0];
     if (d == 3) {
       const int g0 = row / ca.G[1], g1 = row - g0 * ca.G[1];
-      src = (int64_t)(g0 + ca.qout[0]) * ca.L[1] + g1 + ca.qout[1];
+      src = (ca.nb ? ((int64_t)g0 * ca.nb + blockIdx.y) : (int64_t)(g0 + ca.qout[0])) * ca.L[1] +
+            g1 + ca.qout[1];
     }
     s_src[threadIdx.x] = src * ca.L[d - 1] + ca.qout[d - 1];
   }
   __syncthreads();
-  const Real* src = full + (int64_t)blockIdx.y * ca.cells;
+  const Real* src = full + (ca.nb ? 0 : (int64_t)blockIdx.y * ca.cells);
   Real* dst = out + (int64_t)(p0 + blockIdx.y) * ca.M + (int64_t)row0 * Gl;
   const double eps = 2.220446049250313e-16;
   const int total = nr * Gl;
@@ -605,6 +613,36 @@ int flpr_kernel_factors(flpr_handle_t handle, int d, const int* h_G, const int* 
   return FLPR_OK;
 }
 
+// 3-D inverse transform of nb products in the layout of ConvArgs::nb: axis 0
+// of every column, then axes 1 and 2 of the kept planes (half of the work of
+// those two axes for a grid padded to twice its size).
+static PlanKey conv3_axis0(const int* L, int nb, int prec) {
+  PlanKey k{};
+  k.rank = 1;
+  k.n[0] = L[0];
+  k.type = prec == FLPR_PREC_F32 ? CUFFT_C2C : CUFFT_Z2Z;
+  k.batch = nb * L[1] * (L[2] / 2 + 1);
+  k.stride = k.batch;
+  k.idist = 1;
+  k.odist = 1;
+  k.inverse = 1;
+  return k;
+}
+
+static PlanKey conv3_planes(const int* L, int planes, int prec) {
+  return grid_plan(2, L + 1, prec == FLPR_PREC_F32 ? CUFFT_C2R : CUFFT_Z2D, planes);
+}
+
+// Largest work area of a batch of nb products; G0 is unknown to the size
+// query, whose caller may keep every plane.
+static int conv3_work(flpr_handle_t handle, const int* L, int nb, int prec, size_t* out) {
+  size_t a = 0, b = 0;
+  FLPR_TRY(plans_of(handle).work_size(conv3_axis0(L, nb, prec), &a));
+  FLPR_TRY(plans_of(handle).work_size(conv3_planes(L, nb * L[0], prec), &b));
+  *out = a > b ? a : b;
+  return FLPR_OK;
+}
+
 size_t flpr_conv_ws(flpr_handle_t handle, int d, const int* h_L, int nprod, int prec) {
   if (d < 1 || d > 3 || nprod < 1) return 0;
   int B = conv_batch(d, h_L, nprod, prec);
@@ -619,7 +657,14 @@ size_t flpr_conv_ws(flpr_handle_t handle, int d, const int* h_L, int nprod, int 
   if (plans_of(handle).work_size(grid_plan(d, h_L, type, B), &w1) != FLPR_OK) return 0;
   int tail = nprod % B;
   if (tail && plans_of(handle).work_size(grid_plan(d, h_L, type, tail), &w2) != FLPR_OK) return 0;
-  ar.take<char>(w1 > w2 ? w1 : w2);
+  if (w2 > w1) w1 = w2;
+  if (d == 3) {
+    if (conv3_work(handle, h_L, B, prec, &w2) != FLPR_OK) return 0;
+    if (w2 > w1) w1 = w2;
+    if (tail && conv3_work(handle, h_L, tail, prec, &w2) != FLPR_OK) return 0;
+    if (w2 > w1) w1 = w2;
+  }
+  ar.take<char>(w1);
   return ar.used;
 }
 
@@ -679,6 +724,7 @@ int flpr_conv(flpr_handle_t handle, int d, const int* h_G, const int* h_L, const
       for (int a = 0; a < 3; ++a) pd.pw[a] = a < d ? (unsigned short)h_pow[(p0 + b) * d + a] : 0;
       batch.p[b] = pd;
     }
+    ca.nb = d == 3 ? nb : 0;
     if (prec == FLPR_PREC_F32) {
       product_kernel<float><<<prod_grid(ca, nb), 256, 0, s>>>(ca, batch, (const float2*)d_spec,
                                                               (const double2*)d_F, (float2*)pbuf);
@@ -687,7 +733,14 @@ int flpr_conv(flpr_handle_t handle, int d, const int* h_G, const int* h_L, const
           ca, batch, (const double2*)d_spec, (const double2*)d_F, (double2*)pbuf);
     }
     FLPR_LAUNCH_CHECK();
-    FLPR_TRY(plans_of(handle).exec(grid_plan(d, h_L, ctype, nb), pbuf, rbuf, work, work_bytes, s));
+    if (d == 3) {
+      const size_t plane = (size_t)nb * h_L[1] * (h_L[2] / 2 + 1) * 2 * es;
+      FLPR_TRY(plans_of(handle).exec(conv3_axis0(h_L, nb, prec), pbuf, pbuf, work, work_bytes, s));
+      FLPR_TRY(plans_of(handle).exec(conv3_planes(h_L, nb * h_G[0], prec),
+                                     pbuf + plane * h_qout[0], rbuf, work, work_bytes, s));
+    } else {
+      FLPR_TRY(plans_of(handle).exec(grid_plan(d, h_L, ctype, nb), pbuf, rbuf, work, work_bytes, s));
+    }
     if (prec == FLPR_PREC_F32) {
       crop_kernel<float><<<crop_grid(ca, nb), 256, 0, s>>>(ca, p0, (const float*)rbuf, add_eps,
                                                            (float*)d_out);
