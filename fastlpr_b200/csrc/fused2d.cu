@@ -60,8 +60,11 @@ __device__ __forceinline__ float2 csub(float2 a, float2 b) {
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pack2(a)), "l"(pack2(b)));
   return unpack2(d);
 }
+// The FP32 product with its fused sums spelled out: its rounding must not
+// depend on what the compiler makes of a constant factor.
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+  return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)),
+                     __fmaf_rn(a.y, b.x, __fmul_rn(a.x, b.y)));
 }
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) {
   return make_double2(a.x + b.x, a.y + b.y);
@@ -131,21 +134,42 @@ __host__ __device__ constexpr int buf_stride(int E) {
 // for k1 < E, then tw32[m] = exp(2 pi i m / 32).
 __host__ __device__ constexpr int twiddle_entries(int N) { return N + 32; }
 
-// a * exp(2 pi i m / 32), m known after unrolling: quarter turns are exact.
+// cos(2 pi m / 32), m = 0 .. 8, of which every 32nd root of unity is made.
+__host__ __device__ constexpr double cos32(int m) {
+  return m == 0   ? 1.0
+         : m == 1 ? 0.98078528040323044913
+         : m == 2 ? 0.92387953251128675613
+         : m == 3 ? 0.83146961230254523708
+         : m == 4 ? 0.70710678118654752440
+         : m == 5 ? 0.55557023301960222474
+         : m == 6 ? 0.38268343236508977173
+         : m == 7 ? 0.19509032201612826785
+                  : 0.0;
+}
+__host__ __device__ constexpr double root_re(int m) {
+  return m <= 8 ? cos32(m) : m <= 16 ? -cos32(16 - m) : m <= 24 ? -cos32(m - 16) : cos32(32 - m);
+}
+__host__ __device__ constexpr double root_im(int m) { return root_re((m + 24) & 31); }
+
+// a * exp(2 pi i m / 32), m known after unrolling: quarter turns are exact,
+// the other roots are constants of the instructions (a shared-memory table
+// cost a load for each of the 34 products of a 32-point stage: T row pass of
+// 32 bandwidths on 512^2 1.405 -> 1.373 ms, column passes 768 -> 747 us).
 template <typename V>
-__device__ __forceinline__ V rot32(V a, int m, const V* __restrict__ tw32) {
+__device__ __forceinline__ V rot32(V a, int m) {
+  using R = typename RealOf<V>::T;
   m &= 31;
   if (m == 0) return a;
   if (m == 8) return vmake<V>(-a.y, a.x);
   if (m == 16) return vmake<V>(-a.x, -a.y);
   if (m == 24) return vmake<V>(a.y, -a.x);
-  return cmul(a, tw32[m]);
+  return cmul(a, vmake<V>((R)root_re(m), (R)root_im(m)));
 }
 
 // In-register radix-2 DIF (inverse sign) over the E slots: slot s ends up
 // holding output brev(s).  E <= 32, so every twiddle is a power of W_32.
 template <int E, typename V>
-__device__ __forceinline__ void dif_slots(V (&v)[E], const V* __restrict__ tw32) {
+__device__ __forceinline__ void dif_slots(V (&v)[E]) {
 #pragma unroll
   for (int span = E / 2; span >= 1; span >>= 1) {
 #pragma unroll
@@ -153,7 +177,7 @@ __device__ __forceinline__ void dif_slots(V (&v)[E], const V* __restrict__ tw32)
       if ((s & span) == 0) {
         const V a = v[s], b = v[s + span];
         v[s] = cadd(a, b);
-        v[s + span] = rot32(csub(a, b), (s & (span - 1)) * (16 / span), tw32);
+        v[s + span] = rot32(csub(a, b), (s & (span - 1)) * (16 / span));
       }
     }
   }
@@ -177,7 +201,7 @@ __device__ __forceinline__ void warp_ifft(float2 (&v)[E], const float2* __restri
   constexpr int EB = ilog2(E);
   constexpr int P = 32 / E;
   // DFT over n1 (n = 32 n1 + n2) for each n2 = lane
-  dif_slots<E>(v, tw32);
+  dif_slots<E>(v);
   // twiddle W_N^(n2 k1), k1 = brev(s)
 #pragma unroll
   for (int s = 1; s < E; ++s) v[s] = cmul(v[s], tw2[brev(s, EB) * 32 + lane]);
@@ -211,7 +235,7 @@ __device__ __forceinline__ void warp_ifft(float2 (&v)[E], const float2* __restri
     }
     v[n] = z;
   }
-  dif_slots<E>(v, tw32);
+  dif_slots<E>(v);
 }
 
 // warp_ifft in FP64 (same input and output layout).  The 32 values a lane
@@ -227,7 +251,7 @@ __device__ __forceinline__ void warp_ifft64(double2 (&v)[E], const double2* __re
                                             int lane) {
   constexpr int EB = ilog2(E);
   constexpr int P = 32 / E;
-  dif_slots<E>(v, tw32);
+  dif_slots<E>(v);
 #pragma unroll
   for (int s = 1; s < E; ++s) v[s] = cmul(v[s], tw2[brev(s, EB) * 32 + lane]);
   const int k1 = lane & (E - 1), part = lane >> EB;
@@ -272,7 +296,7 @@ __device__ __forceinline__ void warp_ifft64(double2 (&v)[E], const double2* __re
     }
     __syncwarp();
   }
-  dif_slots<E>(v, tw32);
+  dif_slots<E>(v);
 }
 
 // The inverse transform of the precision's vector type.
