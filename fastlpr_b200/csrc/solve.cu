@@ -111,54 +111,70 @@ __global__ void solve_kernel(int order, int H, int HT, int64_t M, int C,
   }
 }
 
-// Solve fused with the dual-form reductions.  blockIdx.y = bandwidth h < HT.
-// Writes m for the first nkeep channels to mkeep (HT, M, nkeep) and adds
-// dots[c][h] += sum_g m_c(g) Q[g][c] for every channel c < C.
-template <typename Real, int NT>
-__global__ void solve_reduce_kernel(int order, int H, int HT, int64_t M, int C,
-                                    const Real* __restrict__ S, const Real* __restrict__ T,
-                                    double reg, const double* __restrict__ scalar, int nkeep,
-                                    double* __restrict__ mkeep, const double* __restrict__ Q,
-                                    double* __restrict__ dots) {
-  __shared__ double sh[32];
+// Solve fused with the dual-form reductions.  blockIdx.y = bandwidth h < HT,
+// blockIdx.z = CMAX of the C channels.  Writes m for the first nkeep channels
+// to mkeep (HT, M, nkeep) and adds dots[c][h] += sum_g m_c(g) Q[g][c] for
+// every channel.  Bound by the latency of a point's planes: the last block's
+// channels beyond C repeat the last one and are dropped, so that no branch
+// stands between the loads, and four channels' loads are in flight.  More
+// than 12 channels a block make the accumulators spill; repeating the solve
+// for the next 12 reads ns planes beside the 12 nt of the channels.  (A test
+// per channel: 540 us for 7 bandwidths of 64^3, 11 channels, 4 terms; 157 now.)
+template <typename Real, int NT, int CMAX>
+__global__ void __launch_bounds__(256)
+solve_reduce_kernel(int order, int H, int HT, int64_t M, int C, const Real* __restrict__ S,
+                    const Real* __restrict__ T, double reg, const double* __restrict__ scalar,
+                    int nkeep, double* __restrict__ mkeep, const double* __restrict__ Q,
+                    double* __restrict__ dots) {
+  __shared__ double sh[8][CMAX];
+  const int cz = blockIdx.z * CMAX;
   const int h = blockIdx.y;
   const int64_t HM = (int64_t)H * M;
   const int64_t HTM = (int64_t)HT * M;
-  double acc[kMaxDotChan];
+  double acc[CMAX];
 #pragma unroll
-  for (int c = 0; c < kMaxDotChan; ++c) acc[c] = 0.0;
+  for (int c = 0; c < CMAX; ++c) acc[c] = 0.0;
   for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < M;
        g += (int64_t)gridDim.x * blockDim.x) {
     const int64_t t = (int64_t)h * M + g;
     double z[NT];
     const bool ok = zvec_at<Real, NT>(order, HM, t, S, scalar[0], reg, z);
     const double* q = Q + g * C;
+    constexpr int CB = 4;  // channels in flight
 #pragma unroll
-    for (int c = 0; c < kMaxDotChan; ++c) {
-      if (c < C) {
+    for (int c0 = 0; c0 < CMAX; c0 += CB) {
+      Real tv[CB][NT];
+      double qv[CB];
+#pragma unroll
+      for (int k = 0; k < CB; ++k) {
+        const int c = min(cz + c0 + k, C - 1);
+#pragma unroll
+        for (int i = 0; i < NT; ++i) tv[k][i] = T[((int64_t)i * C + c) * HTM + t];
+        qv[k] = q[c];
+      }
+#pragma unroll
+      for (int k = 0; k < CB; ++k) {
         double v = 0.0;
 #pragma unroll
-        for (int i = 0; i < NT; ++i) v += z[i] * (double)T[((int64_t)i * C + c) * HTM + t];
+        for (int i = 0; i < NT; ++i) v += z[i] * (double)tv[k][i];
         if (!ok) v = NAN;
-        if (c < nkeep) mkeep[t * nkeep + c] = v;
-        acc[c] += v * q[c];
+        if (cz + c0 + k < nkeep) mkeep[t * nkeep + cz + c0 + k] = v;
+        acc[c0 + k] += v * qv[k];
       }
     }
   }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
-  for (int c = 0; c < kMaxDotChan; ++c) {
-    if (c < C) {
-      double v = acc[c];
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      __syncthreads();
-      if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double sum = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) sum += sh[w];
-        atomicAdd(&dots[(int64_t)c * HT + h], sum);
-      }
-    }
+  for (int c = 0; c < CMAX; ++c) {
+    double v = acc[c];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) sh[warp][c] = v;
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < CMAX && cz + c < C; c += blockDim.x) {
+    double sum = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) sum += sh[w][c];
+    atomicAdd(&dots[(int64_t)(cz + c) * HT + h], sum);
   }
 }
 
@@ -167,15 +183,22 @@ static int launch_solve_reduce(int order, int H, int HT, int64_t M, int C, const
                                const void* d_T, double reg, const double* scalar, int nkeep,
                                double* mkeep, const double* Q, double* dots, int prec, dim3 grid,
                                cudaStream_t s) {
-  if (prec == FLPR_PREC_F32) {
-    solve_reduce_kernel<float, NT><<<grid, 256, 0, s>>>(order, H, HT, M, C, (const float*)d_S,
-                                                        (const float*)d_T, reg, scalar, nkeep,
-                                                        mkeep, Q, dots);
+#define FLPR_SR(CM)                                                                          \
+  if (prec == FLPR_PREC_F32)                                                                 \
+    solve_reduce_kernel<float, NT, CM><<<grid, 256, 0, s>>>(                                 \
+        order, H, HT, M, C, (const float*)d_S, (const float*)d_T, reg, scalar, nkeep, mkeep, \
+        Q, dots);                                                                            \
+  else                                                                                       \
+    solve_reduce_kernel<double, NT, CM><<<grid, 256, 0, s>>>(                                \
+        order, H, HT, M, C, (const double*)d_S, (const double*)d_T, reg, scalar, nkeep,      \
+        mkeep, Q, dots);
+  if (C <= 4) {
+    FLPR_SR(4)
   } else {
-    solve_reduce_kernel<double, NT><<<grid, 256, 0, s>>>(order, H, HT, M, C, (const double*)d_S,
-                                                         (const double*)d_T, reg, scalar, nkeep,
-                                                         mkeep, Q, dots);
+    grid.z = (C + 11) / 12;
+    FLPR_SR(12)
   }
+#undef FLPR_SR
   FLPR_LAUNCH_CHECK();
   return FLPR_OK;
 }

@@ -203,3 +203,29 @@ def test_density_scores_at_the_edges(cuda_ok, d, n, G, H):
     k, o = fastlpr_b200.cv_fastkde(x, h, dict(opts)), oracle.cv_fastkde(x, h, {"N": opts["N"]})
     assert rel_err(k.metadata["fhat_all"], o["fhat_all"]) < 1e-9
     assert rel_err(k.lcv["lcv_m"], o["lcv_m"]) < 1e-9 and rel_err(k.lcv["lcv_sd"], o["lcv_sd"]) < 1e-9
+
+
+@pytest.mark.parametrize("C", [1, 4, 5, 12, 13, 24, 25, 32])
+@pytest.mark.parametrize("order,nt,f32", [(0, 1, True), (1, 3, True), (1, 4, False), (2, 6, True)])
+def test_solve_reduce_channels(cuda_ok, C, order, nt, f32):
+    """Every padded channel count, against the unfused solve and its sums."""
+    import torch
+    from fastlpr_b200 import _lib, api
+    rng = np.random.default_rng(C * 10 + nt)
+    ctx = api._Ctx(torch.device("cuda", 0))
+    H, M, keep, prec = 3, 1237, min(C, 2), 0 if f32 else 1
+    real = torch.float32 if f32 else torch.float64
+    A = rng.standard_normal((H, M, nt, nt + 2))
+    A = A @ A.transpose(0, 1, 3, 2)
+    S = np.stack([A[:, :, i, j] for i in range(nt) for j in range(i, nt)])
+    S, T = ctx.upload(S).to(real), ctx.upload(rng.standard_normal((nt, C, H, M))).to(real)
+    Q = ctx.upload(rng.standard_normal((M, C)))
+    m, kept, dots, sc = (ctx.empty(s) for s in ((H, M, C), (H, M, keep), (C, H), (1,)))
+    a = (order, nt, H, H, M, C, S.data_ptr(), T.data_ptr(), 1e-6)
+    _lib.check(ctx.lib.flpr_solve(*a, m.data_ptr(), sc.data_ptr(), prec, ctx.stream), "solve")
+    _lib.check(ctx.lib.flpr_solve_reduce(*a, keep, kept.data_ptr(), Q.data_ptr(), dots.data_ptr(),
+                                         sc.data_ptr(), prec, ctx.stream), "solve_reduce")
+    m, kept, q = m.cpu().numpy(), kept.cpu().numpy(), Q.cpu().numpy()
+    np.testing.assert_allclose(kept, m[:, :, :keep], rtol=1e-9, atol=1e-9)
+    scale = np.einsum("hmc,mc->ch", np.abs(m), np.abs(q))
+    assert np.all(np.abs(dots.cpu().numpy() - np.einsum("hmc,mc->ch", m, q)) <= 1e-11 * scale)
