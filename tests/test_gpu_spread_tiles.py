@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 import oracle.lpr as oracle
-from conftest import rel_err
+from conftest import elem_rel_err, rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -229,3 +229,24 @@ def test_solve_reduce_channels(cuda_ok, C, order, nt, f32):
     np.testing.assert_allclose(kept, m[:, :, :keep], rtol=1e-9, atol=1e-9)
     scale = np.einsum("hmc,mc->ch", np.abs(m), np.abs(q))
     assert np.all(np.abs(dots.cpu().numpy() - np.einsum("hmc,mc->ch", m, q)) <= 1e-11 * scale)
+
+
+@pytest.mark.parametrize("prec,tol", [("fp32", 1e-5), ("fp64", 1e-11)])
+@pytest.mark.parametrize("order,dof", [(0, False), (0, True), (1, False)])
+@pytest.mark.parametrize("G", [[20, 24], [48, 40], [90, 120], [200, 250], [300, 400]])
+def test_row_products_up_to_the_nyquist_term(cuda_ok, G, order, dof, prec, tol):
+    """Kernels narrower than a grid step fill the whole band: every element of a
+    row, the real DC and Nyquist ones too, single products and pairs, for each
+    transform length."""
+    import fastlpr_b200
+    rng = np.random.default_rng(G[0] + order)
+    n = 40 * G[0] * G[1]
+    x = rng.random((n, 2))
+    y = np.sin(2 * np.pi * x[:, 0]) * np.cos(2 * np.pi * x[:, 1]) + 0.1 * rng.standard_normal(n)
+    step = np.sqrt(12.0) / np.array(G)
+    h = np.outer([0.8, 1.5, 4.0], step)
+    opts = {"order": order, "N": G, "precision": prec, "calc_dof": dof}
+    a = fastlpr_b200.cv_fastlpr(x, y, h, opts)
+    b = fastlpr_b200.cv_fastlpr(x, y, h, dict(opts, _no_fused=True))
+    assert rel_err(a.yhat, b.yhat) < tol and rel_err(a.s0, b.s0) < tol
+    assert elem_rel_err(a.gcv_yhat["gcv_m"], b.gcv_yhat["gcv_m"]) < tol
