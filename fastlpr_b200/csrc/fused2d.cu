@@ -612,7 +612,7 @@ rowpass_s_kernel(RowArgs ra, int H, int nslots_w, const typename Vec2<T>::V* __r
 #pragma unroll
   for (int s = 0; s < E; ++s) {
     const int x = out_index<E>(lane, s) - ra.q1;
-    if (x >= 0 && x < ra.G1) {
+    if ((unsigned)x < (unsigned)ra.G1) {
       da[x] = v[s].x;
       if (pair) db[x] = v[s].y;
     }
@@ -643,7 +643,10 @@ inline int t_warps(int njobs) { return njobs < kTWarps ? njobs : kTWarps; }
 // solve vectors, the response fits go to `my`, and sum_x1 m_c Q_c
 // accumulates into one partial per (c, h, row).  A channel's NT products
 // span at most two consecutive rounds (NT <= 2 nwarps + 1), so the buffers
-// of the previous round still hold its earlier products.
+// of the previous round still hold its earlier products.  A point's solve
+// vector and deposits are loaded once for all channels of a round, whose
+// sums then have their loads in flight together (channel by channel the pass
+// took 1.213 ms for 32 bandwidths on 512^2, 11 channels and 3 terms, now 1.034).
 template <int E, int NT, typename T>
 __device__ __forceinline__ void rowpass_t_solve_body(
     RowArgs ra, int H, int nslots_w, const typename Vec2<T>::V* __restrict__ W,
@@ -687,6 +690,7 @@ __device__ __forceinline__ void rowpass_t_solve_body(
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kc = kcut1[h];
   const int nprod = C * NT;
+  constexpr int CR = (2 * kTWarps + NT - 1) / NT;  // channels that one round can complete
   for (int r0 = 0; r0 < njobs; r0 += nwarps) {
     const int j = r0 + warp;
     T* buf = bufs + ((size_t)(((r0 / nwarps) & 1) * nwarps) + warp) * SW;
@@ -698,7 +702,7 @@ __device__ __forceinline__ void rowpass_t_solve_body(
 #pragma unroll
       for (int s = 0; s < E; ++s) {
         const int x = out_index<E>(lane, s) - ra.q1;
-        if (x >= 0 && x < G1) {
+        if ((unsigned)x < (unsigned)G1) {
           buf[x] = v[s].x;
           if (pair) buf[G1 + x] = v[s].y;
         }
@@ -708,25 +712,42 @@ __device__ __forceinline__ void rowpass_t_solve_body(
     // channels whose NT products all came out of this round
     const int p_end = min(nprod, 2 * (r0 + nwarps));
     const int c_begin = (2 * r0) / NT, c_end = p_end / NT;
-    for (int c = c_begin; c < c_end; ++c) {
-      const T* src[NT];
+    const int par = (r0 / nwarps) & 1;
+    const T* src[CR][NT];
+#pragma unroll
+    for (int k = 0; k < CR; ++k) {
 #pragma unroll
       for (int i = 0; i < NT; ++i) {
-        const int p = c * NT + i, jj = p >> 1, kk = jj / nwarps;
-        src[i] = bufs + ((size_t)((kk & 1) * nwarps) + (jj - kk * nwarps)) * SW + (p & 1) * G1;
+        const int p = min((c_begin + k) * NT + i, p_end - 1), jj = p >> 1;
+        const int w = jj >= r0 ? par * nwarps + jj - r0 : (par ^ 1) * nwarps + jj - r0 + nwarps;
+        src[k][i] = bufs + (size_t)w * SW + (p & 1) * G1;
       }
-      double acc = 0.0;
-      for (int x = threadIdx.x; x < G1; x += blockDim.x) {
-        const int64_t g = (int64_t)r * G1 + x;
-        const double* z = zg + ((int64_t)h * M + g) * NT;
+    }
+    double acc[CR];
+#pragma unroll
+    for (int k = 0; k < CR; ++k) acc[k] = 0.0;
+    for (int x = threadIdx.x; x < G1; x += blockDim.x) {
+      const int64_t g = (int64_t)r * G1 + x;
+      const double* zp = zg + ((int64_t)h * M + g) * NT;
+      double z[NT], q[CR];
+#pragma unroll
+      for (int i = 0; i < NT; ++i) z[i] = zp[i];
+#pragma unroll
+      for (int k = 0; k < CR; ++k) q[k] = c_begin + k < c_end ? Q[g * C + c_begin + k] : 0.0;
+#pragma unroll
+      for (int k = 0; k < CR; ++k) {
         double m = 0.0;
 #pragma unroll
-        for (int i = 0; i < NT; ++i) m += z[i] * (double)src[i][x];
-        if (c < ny) my[((int64_t)h * M + g) * ny + c] = m;
-        acc += m * Q[g * C + c];
+        for (int i = 0; i < NT; ++i) m += z[i] * (double)src[k][i][x];
+        if (c_begin + k < min(ny, c_end)) my[((int64_t)h * M + g) * ny + c_begin + k] = m;
+        if (c_begin + k < c_end) acc[k] += m * q[k];
       }
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane == 0) red[c * nwarps + warp] = acc;  // C * nwarps <= 32 * kTWarps
+    }
+#pragma unroll
+    for (int k = 0; k < CR; ++k) {
+      for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+      if (lane == 0 && c_begin + k < c_end)
+        red[(c_begin + k) * nwarps + warp] = acc[k];  // C * nwarps <= 32 * kTWarps
     }
     __syncthreads();  // the next round overwrites the buffers
   }
@@ -738,9 +759,10 @@ __device__ __forceinline__ void rowpass_t_solve_body(
   }
 }
 
-// FP32: four CTAs of four warps per SM at the 112-register cap.
+// FP32: four CTAs of four warps per SM at the 112-register cap (five or six at
+// the caps of the shorter transforms; 80 registers spill below 8 slots).
 template <int E, int NT>
-__global__ void __maxnreg__(E <= 16 ? 80 : 112)
+__global__ void __maxnreg__(E <= 4 ? 96 : E <= 16 ? 80 : 112)
 rowpass_t_solve_kernel(RowArgs ra, int H, int nslots_w, const float2* __restrict__ W,
                        const float2* __restrict__ F1f, const float2* __restrict__ tab,
                        const int* __restrict__ kcut1, int C, int ny, const double* __restrict__ zg,
