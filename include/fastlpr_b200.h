@@ -47,8 +47,8 @@ int64_t flpr_launch_count(void);
 /* Tuning parameters, process-wide (they hold for every later call on every
  * device; calls already enqueued keep the values they were launched with).
  * Set by the autotuner of the Python host (fastlpr_b200/autotune.py).
- *   FLPR_TUNE_SPREAD_ITEM_POINTS: points per spread work item (one CTA),
- *     256..65536, default 4096;
+ *   FLPR_TUNE_SPREAD_ITEM_POINTS: most points per spread work item,
+ *     256..65536, default 4096 (2-D and 3-D items: at most 1024);
  *   FLPR_TUNE_FUSED_CHUNK_MB: column-pass output budget of the fused 2-D
  *     convolution (bandwidths per chunk), 8..16384 MB, default 768. */
 #define FLPR_TUNE_SPREAD_ITEM_POINTS 0
@@ -117,9 +117,10 @@ int flpr_point_stats_noalloc(int d, int64_t n, const double* d_x, double* d_stat
  *   nchan-ones_channel channels are h_cols[i] (device float64 arrays of n).
  * d_grid_out: (nchan, L...) real, float (FLPR_PREC_F32) or double, scaled
  *   by 1/n (the 1/M of nufftn_type1.py:709-711).
- * Accumulation is per-tile in shared memory after binning the points by
- * tile; FLPR_PREC_F32 accumulates in 64-bit fixed point (order independent,
- * deterministic), FLPR_PREC_F64 in float64.
+ * Accumulation is per tile after binning the points by tile (2-D and 3-D
+ * FLPR_PREC_F32: in registers; otherwise in shared memory); FLPR_PREC_F32
+ * accumulates in 64-bit fixed point (order independent, deterministic),
+ * FLPR_PREC_F64 in float64.
  * --------------------------------------------------------------------- */
 size_t flpr_spread_ws(int d, int64_t n, const int* h_L, int msp, int nchan, int prec);
 int flpr_spread(int d, int64_t n, const double* d_x, const double* h_kmap,
