@@ -551,7 +551,8 @@ tile_accumulate_kernel(SpreadGeom g, int nchan, int cgroup,
 // about 2.2 cycles each) and by latency: the multiply-add takes 23 cycles,
 // so the next point's values are read and scaled beside this point's sums,
 // and UC stays at 3 or less, which leaves registers for 12 to 16 warps.
-// Measured: 1e6 points, 12 channels, grid 512^2: 527 -> 220 us (UC = 4 in one
+// Measured: 1e6 points, 12 channels, grid 512^2: 527 -> 220 us
+// (264 with the exponentials of tap_weights_exp; UC = 4 in one
 // warp: 266 us; the multiply-adds alone: 90 us); 1e7 points, one channel,
 // grid 128^3: 7.63 -> 1.90 ms.
 constexpr int kT2 = 8;            // tile edge of the 2-D path
