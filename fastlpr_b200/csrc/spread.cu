@@ -537,8 +537,8 @@ tile_accumulate_kernel(SpreadGeom g, int nchan, int cgroup,
 // row leaves the registers once, when the walk has passed it.  It goes
 // through a small shared buffer to one global atomic per non-zero cell: no
 // atomics on shared memory, no accumulator tile.  In the fixed-point
-// accumulator every product is rounded to an integer as it is added, so sums
-// are exact and the grid does not depend on the order of the points.
+// accumulator every product is rounded to an integer before it is added, so
+// sums are exact and the grid does not depend on the order of the points.
 //
 // In 3-D a tile is one cell thick on the first axis, and the NT1 taps of that
 // axis take the place of the channels: tap plane j of a point has the value
@@ -547,47 +547,46 @@ tile_accumulate_kernel(SpreadGeom g, int nchan, int cgroup,
 // halo column of an 8 x 8 x 8 tile, rounding every product by two additions,
 // took 37 operations and left more than half of its lanes idle.
 //
-// Bound by the FP64 pipe (UC (NT1 + 1) multiply-adds per point and warp,
-// about 2.2 cycles each) and by latency: the multiply-add takes 23 cycles,
-// so the next point's values are read and scaled beside this point's sums,
-// and UC stays at 3 or less, which leaves registers for 12 to 16 warps.
-// Measured: 1e6 points, 12 channels, grid 512^2: 527 -> 220 us
-// (264 with the exponentials of tap_weights_exp; UC = 4 in one
-// warp: 266 us; the multiply-adds alone: 90 us); 1e7 points, one channel,
-// grid 128^3: 7.63 -> 1.90 ms.
+// Bound by the FP64 pipe (UC (NT1 + 1) multiply-adds per point and warp, about
+// 2.2 cycles each), beside which the FP32 grids issue two integer adds per
+// product, and by latency: the next point's values are read and scaled beside
+// this point's sums, and UC stays at 3 or less, which leaves registers for 12
+// to 16 warps.  FP32 grids: 1e6 points, 12 channels, grid 512^2: 338 us, where
+// an atomic per tile row on a shared tile took 527; 1e7 points, one channel,
+// grid 128^3: 2.40 ms, where a thread per halo column took 7.63.
 constexpr int kT2 = 8;            // tile edge of the 2-D path
 constexpr int kItem2 = 1024;      // most points of a work item
 
-// Register accumulators of the tile kernels, one fused multiply-add per
-// product.  Fixed point with quantum q (a power of two): the register starts
-// at 1.5 * 2^52 q and stays in [2^52 q, 2^53 q), where every double is a
-// multiple of q (the sums stay below 2^50 q), so a = v w + a adds the product
-// rounded to the nearest multiple and the sum is exact.  A product halfway
-// between two multiples would round by the parity of the sum so far, that is
-// by the order of the points; factor() therefore sets the last mantissa bit
-// of v: with |v w| < 2^50 q and w <= 1 the product then has a non-zero bit
-// below q / 2 and no tie can occur.  (One FP64 instruction instead of a fused
-// multiply-add and a 64-bit integer add, or of a product and two roundings.)
-// Float64 accumulation adds the fused product.
+// Register accumulators of the tile kernels.  Fixed point with quantum q (a
+// power of two): the product v w is rounded once, to the nearest multiple of
+// q, by the fused multiply-add t = v w + 1.5 * 2^52 q (every double in
+// [2^52 q, 2^53 q) is a multiple of q, and |v w| < 2^50 q keeps t there).  The
+// bit pattern of t is that of the bias plus v w / q, so the register adds the
+// bit patterns as integers: no carry is lost in the low 51 bits, where the
+// bias has none, and the sum (below 2^50 in magnitude) is their value as a
+// signed number.  The sum is exact and independent of the order of the points,
+// and v enters with all its bits.  (Adding in the multiply-add itself, with the
+// sum in place of the bias, rounds a product halfway between two multiples by
+// the parity of the sum so far; keeping such products away by setting v's last
+// bit costs that bit, and rounds every one of them up.)  Float64 accumulation
+// adds the fused product.
 template <typename Acc>
 struct RegSum;
 template <>
 struct RegSum<long long> {
-  static constexpr double kBias = 6755399441055744.0;  // 1.5 * 2^52
-  __device__ static double zero(double q) { return kBias * q; }
-  __device__ static double factor(double v) {
-    return __longlong_as_double(__double_as_longlong(v) | 1ll);
+  using T = unsigned long long;
+  __device__ static double bias(double q) { return 6755399441055744.0 * q; }  // 1.5 * 2^52 q
+  __device__ static void add(T& a, double v, double w, double bias) {
+    a += (T)__double_as_longlong(__fma_rn(v, w, bias));
   }
-  // the sum in units of q, scale = 1 / q
-  __device__ static long long value(double a, double scale) {
-    return __double_as_longlong(a * scale) - __double_as_longlong(kBias);
-  }
+  __device__ static long long value(T a) { return (long long)(a << 13) >> 13; }
 };
 template <>
 struct RegSum<double> {
-  __device__ static double zero(double) { return 0.0; }
-  __device__ static double factor(double v) { return v; }
-  __device__ static double value(double a, double) { return a; }
+  using T = double;
+  __device__ static double bias(double) { return 0.0; }
+  __device__ static void add(T& a, double v, double w, double) { a = __fma_rn(v, w, a); }
+  __device__ static double value(T a) { return a; }
 };
 
 // Tap weights of one axis from the knot's offset f to its cell:
@@ -672,7 +671,7 @@ __host__ __device__ constexpr int warps2(int nt1, int uc) {
 // Shared memory of one CTA.  The rows that the lanes still hold at the end
 // go through the space of the staged points.  A warp's NCW "channels" are its
 // value channels in 2-D and the tap planes of its one channel in 3-D.
-template <int D, int NT1, int UC, int NW>
+template <typename Acc, int D, int NT1, int UC, int NW>
 struct Stage2 {
   static constexpr int W = kT2 + NT1 - 1;     // halo cells per axis
   static constexpr int GPL = groups2(NT1);    // channel groups of a warp
@@ -688,15 +687,15 @@ struct Stage2 {
     double wx[32 * WXS];     // weights of the last axis
     double wy[33 * NT1];     // weights of the axis before it
     double val[D == 3 ? 33 * VS : 1];  // 3-D: axis-0 weights times the channels' values
-    double row[NCB * WR];
+    Acc row[NCB * WR];
     unsigned short order[kItem2];
     unsigned char cell[kItem2];
   };
   union {
     Points st;
-    double rows[NT1 * NCB * WR];
+    Acc rows[NT1 * NCB * WR];
   };
-  double scale[NVB], zero[NVB];
+  double bias[NVB];
   double cj[D][(NT1 - 1) / 2 + 1];
   int off[kT2 * kT2 + 1];
   int cur[kT2 * kT2];
@@ -704,11 +703,11 @@ struct Stage2 {
   int64_t plane[D == 3 ? NT1 : 1];  // 3-D: start of the grid planes of the tap planes
 };
 
-// Adds `nrows` halo rows from grid row gr0 on, (rows, NCW, WR) registers of
+// Adds `nrows` halo rows from grid row gr0 on, (rows, NCW, WR) sums of
 // one warp's lanes for its first nc channels, to the global accumulator: one
 // atomic per non-zero cell.  v_w: its first value channel in the CTA.
 template <typename Acc, int D, typename S>
-__device__ __forceinline__ void add_rows(const SpreadGeom& g, const S& sh, const double* buf,
+__device__ __forceinline__ void add_rows(const SpreadGeom& g, const S& sh, const Acc* buf,
                                          int nrows, int gr0, int c_begin, int v_w, int nc,
                                          int lane, Acc* __restrict__ gacc) {
   constexpr int W = S::W, N = S::NCW * W, U = (N + 31) / 32;
@@ -717,12 +716,12 @@ __device__ __forceinline__ void add_rows(const SpreadGeom& g, const S& sh, const
     int gr = (gr0 + r) % Lr;
     if (gr < 0) gr += Lr;
     Acc* grow = gacc + (int64_t)(c_begin + v_w) * g.cells + (int64_t)gr * Lc;
-    const double* rb = buf + r * S::NCW * S::WR;
+    const Acc* rb = buf + r * S::NCW * S::WR;
     Acc v[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int idx = u * 32 + lane, c = idx / W, j = idx - c * W;
-      v[u] = c < nc ? RegSum<Acc>::value(rb[c * S::WR + j], sh.scale[D == 2 ? v_w + c : v_w]) : Acc(0);
+      v[u] = c < nc ? rb[c * S::WR + j] : Acc(0);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -748,7 +747,8 @@ tile_accumulate_reg_kernel(SpreadGeom g, int nchan, const int* __restrict__ offs
                            const double* __restrict__ rec, int stride,
                            const double* __restrict__ absum, int margin_bits,
                            Acc* __restrict__ gacc) {
-  using S = Stage2<D, NT1, UC, NW>;
+  using S = Stage2<Acc, D, NT1, UC, NW>;
+  using R = RegSum<Acc>;
   constexpr int MSP = (NT1 - 1) / 2;
   constexpr int NLC = kT2 * kT2;
   constexpr int NT = 32 * NW;
@@ -769,8 +769,7 @@ tile_accumulate_reg_kernel(SpreadGeom g, int nchan, const int* __restrict__ offs
   const double ify = 1.0 / g.four_tau[D - 2], ifx = 1.0 / g.four_tau[D - 1];
   for (int c = tid; c < NVB; c += NT) {
     const double sc = (c < nv && absum != nullptr) ? fixed_scale(absum[c_begin + c], margin_bits) : 1.0;
-    sh.scale[c] = sc;
-    sh.zero[c] = RegSum<Acc>::zero(1.0 / sc);
+    sh.bias[c] = R::bias(1.0 / sc);
   }
   for (int k = tid; k < D * (MSP + 1); k += NT) {
     const int ax = k / (MSP + 1), j = k - ax * (MSP + 1);
@@ -853,12 +852,14 @@ tile_accumulate_reg_kernel(SpreadGeom g, int nchan, const int* __restrict__ offs
 
     // idle lanes repeat group 0 and drop it
     const int c_w = warp * NCW, vofs = c_w + (active ? grp * UC : 0);
-    auto zero_of = [&](int k) { return sh.zero[D == 2 ? vofs + k : v_w]; };
-    double a[UC][W];
+    double bias[UC];
+#pragma unroll
+    for (int k = 0; k < UC; ++k) bias[k] = sh.bias[D == 2 ? vofs + k : v_w];
+    typename R::T a[UC][W];
 #pragma unroll
     for (int k = 0; k < UC; ++k)
 #pragma unroll
-      for (int j = 0; j < W; ++j) a[k][j] = zero_of(k);
+      for (int j = 0; j < W; ++j) a[k][j] = 0;
     int row = 0, half = 0;
     for (int b0 = 0; b0 < np; b0 += 32, half ^= 1) {
       const int b1 = min(b0 + 32, np);
@@ -895,7 +896,7 @@ tile_accumulate_reg_kernel(SpreadGeom g, int nchan, const int* __restrict__ offs
         const double2* xp = reinterpret_cast<const double2*>(sh.st.wx + pp * WXS);
         double v[UC];  // the next point's values times its axis-0 weight
 #pragma unroll
-        for (int k = 0; k < UC; ++k) v[k] = RegSum<Acc>::factor(*yp * vp[k]);
+        for (int k = 0; k < UC; ++k) v[k] = *yp * vp[k];
 #pragma unroll
         for (int cr = 0; cr < kT2; ++cr) {
           const int pe = min(ro[cr + 1], b1) - b0;
@@ -917,26 +918,24 @@ tile_accumulate_reg_kernel(SpreadGeom g, int nchan, const int* __restrict__ offs
 #pragma unroll
             for (int jx = 0; jx < NT1; ++jx)
 #pragma unroll
-              for (int k = 0; k < UC; ++k) a[k][cr + jx] = __fma_rn(v[k], w[jx], a[k][cr + jx]);
+              for (int k = 0; k < UC; ++k) R::add(a[k][cr + jx], v[k], w[jx], bias[k]);
 #pragma unroll
-            for (int k = 0; k < UC; ++k) v[k] = RegSum<Acc>::factor(wyn * u[k]);
+            for (int k = 0; k < UC; ++k) v[k] = wyn * u[k];
           }
         }
         if (ro[kT2] > b1) break;      // the row goes on in the next batch
         if (row >= W - NT1) break;    // every lane on its last row
         // halo row `row` is complete: its lanes hand it over and start row + NT1
-        double* rb = sh.st.row + c_w * WR;
+        Acc* rb = sh.st.row + c_w * WR;
         if (active && jm == row % NT1) {
-          double* rp = rb + grp * UC * WR;
+          Acc* rp = rb + grp * UC * WR;
 #pragma unroll
-          for (int k = 0; k < UC; ++k) {
-            const double z = zero_of(k);
+          for (int k = 0; k < UC; ++k)
 #pragma unroll
             for (int j = 0; j < W; ++j) {
-              rp[k * WR + j] = a[k][j];
-              a[k][j] = z;
+              rp[k * WR + j] = R::value(a[k][j]);
+              a[k][j] = 0;
             }
-          }
         }
         __syncwarp();
         add_rows<Acc, D, S>(g, sh, rb, 1, tcy * kT2 + row - MSP, c_begin, v_w, nc_w, lane, gacc);
@@ -946,15 +945,15 @@ tile_accumulate_reg_kernel(SpreadGeom g, int nchan, const int* __restrict__ offs
     }
     // the last NT1 rows, each in its own lanes
     sync2<NW>();
-    double* rb = sh.rows + (size_t)warp * NT1 * NCW * WR;
+    Acc* rb = sh.rows + (size_t)warp * NT1 * NCW * WR;
     if (active) {
       int r = (jm - (W - NT1)) % NT1;  // position of this lane's row among W - NT1 .. W - 1
       if (r < 0) r += NT1;
-      double* rp = rb + (r * NCW + grp * UC) * WR;
+      Acc* rp = rb + (r * NCW + grp * UC) * WR;
 #pragma unroll
       for (int k = 0; k < UC; ++k)
 #pragma unroll
-        for (int j = 0; j < W; ++j) rp[k * WR + j] = a[k][j];
+        for (int j = 0; j < W; ++j) rp[k * WR + j] = R::value(a[k][j]);
     }
     __syncwarp();
     add_rows<Acc, D, S>(g, sh, rb, NT1, tcy * kT2 + (W - NT1) - MSP, c_begin, v_w, nc_w, lane, gacc);
@@ -1153,7 +1152,7 @@ static int launch_reg_k(const SpreadGeom& g, int nchan, const SpreadWs& w, const
   auto k = tile_accumulate_reg_kernel<Acc, D, NT1, UC, NW>;
   FLPR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared));
-  constexpr int NVB = Stage2<D, NT1, UC, NW>::NVB;
+  constexpr int NVB = Stage2<Acc, D, NT1, UC, NW>::NVB;
   // a CTA per item in 2-D (dealing them out in turn cost 5% there); in 3-D
   // the slabs of the padded grid are 8 times the occupied ones and more: four
   // rounds of the resident CTAs, each taking items in turn
