@@ -18,8 +18,6 @@
 // FLPR_PREC_F32 accumulates 64-bit fixed point: integer addition is
 // associative, so the result does not depend on the order of the atomics
 // and the grid is deterministic.  FLPR_PREC_F64 accumulates float64.
-#include <type_traits>
-
 #include "common.cuh"
 
 namespace flpr {
@@ -551,9 +549,10 @@ tile_accumulate_kernel(SpreadGeom g, int nchan, int cgroup,
 // 2.2 cycles each), beside which the FP32 grids issue two integer adds per
 // product, and by latency: the next point's values are read and scaled beside
 // this point's sums, and UC stays at 3 or less, which leaves registers for 12
-// to 16 warps.  FP32 grids: 1e6 points, 12 channels, grid 512^2: 338 us, where
-// an atomic per tile row on a shared tile took 527; 1e7 points, one channel,
-// grid 128^3: 2.40 ms, where a thread per halo column took 7.63.
+// to 16 warps.  1e6 points, 12 channels, FP32 grid 512^2: 340 us, where an
+// atomic per tile row on a shared tile took 527; 2e6 points, 12 channels, FP64:
+// 421 us (758); 1e7 points, one channel, FP32 grid 128^3: 2.80 ms, where a
+// thread per halo column took 7.63.
 constexpr int kT2 = 8;            // tile edge of the 2-D path
 constexpr int kItem2 = 1024;      // most points of a work item
 
@@ -590,44 +589,20 @@ struct RegSum<double> {
 };
 
 // Tap weights of one axis from the knot's offset f to its cell:
-// exp(-(f - hx j)^2 / ft) = exp(-f^2 / ft) r^j C_|j|, r = exp(2 f hx / ft),
-// C_j = exp(-(hx j)^2 / ft), times val for j = -MSP .. MSP into w (two exponentials
-// and one reciprocal per axis instead of an exponential and a division per tap).
+// val exp(-(f - hx j)^2 / ft), j = -MSP .. MSP, into w: an exponential per tap.
+// (The products e0 r^j C_j, two exponentials and a reciprocal per axis, save
+// 10% of a 2-D FP64 spread and 15% of a 3-D one and err 1.6 times as much in
+// the root mean square of a 2-D stencil.)
 template <int NT1>
-__device__ __forceinline__ void tap_weights(double f, double val, double hx, double inv_ft,
-                                            const double* __restrict__ cj, double* __restrict__ w) {
-  constexpr int MSP = (NT1 - 1) / 2;
-  const double e0 = val * exp(-(f * f) * inv_ft);
-  w[MSP] = e0;
-  if constexpr (MSP > 0) {
-    const double b = 2.0 * f * hx * inv_ft;
-    const double rp = exp(b), rm = 1.0 / rp;
-    double p = e0, m = e0;
-#pragma unroll
-    for (int j = 1; j <= MSP; ++j) {
-      p *= rp;
-      m *= rm;
-      const double c = cj[j];
-      w[MSP + j] = p * c;
-      w[MSP - j] = m * c;
-    }
-  }
-}
-
-// The same with an exponential per tap, for the FP32 grids in 2-D: the last
-// bits of the products above move the FP32 rounding of about one cell in 1e8,
-// and the fits see a cell's last bit.  (1e6 points, 12 channels, 512^2: 231 us
-// with the products, 264 with the exponentials.)
-template <int NT1>
-__device__ __forceinline__ void tap_weights_exp(double f, double hx, double ft, double inv_ft,
-                                                double* __restrict__ w) {
+__device__ __forceinline__ void tap_weights(double f, double val, double hx, double ft,
+                                            double inv_ft, double* __restrict__ w) {
 #pragma unroll 3
   for (int j = 0; j < NT1; ++j) {
     const double t = f - hx * (double)(j - (NT1 - 1) / 2);
     // the quotient (t^2) / ft, corrected by its residual (Markstein); a single
     // tap has ft infinite and weight 1
     const double p = t * t, q = p * inv_ft;
-    w[j] = exp(-(NT1 == 1 ? q : __fma_rn(__fma_rn(-q, ft, p), inv_ft, q)));
+    w[j] = val * exp(-(NT1 == 1 ? q : __fma_rn(__fma_rn(-q, ft, p), inv_ft, q)));
   }
 }
 
@@ -696,7 +671,6 @@ struct Stage2 {
     Acc rows[NT1 * NCB * WR];
   };
   double bias[NVB];
-  double cj[D][(NT1 - 1) / 2 + 1];
   int off[kT2 * kT2 + 1];
   int cur[kT2 * kT2];
   int col[W];  // grid columns of the halo
@@ -767,14 +741,10 @@ tile_accumulate_reg_kernel(SpreadGeom g, int nchan, const int* __restrict__ offs
   const bool active = grp < GPL && grp * UC < nc_w;
   const double hy = g.ax[D - 2].hx, hx = g.ax[D - 1].hx;
   const double ify = 1.0 / g.four_tau[D - 2], ifx = 1.0 / g.four_tau[D - 1];
+  const double ifz = 1.0 / g.four_tau[0];
   for (int c = tid; c < NVB; c += NT) {
     const double sc = (c < nv && absum != nullptr) ? fixed_scale(absum[c_begin + c], margin_bits) : 1.0;
     sh.bias[c] = R::bias(1.0 / sc);
-  }
-  for (int k = tid; k < D * (MSP + 1); k += NT) {
-    const int ax = k / (MSP + 1), j = k - ax * (MSP + 1);
-    const double t = g.ax[ax].hx * (double)j;
-    sh.cj[ax][j] = exp(-(t * t) / g.four_tau[ax]);
   }
   // items in a grid-stride loop: most CTAs of a launch sized by the tiles of
   // the whole (padded) grid would find none
@@ -867,21 +837,12 @@ tile_accumulate_reg_kernel(SpreadGeom g, int nchan, const int* __restrict__ offs
       sync2<NW>();  // this batch's records are there, the last one's readers done
       if (b0 + lane < b1) {
         const double* r = &sh.st.rec[half][lane * RS];
-        constexpr bool kExp = D == 2 && !std::is_same<Acc, double>::value;
-        if (NW == 1 || warp == 0) {
-          if constexpr (kExp)
-            tap_weights_exp<NT1>(r[D - 2], hy, g.four_tau[D - 2], ify, sh.st.wy + lane * NT1);
-          else
-            tap_weights<NT1>(r[D - 2], 1.0, hy, ify, sh.cj[D - 2], sh.st.wy + lane * NT1);
-        }
-        if (NW == 1 || warp == 1) {
-          if constexpr (kExp)
-            tap_weights_exp<NT1>(r[D - 1], hx, g.four_tau[D - 1], ifx, sh.st.wx + lane * WXS);
-          else
-            tap_weights<NT1>(r[D - 1], 1.0, hx, ifx, sh.cj[D - 1], sh.st.wx + lane * WXS);
-        }
+        if (NW == 1 || warp == 0)
+          tap_weights<NT1>(r[D - 2], 1.0, hy, g.four_tau[D - 2], ify, sh.st.wy + lane * NT1);
+        if (NW == 1 || warp == 1)
+          tap_weights<NT1>(r[D - 1], 1.0, hx, g.four_tau[D - 1], ifx, sh.st.wx + lane * WXS);
         if (D == 3 && warp < nv)
-          tap_weights<NT1>(r[0], r[3 + warp], g.ax[0].hx, 1.0 / g.four_tau[0], sh.cj[0],
+          tap_weights<NT1>(r[0], r[3 + warp], g.ax[0].hx, g.four_tau[0], ifz,
                            sh.st.val + lane * VS + c_w);
       }
       sync2<NW>();
