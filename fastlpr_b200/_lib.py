@@ -54,6 +54,7 @@ SIGNATURES = [
     ("flpr_conv_full", _I, [_VP, _I, _PI, _PI, _PI, _I, _VP, _VP, _I, _PI, _PI, _D, _I, _VP, _I,
                             _VP, _SZ, _VP]),
     ("flpr_conv_ws", _SZ, [_VP, _I, _PI, _I, _I]),
+    ("flpr_conv_grid_ws", _SZ, [_VP, _I, _PI, _PI, _I, _I]),
     ("flpr_conv2d_sep_ws", _SZ, [_VP, _PI, _PI, _I, _I]),
     ("flpr_conv2d_sep", _I, [_VP, _PI, _PI, _PI, _I, _I, _VP, _VP, _I, _PI, _PI, _PI, _D, _I, _VP,
                              _I, _VP, _SZ, _VP]),

@@ -828,14 +828,15 @@ def _conv(ctx: _Ctx, geom: _Geom, spec, kern: _Kernel, prods: _Products, prec: i
                                           out.data_ptr(), prec, ws.data_ptr(), ws.numel(),
                                           ctx.stream), "flpr_conv2d_sep")
         return out
-    ws = ctx.ws(ctx.lib.flpr_conv_ws(ctx.handle, d, tab.L_c, nprod, prec))
     if kern.separable:
+        ws = ctx.ws(ctx.lib.flpr_conv_grid_ws(ctx.handle, d, tab.G_c, tab.L_c, nprod, prec))
         ctx.check(ctx.lib.flpr_conv(ctx.handle, d, *tab.lq, kern.H, kern.npow, spec.data_ptr(),
                                     kern.data_ptr(), nprod, prods.chan, prods.hidx, prods.pw,
                                     kern.scale, 1 if add_eps else 0, out.data_ptr(), prec,
                                     ws.data_ptr(), ws.numel(), ctx.stream), "flpr_conv")
     else:
         kidx = [kern.elems[p[2]] * kern.H + p[1] for p in prods.prods]
+        ws = ctx.ws(ctx.lib.flpr_conv_ws(ctx.handle, d, tab.L_c, nprod, prec))
         ctx.check(ctx.lib.flpr_conv_full(ctx.handle, d, *tab.lq, len(kern.elems) * kern.H,
                                          spec.data_ptr(), kern.data_ptr(), nprod, prods.chan,
                                          _lib.ivec(kidx), kern.scale, 1 if add_eps else 0,

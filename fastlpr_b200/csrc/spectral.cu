@@ -446,6 +446,22 @@ static int conv_batch(int d, const int* L, int nprod, int prec) {
   return (int)b;
 }
 
+// Workspace of a batch of products and of their transforms, whose plans
+// `work(nb, &bytes)` sizes: the full batches and the last one.
+template <typename Work>
+static size_t conv_ws_of(int d, const int* L, int nprod, int prec, Work work) {
+  const int B = conv_batch(d, L, nprod, prec), tail = nprod % B;
+  const int64_t cells = prod(L, d), half = cells / L[d - 1] * (L[d - 1] / 2 + 1);
+  const size_t es = prec == FLPR_PREC_F32 ? 4 : 8;
+  size_t w1 = 0, w2 = 0;
+  if (work(B, &w1) != FLPR_OK || (tail && work(tail, &w2) != FLPR_OK)) return 0;
+  ArenaSize ar;
+  ar.take<char>((size_t)B * half * 2 * es);
+  ar.take<char>((size_t)B * cells * es);
+  ar.take<char>(w1 > w2 ? w1 : w2);
+  return ar.used;
+}
+
 static int grid_blocks(int64_t total) {
   int64_t b = (total + 255) / 256;
   int64_t cap = 32 * (int64_t)sm_count();
@@ -633,39 +649,25 @@ static PlanKey conv3_planes(const int* L, int planes, int prec) {
   return grid_plan(2, L + 1, prec == FLPR_PREC_F32 ? CUFFT_C2R : CUFFT_Z2D, planes);
 }
 
-// Largest work area of a batch of nb products; G0 is unknown to the size
-// query, whose caller may keep every plane.
-static int conv3_work(flpr_handle_t handle, const int* L, int nb, int prec, size_t* out) {
-  size_t a = 0, b = 0;
-  FLPR_TRY(plans_of(handle).work_size(conv3_axis0(L, nb, prec), &a));
-  FLPR_TRY(plans_of(handle).work_size(conv3_planes(L, nb * L[0], prec), &b));
-  *out = a > b ? a : b;
-  return FLPR_OK;
-}
-
 size_t flpr_conv_ws(flpr_handle_t handle, int d, const int* h_L, int nprod, int prec) {
   if (d < 1 || d > 3 || nprod < 1) return 0;
-  int B = conv_batch(d, h_L, nprod, prec);
-  int64_t cells = prod(h_L, d);
-  int64_t half = cells / h_L[d - 1] * (h_L[d - 1] / 2 + 1);
-  size_t es = prec == FLPR_PREC_F32 ? 4 : 8;
-  ArenaSize ar;
-  ar.take<char>((size_t)B * half * 2 * es);
-  ar.take<char>((size_t)B * cells * es);
-  int type = prec == FLPR_PREC_F32 ? CUFFT_C2R : CUFFT_Z2D;
-  size_t w1 = 0, w2 = 0;
-  if (plans_of(handle).work_size(grid_plan(d, h_L, type, B), &w1) != FLPR_OK) return 0;
-  int tail = nprod % B;
-  if (tail && plans_of(handle).work_size(grid_plan(d, h_L, type, tail), &w2) != FLPR_OK) return 0;
-  if (w2 > w1) w1 = w2;
-  if (d == 3) {
-    if (conv3_work(handle, h_L, B, prec, &w2) != FLPR_OK) return 0;
-    if (w2 > w1) w1 = w2;
-    if (tail && conv3_work(handle, h_L, tail, prec, &w2) != FLPR_OK) return 0;
-    if (w2 > w1) w1 = w2;
-  }
-  ar.take<char>(w1);
-  return ar.used;
+  const int type = prec == FLPR_PREC_F32 ? CUFFT_C2R : CUFFT_Z2D;
+  return conv_ws_of(d, h_L, nprod, prec, [&](int nb, size_t* out) {
+    return plans_of(handle).work_size(grid_plan(d, h_L, type, nb), out);
+  });
+}
+
+size_t flpr_conv_grid_ws(flpr_handle_t handle, int d, const int* h_G, const int* h_L, int nprod,
+                         int prec) {
+  if (d != 3) return flpr_conv_ws(handle, d, h_L, nprod, prec);
+  if (nprod < 1 || h_G[0] < 1) return 0;
+  return conv_ws_of(d, h_L, nprod, prec, [&](int nb, size_t* out) {
+    size_t a = 0, b = 0;
+    FLPR_TRY(plans_of(handle).work_size(conv3_axis0(h_L, nb, prec), &a));
+    FLPR_TRY(plans_of(handle).work_size(conv3_planes(h_L, nb * h_G[0], prec), &b));
+    *out = a > b ? a : b;
+    return FLPR_OK;
+  });
 }
 
 int flpr_conv(flpr_handle_t handle, int d, const int* h_G, const int* h_L, const int* h_qout,
@@ -697,7 +699,11 @@ int flpr_conv(flpr_handle_t handle, int d, const int* h_G, const int* h_L, const
     for (int a = 0; a < d; ++a)
       FLPR_CHECK_ARG(h_pow[p * d + a] >= 0 && h_pow[p * d + a] < npow, "conv: pow out of range");
   }
-  if (ws_bytes < flpr_conv_ws(handle, d, h_L, nprod, prec)) {
+  // 3-D: the kept planes only, unless the workspace was sized without the grid
+  // (flpr_conv_ws) and the plans of that form want more
+  const size_t grid_ws = d == 3 ? flpr_conv_grid_ws(handle, d, h_G, h_L, nprod, prec) : 0;
+  const bool kept_planes = grid_ws > 0 && ws_bytes >= grid_ws;
+  if (!kept_planes && ws_bytes < flpr_conv_ws(handle, d, h_L, nprod, prec)) {
     set_error("conv: workspace too small");
     return FLPR_ERR_WORKSPACE;
   }
@@ -724,7 +730,7 @@ int flpr_conv(flpr_handle_t handle, int d, const int* h_G, const int* h_L, const
       for (int a = 0; a < 3; ++a) pd.pw[a] = a < d ? (unsigned short)h_pow[(p0 + b) * d + a] : 0;
       batch.p[b] = pd;
     }
-    ca.nb = d == 3 ? nb : 0;
+    ca.nb = kept_planes ? nb : 0;
     if (prec == FLPR_PREC_F32) {
       product_kernel<float><<<prod_grid(ca, nb), 256, 0, s>>>(ca, batch, (const float2*)d_spec,
                                                               (const double2*)d_F, (float2*)pbuf);
@@ -733,7 +739,7 @@ int flpr_conv(flpr_handle_t handle, int d, const int* h_G, const int* h_L, const
           ca, batch, (const double2*)d_spec, (const double2*)d_F, (double2*)pbuf);
     }
     FLPR_LAUNCH_CHECK();
-    if (d == 3) {
+    if (kept_planes) {
       const size_t plane = (size_t)nb * h_L[1] * (h_L[2] / 2 + 1) * 2 * es;
       FLPR_TRY(plans_of(handle).exec(conv3_axis0(h_L, nb, prec), pbuf, pbuf, work, work_bytes, s));
       FLPR_TRY(plans_of(handle).exec(conv3_planes(h_L, nb * h_G[0], prec),

@@ -210,8 +210,14 @@ int flpr_kernel_factors(flpr_handle_t handle, int d, const int* h_G, const int* 
  * d_out + p * prod(G) elements (float or double, per prec); when
  * add_eps is set the float64 machine epsilon is added (regression.py:116).
  * h_scale: global factor applied to every product (1/(sqrt(2pi) prod L)).
+ * Workspace: flpr_conv_grid_ws, or flpr_conv_ws where the kept grid is not
+ * known.  The inverse of a 3-D product runs axis 0 first and the other two on
+ * the kept planes only; a workspace of flpr_conv_ws that this form's
+ * transforms do not fit is given the whole inverse instead.
  * --------------------------------------------------------------------- */
 size_t flpr_conv_ws(flpr_handle_t handle, int d, const int* h_L, int nprod, int prec);
+size_t flpr_conv_grid_ws(flpr_handle_t handle, int d, const int* h_G, const int* h_L, int nprod,
+                         int prec);
 int flpr_conv(flpr_handle_t handle, int d, const int* h_G, const int* h_L, const int* h_qout,
               int H, int npow, const void* d_spec, const void* d_F,
               int nprod, const int* h_chan, const int* h_hidx, const int* h_pow,
