@@ -87,3 +87,42 @@ def test_tap_weights_are_as_accurate_as_an_exponential_per_tap(cuda_ok, d):
         num += float(np.sum((got[ix] - e2) ** 2))
         den += float(np.sum((w2 - e2) ** 2))
     assert num ** 0.5 < 1.15 * den ** 0.5
+
+
+@pytest.mark.parametrize("d,n,G,C,msp", [
+    (1, 2, [2], 1, 4), (1, 255, [40], 32, 4), (1, 257, [300], 1, 4), (1, 3001, [1500], 31, 0),
+    (2, 257, [40, 9], 11, 7), (2, 1500, [64, 48], 32, 12), (2, 400, [5, 20], 1, 9)])
+def test_sorted_deposits_on_lines_and_under_wide_stencils(cuda_ok, d, n, G, C, msp):
+    """The shared-memory deposits: one dimension, and the wider tiles of 2-D
+    stencils beyond 13 taps, against one FP64 atomic per point, corner and
+    channel (both round 2^-62 and 2^-53 of the channel's sum)."""
+    import torch
+    from conftest import rel_err
+    from fastlpr_b200 import _lib, api
+    rng = np.random.default_rng(n + C)
+    x, cols = rng.random((n, d)), rng.standard_normal((n, C)) * 10.0 ** rng.integers(-3, 4, C)
+    ctx = api._Ctx(torch.device("cuda", 0))
+    dx = ctx.upload(x)
+    geom = api._make_geom(api._point_stats(ctx, dx, n, d), n, d, np.asarray(G), 4, True)
+    dc = [ctx.upload(np.ascontiguousarray(c)) for c in cols.T]
+    ptrs = _lib.pvec([c.data_ptr() for c in dc])
+    L, Gv = _lib.ivec(geom.L), _lib.ivec(G)
+    grid = ctx.empty((1 + C, int(np.prod(geom.L))))
+    ws = ctx.ws(ctx.lib.flpr_spread_ws(d, n, L, msp, 1 + C, 1))
+    _lib.check(ctx.lib.flpr_spread(d, n, dx.data_ptr(), _lib.dvec(geom.kmap.ravel()), L, msp,
+                                   _lib.dvec(geom.tau), 1 + C, 1, ptrs, grid.data_ptr(), 1,
+                                   ws.data_ptr(), ws.numel(), ctx.stream), "spread")
+    ax = _lib.dvec(api._axes_arg(api._raw_axes(geom, {})))
+    M, NP = int(np.prod(G)), (2 ** d) * (2 ** d + 1) // 2
+    a, b = ([ctx.empty((M, C)), ctx.empty((M, NP)), ctx.empty(C)] for _ in range(2))
+    ws2 = ctx.ws(ctx.lib.flpr_deposit_sorted_ws(d, n, L, msp, 1 + C))
+    _lib.check(ctx.lib.flpr_deposit_sorted(d, n, dx.data_ptr(), L, msp, 1 + C, 1, ptrs, ws.data_ptr(),
+                                           ws.numel(), ax, Gv, _lib.ivec(api._node0_cells(geom)),
+                                           *[t.data_ptr() for t in a], ws2.data_ptr(), ws2.numel(),
+                                           ctx.stream), "deposit_sorted")
+    _lib.check(ctx.lib.flpr_deposit(d, n, dx.data_ptr(), ax, Gv, C, ptrs,
+                                    *[t.data_ptr() for t in b], ctx.stream), "deposit")
+    for u, v in zip(a, b):
+        u, v = u.cpu().numpy(), v.cpu().numpy()
+        for k in range(u.shape[-1]):
+            assert rel_err(u[..., k], v[..., k]) < 1e-12
