@@ -3,8 +3,9 @@
 Tuned parameters (process-wide library settings, ``flpr_set_tuning``):
 
 * ``spread_item_points`` -- points per spread work item (one CTA of the
-  tile-accumulation kernels): small items spread a dense tile over more
-  CTAs, large items cut the per-item overhead;
+  tile-accumulation kernels; in 2-D and 3-D the size that the library chooses
+  from the number of points, times this over 4096): small items spread a dense
+  tile over more CTAs, large items cut the per-item overhead;
 * ``fused_chunk_mb`` -- column-pass output budget of the fused 2-D
   convolution, i.e. how many bandwidths one column pass / row pass pair
   covers (more bandwidths per chunk: more row-pass CTAs, more traffic);
@@ -31,6 +32,9 @@ import torch
 from . import _lib
 
 PARAMS = {"spread_item_points": 0, "fused_chunk_mb": 1}
+# of the settings' meaning; part of every cache key, so that records of another
+# meaning are measured again
+VERSION = 2
 ITEM_POINTS = (1024, 2048, 4096, 8192)
 CHUNK_MB = (192, 384, 768, 1536)
 
@@ -121,7 +125,7 @@ def tune_fit(x, y, h, options: Optional[dict] = None, force: bool = False) -> di
     su = api._lpr_setup(x, y, h, options)
     dev = api._device(su.opts)
     G = api._grid_shape(su.opts, su.n, su.d)
-    key = "fit|" + "|".join(str(v) for v in (
+    key = f"fit/{VERSION}|" + "|".join(str(v) for v in (
         device_key(dev), su.d, tuple(int(g) for g in G), su.order, su.dy, su.y_is_complex,
         su.prec, su.bandwidths.shape[0], int(su.opts.get("num_dof_sample", 10)),
         int(np.round(np.log2(max(su.n, 1)))), str(su.opts.get("kernel_type", "gaussian"))))

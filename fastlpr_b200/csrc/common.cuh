@@ -23,6 +23,7 @@ void set_error(const char* fmt, ...);
 // Number of kernels this library has launched (flpr_launch_count()).
 void count_launch();
 // process-wide tuning parameters (flpr_set_tuning)
+constexpr int kTuneItemPoints = 4096;  // default of FLPR_TUNE_SPREAD_ITEM_POINTS
 int tuning(int param);
 
 #define FLPR_CHECK_ARG(cond, ...)            \

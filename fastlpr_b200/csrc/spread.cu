@@ -999,13 +999,15 @@ static void make_geom(SpreadGeom& g, int d, const int* L, int msp, const double*
 // Points per work item, the same for the spread and for the deposits that
 // read its records.  Grids with few tiles (small 1-D grids): about four items
 // per SM.  Register path, one or two warps per item: at least 24 warps' worth of items per
-// SM (two rounds of the resident ones), 256 to 1024 points.
+// SM (two rounds of the resident ones), 256 to 1024 points, times the setting
+// over its default, with a batch of the staged points at least.
 static void size_items(SpreadGeom& g, int64_t n, bool reg) {
   if (reg) {
     const int64_t per = n / (24LL * sm_count());
-    int ip = 256;
+    int64_t ip = 256;
     while (ip < per && ip < kItem2) ip <<= 1;
-    if (ip < g.item_points) g.item_points = ip;
+    ip = ip * g.item_points / kTuneItemPoints;
+    g.item_points = (int)(ip < 32 ? 32 : (ip > kItem2 ? kItem2 : ip));
     return;
   }
   const int64_t target = 4LL * sm_count();

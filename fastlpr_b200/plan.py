@@ -259,7 +259,7 @@ class LprPlan:
         sig = sorted((p.d, tuple(int(v) for v in p.geom.L), p.su.order, p.su.dy,
                       p.su.y_is_complex, int(np.round(np.log2(p.su.n))), len(p.filt[2]))
                      for p in self.probs)
-        key = "plan|" + at.device_key(self.device) + "|" + str(hash(tuple(sig)) & 0xFFFFFFFF)
+        key = f"plan/{at.VERSION}|" + at.device_key(self.device) + "|" + str(hash(tuple(sig)) & 0xFFFFFFFF)
         saved = at.get_params()
         cands = [{"streams": s, "spread_item_points": a}
                  for s in (2, 4, 8, 16) if s <= max(2, len(self.probs))

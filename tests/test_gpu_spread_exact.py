@@ -126,3 +126,74 @@ def test_sorted_deposits_on_lines_and_under_wide_stencils(cuda_ok, d, n, G, C, m
         u, v = u.cpu().numpy(), v.cpu().numpy()
         for k in range(u.shape[-1]):
             assert rel_err(u[..., k], v[..., k]) < 1e-12
+
+
+@pytest.mark.parametrize("d,G,n", [(2, [96, 80], 40000), (3, [12, 10, 14], 60000), (1, [400], 500000)])
+def test_the_item_size_setting_changes_the_work_items(cuda_ok, d, G, n):
+    """Every candidate of the autotuner makes another number of work items of
+    clustered points, and the same grid."""
+    import torch
+    from fastlpr_b200 import _lib, api, autotune
+    rng = np.random.default_rng(n)
+    x = 0.4 + 0.02 * rng.random((n, d))
+    x[0], x[1] = 0.0, 1.0
+    ctx = api._Ctx(torch.device("cuda", 0))
+    dx, y = ctx.upload(x), ctx.upload(rng.standard_normal(n))
+    geom = api._make_geom(api._point_stats(ctx, dx, n, d), n, d, np.asarray(G), 4, True)
+    L = _lib.ivec(geom.L)
+    ws = ctx.ws(ctx.lib.flpr_spread_ws(d, n, L, 4, 2, 0))
+    tiles = [-(-int(v) // t) for v, t in zip(geom.L, {1: [256], 2: [8, 8], 3: [1, 8, 8]}[d])]
+    # the workspace begins with the tiles' counts, their offsets and their first work items
+    ntiles = int(np.prod(tiles))
+    first = (-(-4 * ntiles // 256) - (-4 * (ntiles + 1) // 256)) * 64
+    saved = autotune.get_params()
+    items, grids = [], []
+    try:
+        for ip in autotune.ITEM_POINTS:
+            autotune.set_params({"spread_item_points": ip})
+            grid = ctx.empty((2, int(np.prod(geom.L))), dtype=torch.float32)
+            _lib.check(ctx.lib.flpr_spread(d, n, dx.data_ptr(), _lib.dvec(geom.kmap.ravel()), L, 4,
+                                           _lib.dvec(geom.tau), 2, 1, _lib.pvec([y.data_ptr()]),
+                                           grid.data_ptr(), 0, ws.data_ptr(), ws.numel(), ctx.stream),
+                       "spread")
+            items.append(int(ws[:4 * (first + ntiles + 1)].view(torch.int32)[-1]))
+            grids.append(grid)
+    finally:
+        autotune.set_params(saved)
+    assert len(set(items)) == (len(items) if d > 1 else 1)
+    assert all(torch.equal(g, grids[0]) for g in grids)
+
+
+@pytest.mark.parametrize("m", [1023, 1024, 1025])
+@pytest.mark.parametrize("d,prec", [(2, 0), (2, 1), (3, 0), (3, 1)])
+def test_the_largest_work_items(cuda_ok, d, prec, m):
+    """A tile that fills the largest work item but one point, all of it, and
+    one point more, against the oracle; the rounding of the grid's type."""
+    import torch
+    from conftest import rel_err
+    from fastlpr_b200 import _lib, api, autotune
+    rng = np.random.default_rng(m + d)
+    G, n = [40, 40, 40][:d], m + 2
+    ctx = api._Ctx(torch.device("cuda", 0))
+    x = 0.5 + 0.0001 * rng.random((n, d))
+    x[0], x[1] = 0.0, 1.0
+    dx, v = ctx.upload(x), rng.standard_normal((n, 3))
+    geom = api._make_geom(api._point_stats(ctx, dx, n, d), n, d, np.asarray(G), 4, True)
+    cols = [ctx.upload(np.ascontiguousarray(c)) for c in v.T]
+    L = _lib.ivec(geom.L)
+    grid = ctx.empty((3, int(np.prod(geom.L))), dtype=torch.float64 if prec else torch.float32)
+    ws = ctx.ws(ctx.lib.flpr_spread_ws(d, n, L, 4, 3, prec))
+    saved = autotune.get_params()
+    try:
+        autotune.set_params({"spread_item_points": 65536})
+        _lib.check(ctx.lib.flpr_spread(d, n, dx.data_ptr(), _lib.dvec(geom.kmap.ravel()), L, 4,
+                                       _lib.dvec(geom.tau), 3, 0, _lib.pvec([c.data_ptr() for c in cols]),
+                                       grid.data_ptr(), prec, ws.data_ptr(), ws.numel(), ctx.stream), "spread")
+    finally:
+        autotune.set_params(saved)
+    xs = (x - geom.mean) / geom.std - geom.center
+    knots = oracle.knot_coordinates(xs, geom.L, np.asarray(G), geom.qin)
+    want = oracle.spread_grid(knots, v, geom.L, 4, geom.tau)
+    got = grid.double().cpu().numpy().reshape(want.shape) * n
+    for c in range(3):
+        assert rel_err(got[c], want[c]) < (1e-12 if prec else 2e-7)
