@@ -221,6 +221,10 @@ class LprPlan:
                         p.bufs[k] = torch.empty(t.shape, dtype=t.dtype, pin_memory=True)
             self._graph_downloads = True
         del outs
+        # an earlier plan that only the collector can free (an exception's
+        # frames hold it) would be freed inside a capture, where releasing its
+        # graphs and buffers is an error: free it now
+        gc.collect()
         # one graph per part, each with its own memory pool (the parts'
         # replays overlap on the device)
         self.segs = []
@@ -228,16 +232,8 @@ class LprPlan:
             graph = torch.cuda.CUDAGraph()
             cap = torch.cuda.Stream(self.device)
             cap.wait_stream(torch.cuda.current_stream(self.device))
-            # a collection inside the capture could free an earlier plan's
-            # graphs and buffers, a call that ends the capture
-            collecting = gc.isenabled()
-            gc.disable()
-            try:
-                with torch.cuda.graph(graph, stream=cap):
-                    outs = self._issue(idx)
-            finally:
-                if collecting:
-                    gc.enable()
+            with torch.cuda.graph(graph, stream=cap):
+                outs = self._issue(idx)
             self.segs.append(_Segment(idx, graph, outs, self._finite,
                                       torch.cuda.Stream(self.device)))
         torch.cuda.synchronize(self.device)
