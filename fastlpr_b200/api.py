@@ -1614,7 +1614,7 @@ def _finalize_enqueue(ctx, st: _LprState, r: dict, ev, device_select: bool = Fal
         if not st.variance and st.methods["output"] != "cubic" and ny <= 32:
             # every output in one buffer: one launch forms them in the layouts
             # of the result, one copy brings them down
-            pack = ctx.empty(2 * n * ny + M * (ny + 1) + 4 * H + 1)
+            pack = ctx.empty(sum(_pack_sizes(st, H)))
         sel_dev = ctx.empty(1, dtype=torch.int32)
         if st.calc_dof:
             if hsum_dev is None:
@@ -1651,7 +1651,7 @@ def _finalize_enqueue(ctx, st: _LprState, r: dict, ev, device_select: bool = Fal
                       "flpr_fit_outputs")
             ev.mark("final_interp")
             if bufs is None:
-                return {"pack": _to_host(pack)}
+                return {"pack": _pack_to_host(pack, _pack_sizes(st, H))}
             if bufs.get("pack") is None:
                 return {"pack": pack}
             bufs["pack"].copy_(pack, non_blocking=True)
@@ -1739,22 +1739,42 @@ def _output_bufs(st: _LprState, H: int) -> dict:
             "gcv": pin(4 * H) if st.calc_dof else None, "sel": pin(1, torch.int32)}
 
 
-def _unpack_outputs(st: _LprState, r: dict, pack: torch.Tensor) -> dict:
-    """The outputs of _finalize_enqueue as views of the downloaded buffer
-    {fitted values (n, ny), residuals (n, ny), surface (M, ny), s0 (M), GCV
-    arrays (4 H), index}."""
+def _pack_sizes(st: _LprState, H: int) -> List[int]:
+    """Numbers in the parts of the buffer of _finalize_enqueue: {fitted values
+    (n, ny), residuals (n, ny), surface (M, ny), s0 (M), GCV arrays (4 H) and
+    index}."""
+    return [st.n * st.ny, st.n * st.ny, st.geom.M * st.ny, st.geom.M, 4 * H + 1]
+
+
+def _pack_to_host(pack: torch.Tensor, sizes: List[int]):
+    """Asynchronous copy of the outputs into fresh pinned memory: one copy, or,
+    from _STAGE_MIN_BYTES on, one per part (a result that the caller keeps then
+    keeps no more than itself page-locked; a copy and its buffer cost about
+    10 us)."""
+    if pack.numel() * 8 < _STAGE_MIN_BYTES:
+        return _to_host(pack)
+    return [_to_host(t) for t in pack.split(sizes)]
+
+
+def _unpack_outputs(st: _LprState, r: dict, pack) -> dict:
+    """The outputs of _finalize_enqueue from the downloaded buffer, or from the
+    buffers of its parts (_pack_to_host).  Parts of one buffer are views of it,
+    which keep all of it: those of less than an eighth are copied out."""
     n, ny, M, H = st.n, st.ny, st.geom.M, r["H"]
-    v = pack.numpy()
+    if isinstance(pack, torch.Tensor):
+        parts = [t.numpy() for t in pack.split(_pack_sizes(st, H))]
+        parts = [v.copy() if 8 * v.size < pack.numel() else v for v in parts]
+    else:
+        parts = [t.numpy() for t in pack]
 
     def shaped(t, k):
         if st.y_is_complex:
             t = t.view(np.complex128)
         return t if st.dy == 1 else t.reshape(k, st.dy)
 
-    a, b, c = n * ny, 2 * n * ny, 2 * n * ny + M * ny
-    return {"yh": shaped(v[:a], n), "rh": shaped(v[a:b], n), "gvh": shaped(v[b:c], M),
-            "s0h": v[c:c + M], "dn": None,
-            "gcv": v[c + M:c + M + 4 * H] if st.calc_dof else None, "sel": v[-1:]}
+    yh, rh, gvh, s0h, tail = parts
+    return {"yh": shaped(yh, n), "rh": shaped(rh, n), "gvh": shaped(gvh, M), "s0h": s0h,
+            "dn": None, "gcv": tail[:4 * H] if st.calc_dof else None, "sel": tail[-1:]}
 
 
 def _finalize_build(ctx, st: _LprState, r: dict, pend: dict, ev, search,

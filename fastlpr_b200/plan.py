@@ -542,7 +542,8 @@ class LprPlan:
                     p = self.probs[i]
                     st, r, pend = outs[i]
                     self._copy.wait_event(p.done)
-                    pends[i] = {k: (api._to_host(v) if isinstance(v, torch.Tensor)
+                    pends[i] = {k: (api._pack_to_host(v, api._pack_sizes(st, r["H"])) if k == "pack"
+                                    else api._to_host(v) if isinstance(v, torch.Tensor)
                                     and v.is_cuda else v) for k, v in pend.items()}
                     if p.lidx is None:
                         done[i] = torch.cuda.Event()
