@@ -177,8 +177,7 @@ class _Ctx:
         self.index = device.index if device.index is not None else torch.cuda.current_device()
         self.lib = _lib.load()
         self.handle = _lib.handle(self.index)
-        torch.cuda.init()
-        self.stream = torch._C._cuda_getCurrentRawStream(self.index)
+        self.stream = torch.cuda.current_stream(device).cuda_stream
 
     def empty(self, shape, dtype=torch.float64):
         return torch.empty(shape, dtype=dtype, device=self.device)
