@@ -1233,8 +1233,9 @@ def _prepare_lpr(ctx, x_arr, y_arr, dy, opts, order, prec, variance, y_is_comple
         st.Q = ctx.empty((M, Cv))
         st.Bst = ctx.empty((M, npair))
         st.sq = ctx.empty(Cv)
-        if kept and d <= 2 and kept["C"] == 1 + Cv:
-            # from the spread's tile-sorted records: exact and order-free
+        if kept and d <= 2 and kept["C"] == 1 + Cv and all(st.ax_arg[1::2]):
+            # from the spread's tile-sorted records: exact and order-free (but
+            # no NaN, which an axis without extent makes of every sum)
             ws2 = ctx.ws(lib.flpr_deposit_sorted_ws(d, n, kept["L_c"], kept["msp"],
                                                     kept["C"]))
             ctx.check(lib.flpr_deposit_sorted(d, n, dx.data_ptr(), kept["L_c"],

@@ -220,4 +220,26 @@ __device__ __forceinline__ double knot_of(double x, const KnotAxis& a) {
   return np_mod(k, 6.283185307179586);
 }
 
+// Cell and fraction on one axis, clamped like interp_optimized.py:60-78.  A
+// coordinate that is NaN, or any on an axis without extent (0 / 0), has no
+// cell: its fraction is NaN, in cell 0, so that the value is NaN and the reads
+// stay on the grid.
+__device__ __forceinline__ void axis_cell(double xi, double x0, double dx, int nx, int* ix,
+                                          double* fr) {
+  const double t = (xi - x0) / dx;
+  if (t < 0.0) {
+    *ix = 0;
+    *fr = 0.0;
+  } else if (t >= (double)(nx - 1)) {
+    *ix = nx - 2 < 0 ? 0 : nx - 2;
+    *fr = 1.0;
+  } else if (t != t) {
+    *ix = 0;
+    *fr = t;
+  } else {
+    *ix = (int)t;
+    *fr = t - (double)*ix;
+  }
+}
+
 }  // namespace flpr

@@ -12,23 +12,6 @@ struct InterpGeom {
   int64_t M;
 };
 
-// Cell and fraction on one axis, clamped like interp_optimized.py:60-78.
-__device__ __forceinline__ void axis_cell(double xi, double x0, double dx, int nx, int* ix,
-                                          double* fr) {
-  double t = (xi - x0) / dx;
-  if (t < 0.0) {
-    *ix = 0;
-    *fr = 0.0;
-  } else if (t >= (double)(nx - 1)) {
-    *ix = nx - 2 < 0 ? 0 : nx - 2;
-    *fr = 1.0;
-  } else {
-    int i = (int)t;
-    *ix = i;
-    *fr = t - (double)i;
-  }
-}
-
 // Corner offsets/weights of the multilinear stencil of point i.
 struct Stencil {
   int64_t base[8];

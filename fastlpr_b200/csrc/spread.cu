@@ -1511,18 +1511,8 @@ tile_deposit_kernel(SpreadGeom g, DepositGeom dg, int64_t n, const double* __res
       double fr[2] = {0.0, 0.0};
 #pragma unroll
       for (int a = 0; a < D; ++a) {
-        // the clamped cell of interp_optimized.py:60-78 (the fitted values' stencil)
-        const double t = (x[i * D + a] - dg.x0[a]) / dg.dx[a];
-        if (t < 0.0) {
-          ix[a] = 0;
-          fr[a] = 0.0;
-        } else if (t >= (double)(dg.G[a] - 1)) {
-          ix[a] = dg.G[a] - 2;
-          fr[a] = 1.0;
-        } else {
-          ix[a] = (int)t;
-          fr[a] = t - (double)ix[a];
-        }
+        axis_cell(x[i * D + a], dg.x0[a], dg.dx[a], dg.G[a], &ix[a], &fr[a]);
+        if (fr[a] != fr[a]) fr[a] = 0.0;  // no cell; integers hold no NaN
       }
       bool inside = true;
 #pragma unroll
@@ -1663,18 +1653,8 @@ tile_deposit2_kernel(SpreadGeom g, DepositGeom dg, const double* __restrict__ x,
       bool inside = true;
 #pragma unroll
       for (int a = 0; a < 2; ++a) {
-        // the clamped cell of interp_optimized.py:60-78 (the fitted values' stencil)
-        const double t = (x[i * 2 + a] - dg.x0[a]) / dg.dx[a];
-        if (t < 0.0) {
-          ix[a] = 0;
-          fr[a] = 0.0;
-        } else if (t >= (double)(dg.G[a] - 1)) {
-          ix[a] = dg.G[a] - 2;
-          fr[a] = 1.0;
-        } else {
-          ix[a] = (int)t;
-          fr[a] = t - (double)ix[a];
-        }
+        axis_cell(x[i * 2 + a], dg.x0[a], dg.dx[a], dg.G[a], &ix[a], &fr[a]);
+        if (fr[a] != fr[a]) fr[a] = 0.0;  // no cell; integers hold no NaN
         const int l = ix[a] - org[a];
         inside = inside && l >= 0 && l < kDepCells;
       }
