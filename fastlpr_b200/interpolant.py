@@ -11,6 +11,7 @@ convention: points are ``np.atleast_2d``'d, so 1-D data is passed as an
 """
 from __future__ import annotations
 
+import functools
 from typing import Sequence
 
 import numpy as np
@@ -46,7 +47,7 @@ class GridInterpolant:
             ax += [float(a[0]), float(a[1] - a[0]) if len(a) > 1 else 1.0]
         self._ax = ax
 
-    @property
+    @functools.cached_property
     def bounds(self):
         return [(a.min(), a.max()) for a in self.grid_axes]
 
