@@ -1760,10 +1760,13 @@ def _unpack_outputs(st: _LprState, r: dict, pack) -> dict:
     """The outputs of _finalize_enqueue from the downloaded buffer, or from the
     buffers of its parts (_pack_to_host).  Parts of one buffer are views of it,
     which keep all of it: those of less than an eighth are copied out."""
-    n, ny, M, H = st.n, st.ny, st.geom.M, r["H"]
+    n, M, H = st.n, st.geom.M, r["H"]
     if isinstance(pack, torch.Tensor):
-        parts = [t.numpy() for t in pack.split(_pack_sizes(st, H))]
-        parts = [v.copy() if 8 * v.size < pack.numel() else v for v in parts]
+        whole, parts, at = pack.numpy(), [], 0
+        for k in _pack_sizes(st, H):
+            part = whole[at:at + k]
+            parts.append(part.copy() if 8 * k < whole.size else part)
+            at += k
     else:
         parts = [t.numpy() for t in pack]
 
