@@ -998,13 +998,20 @@ static void make_geom(SpreadGeom& g, int d, const int* L, int msp, const double*
 
 // Points per work item, the same for the spread and for the deposits that
 // read its records.  Grids with few tiles (small 1-D grids): about four items
-// per SM.  Register path, one or two warps per item: at least 24 warps' worth of items per
-// SM (two rounds of the resident ones), 256 to 1024 points, times the setting
-// over its default, with a batch of the staged points at least.
+// per SM.  Register path, one or two warps per item, which walk its points one
+// after another: at least 24 warps' worth of items per SM (two rounds of the
+// resident ones), 256 to 1024 points; where those would leave the device
+// empty, 32 to 128, at 3 warps' worth, since every item adds its halo to the
+// grid (spread and deposits, 6 channels: 5e3 points on 70^2 97 us with 256, 84
+// with 32; 2e4 on 40^2 131 with 256, 91 with 64; 12 channels, 1e5 points on
+// 200^2: 178 with 256, 190 with 128).
+// All of it times the setting over its default, with a batch of the staged
+// points at least.
 static void size_items(SpreadGeom& g, int64_t n, bool reg) {
   if (reg) {
     const int64_t per = n / (24LL * sm_count());
-    int64_t ip = 256;
+    int64_t ip = 32;
+    while (ip < 8 * per && ip < 256) ip <<= 1;
     while (ip < per && ip < kItem2) ip <<= 1;
     ip = ip * g.item_points / kTuneItemPoints;
     g.item_points = (int)(ip < 32 ? 32 : (ip > kItem2 ? kItem2 : ip));

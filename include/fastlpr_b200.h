@@ -49,7 +49,7 @@ int64_t flpr_launch_count(void);
  * Set by the autotuner of the Python host (fastlpr_b200/autotune.py).
  *   FLPR_TUNE_SPREAD_ITEM_POINTS: most points per spread work item,
  *     256..65536, default 4096 (2-D and 3-D items in registers: the size
- *     chosen from n, 256 to 1024, times the value / 4096, within 32..1024);
+ *     chosen from n, 32 to 1024, times the value / 4096, within 32..1024);
  *     it must not change between a spread and flpr_deposit_sorted;
  *   FLPR_TUNE_FUSED_CHUNK_MB: column-pass output budget of the fused 2-D
  *     convolution (bandwidths per chunk), 8..16384 MB, default 768. */

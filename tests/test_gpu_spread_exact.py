@@ -197,3 +197,27 @@ def test_the_largest_work_items(cuda_ok, d, prec, m):
     got = grid.double().cpu().numpy().reshape(want.shape) * n
     for c in range(3):
         assert rel_err(got[c], want[c]) < (1e-12 if prec else 2e-7)
+
+
+@pytest.mark.parametrize("d,G,n,item", [(2, [100, 100], 20000, 64), (2, [40, 40], 20000, 64), (3, [12, 12, 12], 9000, 32),
+                                        (2, [60, 80], 100000, 256)])
+def test_few_points_make_small_work_items(cuda_ok, d, G, n, item):
+    """Items of 32 or 64 points where items of 256 would leave most of the device idle."""
+    import torch
+    from fastlpr_b200 import _lib, api
+    x = np.random.default_rng(n).random((n, d))
+    ctx = api._Ctx(torch.device("cuda", 0))
+    dx = ctx.upload(x)
+    geom = api._make_geom(api._point_stats(ctx, dx, n, d), n, d, np.asarray(G), 4, True)
+    L = _lib.ivec(geom.L)
+    ws = ctx.ws(ctx.lib.flpr_spread_ws(d, n, L, 4, 1, 1))
+    grid = ctx.empty(tuple(geom.L))
+    _lib.check(ctx.lib.flpr_spread(d, n, dx.data_ptr(), _lib.dvec(geom.kmap.ravel()), L, 4,
+                                   _lib.dvec(geom.tau), 1, 1, _lib.pvec([]), grid.data_ptr(), 1,
+                                   ws.data_ptr(), ws.numel(), ctx.stream), "spread")
+    ntiles = int(np.prod([-(-int(v) // t) for v, t in zip(geom.L, [8, 8] if d == 2 else [1, 8, 8])]))
+    first = (-(-4 * ntiles // 256) - (-4 * (ntiles + 1) // 256)) * 64
+    ints = ws[:4 * (first + ntiles + 1)].view(torch.int32).cpu().numpy()
+    counts = ints[:ntiles]
+    assert counts.sum() == n and counts.max() > item
+    assert ints[-1] == np.sum(-(-counts // item))
