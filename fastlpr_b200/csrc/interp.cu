@@ -805,26 +805,33 @@ int flpr_kde_scores(int d, int64_t n, const double* d_x, const int* d_order, con
     const int hn = H - h0 < kLcvMaxH ? H - h0 : kLcvMaxH;
     K0g k0;
     for (int j = 0; j < hn; ++j) k0.k0[j] = h_k0[h0 + j];
-    // lanes per point: 16 bandwidths unless 8 leave fewer of them idle
+    // lanes per point: 16 bandwidths unless 8 leave fewer of them idle, and as
+    // many as there are bandwidths up to 4
     const bool wide = (hn + 15) / 16 * 16 <= (hn + 7) / 8 * 8;
-    const int chunks = wide ? (hn + 15) / 16 : (hn + 7) / 8;
+    const int lpp = hn <= 2 ? hn : (hn <= 4 ? 4 : (wide ? 16 : 8));
+    const int chunks = (hn + lpp - 1) / lpp;
     int64_t nb = (8LL * sm_count() + chunks - 1) / chunks;
     const int64_t most = (n + kLcvThreads - 1) / kLcvThreads;
     if (nb > most) nb = most;
     const dim3 grid((unsigned)nb, (unsigned)chunks);
-#define FLPR_LCV(D)                                                                          \
-  if (wide)                                                                                  \
-    kde_lcv_kernel<D, 16><<<grid, kLcvThreads, 0, s>>>(g, n, d_x, d_order, fT, H, h0, hn, k0, \
-                                                       part);                                \
-  else                                                                                       \
-    kde_lcv_kernel<D, 8><<<grid, kLcvThreads, 0, s>>>(g, n, d_x, d_order, fT, H, h0, hn, k0,  \
-                                                      part);
+#define FLPR_LCV_K(D, LPP)                                                                     \
+  kde_lcv_kernel<D, LPP><<<grid, kLcvThreads, 0, s>>>(g, n, d_x, d_order, fT, H, h0, hn, k0, \
+                                                      part)
+#define FLPR_LCV(D)                     \
+  switch (lpp) {                        \
+    case 1: FLPR_LCV_K(D, 1); break;    \
+    case 2: FLPR_LCV_K(D, 2); break;    \
+    case 4: FLPR_LCV_K(D, 4); break;    \
+    case 8: FLPR_LCV_K(D, 8); break;    \
+    default: FLPR_LCV_K(D, 16); break;  \
+  }
     switch (d) {
       case 1: FLPR_LCV(1) break;
       case 2: FLPR_LCV(2) break;
       default: FLPR_LCV(3) break;
     }
 #undef FLPR_LCV
+#undef FLPR_LCV_K
     FLPR_LAUNCH_CHECK();
   }
   kde_lcv_finish_kernel<<<(H + 127) / 128, 128, 0, s>>>(H, n, part, d_lcv);
