@@ -157,7 +157,7 @@ __host__ __device__ constexpr double root_im(int m) { return root_re((m + 24) & 
 // a * exp(2 pi i m / 32), m known after unrolling: quarter turns are exact,
 // the other roots are constants of the instructions (a shared-memory table
 // cost a load for each of the 34 products of a 32-point stage: T row pass of
-// 32 bandwidths on 512^2 1.405 -> 1.373 ms, column passes 768 -> 747 us).
+// 32 bandwidths on 512^2 1.405 -> 1.363 ms, column passes 768 -> 747 us).
 template <typename V>
 __device__ __forceinline__ V rot32(V a, int m) {
   using R = typename RealOf<V>::T;

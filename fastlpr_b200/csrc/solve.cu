@@ -119,7 +119,9 @@ __global__ void solve_kernel(int order, int H, int HT, int64_t M, int C,
 // stands between the loads, and four channels' loads are in flight.  More
 // than 12 channels a block make the accumulators spill; repeating the solve
 // for the next 12 reads ns planes beside the 12 nt of the channels.  (A test
-// per channel: 540 us for 7 bandwidths of 64^3, 11 channels, 4 terms; 157 now.)
+// per channel: 540 us for 7 bandwidths of 64^3, 11 channels, 4 terms, now 157;
+// 20 of 65536 nodes, 2 terms: 11 channels 205 -> 90 us, 13, which solve twice,
+// 236 -> 151.)
 template <typename Real, int NT, int CMAX>
 __global__ void __launch_bounds__(256)
 solve_reduce_kernel(int order, int H, int HT, int64_t M, int C, const Real* __restrict__ S,

@@ -131,7 +131,7 @@ __global__ void knot_map_kernel(int d, double nm1, const double* __restrict__ st
 // for the same few global counters; and a channel per block leaves a thread's
 // loads free of one another (one pass over points and then channels in turn:
 // 62 us for 1e6 points and 11 channels on 512^2, 29 us for 1e5 on a 1-D grid
-// of 1024; now 44 and 4.4 us).
+// of 1024; now 40 and 4.4 us).
 constexpr int kFewTiles = 512;
 
 __global__ void __launch_bounds__(256)
@@ -1923,7 +1923,8 @@ int flpr_deposit_sorted(int d, int64_t n, const double* d_x, const int* h_L, int
         g, dg, d_x, w.offsets, w.items, w.rec_idx, w.rec, rec_stride(d, nchan), w.absum,
         reinterpret_cast<unsigned long long*>(d_Q), reinterpret_cast<unsigned long long*>(d_B));
   } else if (d == 2) {
-    // wider tiles (stencils of more than 13 taps)
+    // wider tiles (stencils of more than 13 taps; the package's fits keep
+    // records of up to 13, so only direct callers get here)
     auto k = tile_deposit_kernel<2>;
     FLPR_CUDA(raise_dyn_smem(k, smem));
     k<<<(unsigned)nitems, kDepThreads, smem, s>>>(

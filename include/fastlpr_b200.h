@@ -119,8 +119,9 @@ int flpr_point_stats_noalloc(int d, int64_t n, const double* d_x, double* d_stat
  *   nchan-ones_channel channels are h_cols[i] (device float64 arrays of n).
  * d_grid_out: (nchan, L...) real, float (FLPR_PREC_F32) or double, scaled
  *   by 1/n (the 1/M of nufftn_type1.py:709-711).
- * Accumulation is per tile after binning the points by tile (2-D and 3-D
- * FLPR_PREC_F32: in registers; otherwise in shared memory); FLPR_PREC_F32
+ * Accumulation is per tile after binning the points by tile: in registers on
+ * grids of 2 or 3 axes with at least 8 cells on the last two and up to 13
+ * (2-D) or 9 (3-D) taps, otherwise in shared memory.  FLPR_PREC_F32
  * accumulates in 64-bit fixed point (order independent, deterministic),
  * FLPR_PREC_F64 in float64.
  * --------------------------------------------------------------------- */
