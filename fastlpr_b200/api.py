@@ -1756,16 +1756,17 @@ def _pack_to_host(pack: torch.Tensor, sizes: List[int]):
     return [_to_host(t) for t in pack.split(sizes)]
 
 
-def _unpack_outputs(st: _LprState, r: dict, pack) -> dict:
+def _unpack_outputs(st: _LprState, r: dict, pack, views: bool = False) -> dict:
     """The outputs of _finalize_enqueue from the downloaded buffer, or from the
     buffers of its parts (_pack_to_host).  Parts of one buffer are views of it,
-    which keep all of it: those of less than an eighth are copied out."""
+    which keep all of it: those of less than an eighth are copied out, unless
+    the caller copies every part itself (views)."""
     n, M, H = st.n, st.geom.M, r["H"]
     if isinstance(pack, torch.Tensor):
         whole, parts, at = pack.numpy(), [], 0
         for k in _pack_sizes(st, H):
             part = whole[at:at + k]
-            parts.append(part.copy() if 8 * k < whole.size else part)
+            parts.append(part.copy() if 8 * k < whole.size and not views else part)
             at += k
     else:
         parts = [t.numpy() for t in pack]
@@ -1788,7 +1789,7 @@ def _finalize_build(ctx, st: _LprState, r: dict, pend: dict, ev, search,
     geom, opts = st.geom, st.opts
     bw_k = r["bw_k"]
     if "pack" in pend:
-        pend = _unpack_outputs(st, r, pend["pack"])
+        pend = _unpack_outputs(st, r, pend["pack"], views=copy)
     if pend.get("sel") is not None:
         sel = int(np.asarray(pend["sel"])[0])
         if st.calc_dof:
