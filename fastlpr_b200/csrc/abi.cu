@@ -69,6 +69,10 @@ int PlanCache::exec(const PlanKey& key, void* in, void* out, void* work, size_t 
     set_error("cuFFT work area %zu < required %zu", work_bytes, p->work);
     return FLPR_ERR_WORKSPACE;
   }
+  // threads that share the plan (and the handle) enqueue in turn: between
+  // another's settings and its execution ours would send its transform to
+  // the wrong stream and scratch
+  std::lock_guard<std::mutex> lock(run);
   FLPR_CUFFT(cufftSetStream(p->plan, stream));
   FLPR_CUFFT(cufftSetWorkArea(p->plan, work));
   switch (key.type) {

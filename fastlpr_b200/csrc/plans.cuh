@@ -29,6 +29,7 @@ struct Plan {
 
 struct PlanCache {
   std::mutex mu;
+  std::mutex run;  // a plan's stream and work area belong to one call at a time
   std::map<PlanKey, Plan> plans;
   ~PlanCache();
   int get(const PlanKey& key, Plan** out);
