@@ -321,7 +321,7 @@ kde_lcv_kernel(InterpGeom g, int64_t n, const double* __restrict__ x,
 #pragma unroll
     for (int k = 0; k < NC; ++k) v += w[k] * p[coff[k]];
     double fl = ratio * (v - k0n);
-    if (!(fl > 1e-10)) fl = 1e-10;
+    if (fl <= 1e-10) fl = 1e-10;  // NaN (a point without a cell) stays
     return log(fl);
   };
   auto stage = [&](int64_t i) {  // point i's stencil into this lane's place

@@ -67,3 +67,19 @@ def test_nan_points_on_the_device_stay_in_range(cuda_ok, d):
         except ValueError:
             pass
         _usable()
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("d", [1, 2, 3])
+def test_a_density_of_a_constant_predictor_is_refused(cuda_ok, d, precision):
+    """As the oracle does: its scores are NaN."""
+    import fastlpr_b200
+    import oracle.lpr as oracle
+    x = np.random.default_rng(d).random((500, d))
+    x[:, d - 1] = 0.3
+    h, N = np.repeat([[0.2], [0.4]], d, 1), [16] * d if d > 1 else 16
+    with pytest.raises(ValueError, match="NaN or Inf"):
+        oracle.cv_fastkde(x, h, {"N": N})
+    with pytest.raises(ValueError, match="NaN or Inf"):
+        fastlpr_b200.cv_fastkde(x, h, {"N": N, "precision": precision})
+    _usable()
