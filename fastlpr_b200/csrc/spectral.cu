@@ -444,18 +444,7 @@ __global__ void sep_crop_kernel(SepArgs sa, int np, SepProds prods, const Real* 
   }
 }
 
-// Products that one call of a whole inverse takes where its rounding depends
-// on their number.  Of 1-D lengths from 4 to 131072, powers of two and others,
-// FP32 results of 4096 are other bits for up to 33 at a time than from 64 on,
-// those of 32768 and 65536 for up to 127 than from 128 on, and a remainder of a
-// list would round unlike the rest of it (all of 242 products of 32768 in one
-// call moved a fit's scores by 1.5e-7 against calls of 128).  FP64 results and
-// lengths up to 2048, where the number of launches counts, are the same for
-// any number; more axes were not looked at and keep 128.
-constexpr int kFftBatch = 128;
-constexpr int kFreeLength = 2048;
-
-static int batch_within(int d, const int* L, int nprod, int prec, int most) {
+static int conv_batch(int d, const int* L, int nprod, int prec) {
   int64_t cells = prod(L, d);
   int64_t half = cells / L[d - 1] * (L[d - 1] / 2 + 1);
   size_t es = prec == FLPR_PREC_F32 ? 4 : 8;
@@ -464,31 +453,19 @@ static int batch_within(int d, const int* L, int nprod, int prec, int most) {
   int64_t b = (int64_t)(budget / per);
   if (b < 1) b = 1;
   if (b > nprod) b = nprod;
-  if (b > most) b = most;
+  if (b > kMaxBatch) b = kMaxBatch;
   return (int)b;
 }
 
-// Products of one product and one crop launch: several calls of kFftBatch, and
-// all that are left in the last one.
-static int conv_batch(int d, const int* L, int nprod, int prec) {
-  const int b = batch_within(d, L, nprod, prec, kMaxBatch);
-  return b > kFftBatch && b < nprod ? b / kFftBatch * kFftBatch : b;
-}
-
-static int fft_batch(int d, const int* L, int nprod, int prec) {
-  const bool any = d == 1 && (prec == FLPR_PREC_F64 || L[0] <= kFreeLength);
-  return any ? conv_batch(d, L, nprod, prec) : batch_within(d, L, nprod, prec, kFftBatch);
-}
-
-// Workspace of a batch of products and of their transforms, `nfft` to a call,
-// whose plans `work(nb, &bytes)` sizes: the full calls and the last one.
+// Workspace of a batch of products and of their transforms, whose plans
+// `work(nb, &bytes)` sizes: the full batches and the last one.
 template <typename Work>
-static size_t conv_ws_of(int d, const int* L, int nprod, int prec, int nfft, Work work) {
-  const int B = conv_batch(d, L, nprod, prec), tail = nprod % nfft;
+static size_t conv_ws_of(int d, const int* L, int nprod, int prec, Work work) {
+  const int B = conv_batch(d, L, nprod, prec), tail = nprod % B;
   const int64_t cells = prod(L, d), half = cells / L[d - 1] * (L[d - 1] / 2 + 1);
   const size_t es = prec == FLPR_PREC_F32 ? 4 : 8;
   size_t w1 = 0, w2 = 0;
-  if (work(nfft, &w1) != FLPR_OK || (tail && work(tail, &w2) != FLPR_OK)) return 0;
+  if (work(B, &w1) != FLPR_OK || (tail && work(tail, &w2) != FLPR_OK)) return 0;
   ArenaSize ar;
   ar.take<char>((size_t)B * half * 2 * es);
   ar.take<char>((size_t)B * cells * es);
@@ -683,23 +660,10 @@ static PlanKey conv3_planes(const int* L, int planes, int prec) {
   return grid_plan(2, L + 1, prec == FLPR_PREC_F32 ? CUFFT_C2R : CUFFT_Z2D, planes);
 }
 
-// Whole inverse transforms of nb products, nfft to a call.
-static int inverse_batches(flpr_handle_t handle, const ConvArgs& ca, const int* L, int nb, int nfft,
-                           int type, char* pbuf, char* rbuf, size_t es, void* work,
-                           size_t work_bytes, cudaStream_t s) {
-  for (int b0 = 0; b0 < nb; b0 += nfft) {
-    const int n = nb - b0 < nfft ? nb - b0 : nfft;
-    FLPR_TRY(plans_of(handle).exec(grid_plan(ca.d, L, type, n), pbuf + (size_t)b0 * ca.half * 2 * es,
-                                   rbuf + (size_t)b0 * ca.cells * es, work, work_bytes, s));
-  }
-  return FLPR_OK;
-}
-
 size_t flpr_conv_ws(flpr_handle_t handle, int d, const int* h_L, int nprod, int prec) {
   if (d < 1 || d > 3 || nprod < 1) return 0;
   const int type = prec == FLPR_PREC_F32 ? CUFFT_C2R : CUFFT_Z2D;
-  const int nfft = fft_batch(d, h_L, nprod, prec);
-  return conv_ws_of(d, h_L, nprod, prec, nfft, [&](int nb, size_t* out) {
+  return conv_ws_of(d, h_L, nprod, prec, [&](int nb, size_t* out) {
     return plans_of(handle).work_size(grid_plan(d, h_L, type, nb), out);
   });
 }
@@ -708,8 +672,7 @@ size_t flpr_conv_grid_ws(flpr_handle_t handle, int d, const int* h_G, const int*
                          int prec) {
   if (d != 3) return flpr_conv_ws(handle, d, h_L, nprod, prec);
   if (nprod < 1 || h_G[0] < 1) return 0;
-  const int nfft = conv_batch(d, h_L, nprod, prec);
-  return conv_ws_of(d, h_L, nprod, prec, nfft, [&](int nb, size_t* out) {
+  return conv_ws_of(d, h_L, nprod, prec, [&](int nb, size_t* out) {
     size_t a = 0, b = 0;
     FLPR_TRY(plans_of(handle).work_size(conv3_axis0(h_L, nb, prec), &a));
     FLPR_TRY(plans_of(handle).work_size(conv3_planes(h_L, nb * h_G[0], prec), &b));
@@ -755,7 +718,7 @@ int flpr_conv(flpr_handle_t handle, int d, const int* h_G, const int* h_L, const
     set_error("conv: workspace too small");
     return FLPR_ERR_WORKSPACE;
   }
-  const int B = conv_batch(d, h_L, nprod, prec), nfft = fft_batch(d, h_L, nprod, prec);
+  const int B = conv_batch(d, h_L, nprod, prec);
   FLPR_CHECK_ARG((int64_t)B * ca.cells < ((int64_t)1 << 31),
                  "conv: grid too large for 32-bit batch indexing");
   for (int p = 0; p < nprod; ++p)
@@ -793,7 +756,7 @@ int flpr_conv(flpr_handle_t handle, int d, const int* h_G, const int* h_L, const
       FLPR_TRY(plans_of(handle).exec(conv3_planes(h_L, nb * h_G[0], prec),
                                      pbuf + plane * h_qout[0], rbuf, work, work_bytes, s));
     } else {
-      FLPR_TRY(inverse_batches(handle, ca, h_L, nb, nfft, ctype, pbuf, rbuf, es, work, work_bytes, s));
+      FLPR_TRY(plans_of(handle).exec(grid_plan(d, h_L, ctype, nb), pbuf, rbuf, work, work_bytes, s));
     }
     if (prec == FLPR_PREC_F32) {
       crop_kernel<float><<<crop_grid(ca, nb), 256, 0, s>>>(ca, p0, (const float*)rbuf, add_eps,
@@ -1080,7 +1043,7 @@ int flpr_conv_full(flpr_handle_t handle, int d, const int* h_G, const int* h_L, 
     set_error("conv_full: workspace too small");
     return FLPR_ERR_WORKSPACE;
   }
-  const int B = conv_batch(d, h_L, nprod, prec), nfft = fft_batch(d, h_L, nprod, prec);
+  const int B = conv_batch(d, h_L, nprod, prec);
   FLPR_CHECK_ARG((int64_t)B * ca.cells < ((int64_t)1 << 31),
                  "conv_full: grid too large for 32-bit batch indexing");
   for (int p = 0; p < nprod; ++p)
@@ -1111,7 +1074,7 @@ int flpr_conv_full(flpr_handle_t handle, int d, const int* h_G, const int* h_L, 
                                                          (const double2*)d_K, (double2*)pbuf);
     }
     FLPR_LAUNCH_CHECK();
-    FLPR_TRY(inverse_batches(handle, ca, h_L, nb, nfft, ctype, pbuf, rbuf, es, work, work_bytes, s));
+    FLPR_TRY(plans_of(handle).exec(grid_plan(d, h_L, ctype, nb), pbuf, rbuf, work, work_bytes, s));
     if (prec == FLPR_PREC_F32) {
       crop_kernel<float><<<crop_grid(ca, nb), 256, 0, s>>>(ca, p0, (const float*)rbuf, add_eps,
                                                            (float*)d_out);
