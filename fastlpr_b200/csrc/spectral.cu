@@ -83,6 +83,11 @@ struct ProdDesc {
 };
 static_assert(sizeof(ProdDesc) == 12, "packed product");
 
+// cuFFT rounds the FP32 transforms of 4096, 32768 and 65536 points one way in
+// small batches and another from 64 or 128 on, so the largest batch is part of
+// a result's last bits: of 242 products of 32768, calls of 128 move the scores
+// of a fit by up to 1.5e-7.  Both ways have the same error (root mean square
+// against 64 bits 5.60e-8 at 32768 points, ratio 0.9995 +- 0.0004).
 constexpr int kMaxBatch = 512;
 
 struct ProdBatch {
